@@ -6,6 +6,7 @@
 #pragma once
 
 #include <type_traits>
+#include <utility>
 
 #include "lattice.cuh"
 
@@ -155,23 +156,88 @@ struct CellBgk {
 // steps are issue-bound); FP32 storage, bound by HBM, keeps the scalar code above.  Every operation is spelled out
 // (no contraction left to the compiler), so a cell's result does not depend on V, and the pull and
 // in-place steps, which share this code, produce the same bits.  The sequence per cell:
-//   s = g0 + g1 + ... + g18, j = the signed sums in q order, rho = 1 + s, inv = 1/rho (IEEE), u = j inv
-//   t = ux ux + uy uy + uz uz (two FMAs), base = -1.5 t, feq0 = w0 (s + rho base)
-//   out0 = (1 - om) g0 + om feq0, and per odd q with a = c_q . u (two terms at most):
-//   sym = fma(om w, s, om w rho (4.5 a a + base)), asym = 3 om w rho a, out_q = (1 - om) g_q + (sym + asym),
-//   out_opp(q) = (1 - om) g_opp(q) + (sym - asym).
+//   S_q = g_q + g_opp, D_q = g_q - g_opp; s = g0 + the S, j = the signed sums of the D, in sum_order
+//   inv = 1 / (1 + s) (IEEE), e = s - 1.5 inv (jx jx + jy jy + jz jz) (two FMAs), out0 = (1-om) g0 + om w0 e
+//   a = (3 om w) (c_q . j), t = om w e + (inv / (2 om w)) a a   [= om w rho (4.5 (c.u)^2 - 1.5 u.u) + om w s]
+//   u = (1-om)/2 S + t, v = (1-om)/2 D + a; out_q = u + v, out_opp(q) = u - v.
+// order in which the pairs enter the sums: those with c_z = 0 first, as a sweep along z has them
+__host__ __device__ constexpr int sum_order(int i) {
+    constexpr int t[Q / 2] = {1, 3, 7, 9, 5, 11, 13, 15, 17};
+    return t[i];
+}
+// The opposite pairs enter as sums S = g_q + g_opp and differences D = g_q - g_opp.
+template <class T>
+struct LaneBgk {
+    using L = Lanes<T>;
+    float om;
+    T s, jx, jy, jz;  // sum and momentum; finish() turns s into e = s - 1.5 j.j / rho
+    T inv;            // 1 / rho
+    T k, b, ax, ay, az;  // of the class at hand (faces, edges)
+
+    // 3 om w of the classes.  A momentum component is relaxed by 2 a1 + 8 a2 in all, which has to be om: the
+    // faces take what the edges' rounding leaves (a common factor off by 3e-8 in every step would be a
+    // systematic gain of momentum).
+    float a1, a2;
+
+    __device__ __forceinline__ explicit LaneBgk(float omega) : om(omega) {
+        a2 = __fmul_rn(omega, 1.f / 12.f);
+        a1 = 0.5f * __fmaf_rn(-8.f, a2, omega);
+    }
+
+    __device__ __forceinline__ void add_rest(T g0) { s = g0; }
+    // the pair (q, q+1), in the order q = sum_order(0), sum_order(1), ...: ga, gb become S, D
+    __device__ __forceinline__ void add(int q, T& ga, T& gb) {
+        const T S = L::add(ga, gb), D = L::sub(ga, gb);
+        s = L::add(s, S);
+        if (cx(q) != 0) jx = q == 1 ? D : L::add(jx, D);
+        if (cy(q) != 0) jy = q == 3 ? D : cy(q) > 0 ? L::add(jy, D) : L::sub(jy, D);
+        if (cz(q) != 0) jz = q == 5 ? D : cz(q) > 0 ? L::add(jz, D) : L::sub(jz, D);
+        ga = S;
+        gb = D;
+    }
+    __device__ __forceinline__ void finish() {
+        inv = L::rcp(L::add(L::bc(1.f), s));
+        T t = L::mul(jx, jx);
+        t = L::fma(jy, jy, t);
+        t = L::fma(jz, jz, t);
+        s = L::fma(L::mul(L::bc(-1.5f), inv), t, s);
+    }
+    __device__ __forceinline__ T rest(T g0) const { return L::fma(L::bc(1.f - om), g0, L::mul(L::bc(om * wf(0)), s)); }
+    // relaxed populations q and q+1 = opp(q) (q odd, ascending from 1) from S and D
+    __device__ __forceinline__ void pair(int q, T S, T D, T& oa, T& ob) {
+        if (q == 1 || q == 7) {
+            const float w = q == 1 ? a1 : a2;
+            b = L::mul(L::bc(om * wf(q)), s);
+            k = L::mul(L::bc(0.5f / (om * wf(q))), inv);
+            ax = L::mul(L::bc(w), jx);
+            ay = L::mul(L::bc(w), jy);
+            az = L::mul(L::bc(w), jz);
+        }
+        // om times the antisymmetric part: 3 om w c.j (c's first non-zero component is positive for odd q)
+        T a = cx(q) != 0 ? ax : (cy(q) != 0 ? ay : az);
+        if (cx(q) != 0 && cy(q) != 0) a = cy(q) > 0 ? L::add(a, ay) : L::sub(a, ay);
+        if ((cx(q) != 0 || cy(q) != 0) && cz(q) != 0) a = cz(q) > 0 ? L::add(a, az) : L::sub(a, az);
+        const T t = L::fma(L::mul(k, a), a, b);  // om times the symmetric part
+        const T h = L::bc(0.5f * (1.f - om));
+        const T u = L::fma(h, S, t), v = L::fma(h, D, a);
+        oa = L::add(u, v);
+        ob = L::sub(u, v);
+    }
+};
+
 template <int V>
 struct CellBgk<float, V, true, true> {
     static constexpr bool PAIR = V % 2 == 0;
-    static constexpr int NP = PAIR ? V / 2 : V;  // lanes
+    static constexpr int NP = PAIR ? V / 2 : V;  // lane sets
     using T = typename std::conditional<PAIR, float2, float>::type;
-    using L = Lanes<T>;
-    float om, omc;
-    T s[NP], rho[NP], ux[NP], uy[NP], uz[NP], base[NP];
-    T owr1[NP], owr2[NP], owr3a[NP], owr3b[NP];
+    float om;
+    LaneBgk<T> c[NP];
     T orest[NP];
 
-    __device__ __forceinline__ explicit CellBgk(float omega) : om(omega), omc(1.f - omega) {}
+    template <int... I>
+    __device__ __forceinline__ CellBgk(float omega, std::integer_sequence<int, I...>)
+        : om(omega), c{((void)I, LaneBgk<T>(omega))...} {}
+    __device__ __forceinline__ explicit CellBgk(float omega) : CellBgk(omega, std::make_integer_sequence<int, NP>{}) {}
 
     static __device__ __forceinline__ T get(const float (&f)[V][Q], int p, int q) {
         if constexpr (PAIR) return make_float2(f[2 * p][q], f[2 * p + 1][q]);
@@ -185,53 +251,22 @@ struct CellBgk<float, V, true, true> {
             o[p] = v;
         }
     }
-    // c_q . u for odd q (its first non-zero component is positive)
-    __device__ __forceinline__ T cdot_odd(int q, int p) const {
-        T a = cx(q) != 0 ? ux[p] : (cy(q) != 0 ? uy[p] : uz[p]);
-        if (cx(q) != 0 && cy(q) != 0) a = cy(q) > 0 ? L::add(a, uy[p]) : L::sub(a, uy[p]);
-        if ((cx(q) != 0 || cy(q) != 0) && cz(q) != 0) a = cz(q) > 0 ? L::add(a, uz[p]) : L::sub(a, uz[p]);
-        return a;
-    }
+
+    T S[NP][Q / 2], D[NP][Q / 2];
 
     __device__ __forceinline__ void moments(const float (&f)[V][Q]) {
 #pragma unroll
         for (int p = 0; p < NP; ++p) {
-            T g[Q];
+            c[p].add_rest(get(f, p, 0));
 #pragma unroll
-            for (int q = 0; q < Q; ++q) g[q] = get(f, p, q);
-            T sm = g[0];
-#pragma unroll
-            for (int q = 1; q < Q; ++q) sm = L::add(sm, g[q]);
-            // j in q order: a signed sum of the populations with that velocity component
-            constexpr int kx[10] = {1, 2, 7, 8, 9, 10, 11, 12, 13, 14}, ky[10] = {3, 4, 7, 8, 9, 10, 15, 16, 17, 18},
-                          kz[10] = {5, 6, 11, 12, 13, 14, 15, 16, 17, 18};
-            T jx = g[1], jy = g[3], jz = g[5];
-#pragma unroll
-            for (int i = 1; i < 10; ++i) {
-                jx = cx(kx[i]) > 0 ? L::add(jx, g[kx[i]]) : L::sub(jx, g[kx[i]]);
-                jy = cy(ky[i]) > 0 ? L::add(jy, g[ky[i]]) : L::sub(jy, g[ky[i]]);
-                jz = cz(kz[i]) > 0 ? L::add(jz, g[kz[i]]) : L::sub(jz, g[kz[i]]);
+            for (int i = 0; i < Q / 2; ++i) {
+                const int q = sum_order(i);
+                S[p][q / 2] = get(f, p, q);
+                D[p][q / 2] = get(f, p, q + 1);
+                c[p].add(q, S[p][q / 2], D[p][q / 2]);
             }
-            const T rh = L::add(L::bc(1.f), sm);
-            const T inv = L::rcp(rh);
-            s[p] = sm;
-            rho[p] = rh;
-            ux[p] = L::mul(jx, inv);
-            uy[p] = L::mul(jy, inv);
-            uz[p] = L::mul(jz, inv);
-            T t = L::mul(ux[p], ux[p]);
-            t = L::fma(uy[p], uy[p], t);
-            t = L::fma(uz[p], uz[p], t);
-            base[p] = L::mul(L::bc(-1.5f), t);
-            // the folded per-class terms and the rest population
-            const T feq0 = L::mul(L::bc(wf(0)), L::fma(rh, base[p], sm));
-            orest[p] = L::fma(L::bc(omc), g[0], L::mul(L::bc(om), feq0));
-            const T orho = L::mul(L::bc(om), rh);
-            owr1[p] = L::mul(orho, L::bc(wf(1)));
-            owr2[p] = L::mul(orho, L::bc(wf(7)));
-            owr3a[p] = L::mul(L::bc(3.f), owr1[p]);
-            owr3b[p] = L::mul(L::bc(3.f), owr2[p]);
-
+            c[p].finish();
+            orest[p] = c[p].rest(get(f, p, 0));
         }
     }
 
@@ -242,18 +277,13 @@ struct CellBgk<float, V, true, true> {
     }
 
     // relaxed populations q and q+1 = opp(q) (q odd) of every cell
-    __device__ __forceinline__ void pair(const float (&f)[V][Q], int q, float (&oa)[V], float (&ob)[V]) const {
+    __device__ __forceinline__ void pair(const float (&)[V][Q], int q, float (&oa)[V], float (&ob)[V]) {
 #pragma unroll
         for (int p = 0; p < NP; ++p) {
-            const T a = cdot_odd(q, p);
-            const T owr = q < 7 ? owr1[p] : owr2[p];
-            const T t = L::mul(owr, L::fma(L::mul(L::bc(4.5f), a), a, base[p]));
-            // + omega w s as one FMA (a product by a broadcast constant then an add is not compiled
-            // alike in every kernel; an FMA is)
-            const T osym = L::fma(L::bc(om * wf(q)), s[p], t);
-            const T oasym = L::mul(q < 7 ? owr3a[p] : owr3b[p], a);
-            put(oa, p, L::fma(L::bc(omc), get(f, p, q), L::add(osym, oasym)));
-            put(ob, p, L::fma(L::bc(omc), get(f, p, q + 1), L::sub(osym, oasym)));
+            T a, b;
+            c[p].pair(q, S[p][q / 2], D[p][q / 2], a, b);
+            put(oa, p, a);
+            put(ob, p, b);
         }
     }
 };
