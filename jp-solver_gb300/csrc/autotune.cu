@@ -7,6 +7,8 @@
 #include "kernels.h"
 #include "solver.h"
 
+#include <algorithm>
+
 using namespace jp;
 
 extern "C" jp_status jp_autotune(jp_config* cfg, int32_t steps, double* best) {
@@ -25,6 +27,9 @@ extern "C" jp_status jp_autotune(jp_config* cfg, int32_t steps, double* best) {
         const int tpbs[4] = {64, 128, 256, 512};
         int bv = s->vec, bt = s->tpb;
         const double cells = double(s->cells);
+        // the mapping belongs to the single step; two-step passes, where they are used, do not follow it
+        const bool two = s->pair.use;
+        s->pair.use = false;
         for (int v : vecs) {
             if (!vec_supported(s->storage, v) || s->n % v || ((long long)s->cells / v) % 32) continue;
             if (s->inplace && v != s->vec) continue;  // the in-place steps run the storage's default width
@@ -45,6 +50,19 @@ extern "C" jp_status jp_autotune(jp_config* cfg, int32_t steps, double* best) {
                     bt = t;
                 }
             }
+        }
+        if (two) {
+            s->pair.use = true;
+            s->vec = bv;
+            s->tpb = bt;
+            float ms = 0.f;
+            st = jp_step(s, 2);
+            if (st == JP_OK) st = jp_step_timed(s, steps, &ms);
+            if (st != JP_OK) {
+                jp_destroy(s);
+                return st;
+            }
+            *best = std::max(*best, cells * steps / (double(ms) * 1e-3));
         }
         jp_destroy(s);
         cfg->vec = bv;

@@ -70,6 +70,73 @@ static jp_status batched_step(const std::vector<jp_solver*>& members, cudaStream
     return JP_OK;
 }
 
+// Two lattice steps of `members` in one pass (uniform_pair.cu), one launch per storage and per kMaxBatch
+// cubes; plans[k] belongs to members[k].  Every member shares the storage.
+static jp_status batched_pair(const std::vector<jp_solver*>& members, const std::vector<PairPlan>& plans, cudaStream_t st) {
+    for (size_t i = 0; i < members.size(); i += kMaxBatch) {
+        const size_t cnt = std::min(members.size() - i, (size_t)kMaxBatch);
+        UniSolve us[kMaxBatch];
+        std::memset(us, 0, sizeof us);
+        for (size_t k = 0; k < cnt; ++k) {
+            jp_solver* m = members[i + k];
+            us[k].src = m->fa;
+            us[k].dst = m->fb;
+            us[k].n = m->n;
+            us[k].omega = float(m->info.omega);
+        }
+        ECK(launch_stream_collide_pair(members[0]->storage, us, plans.data() + i, (int)cnt, members[0]->sms, st),
+            "batched two-step pass");
+        for (size_t k = 0; k < cnt; ++k) {
+            std::swap(members[i + k]->fa, members[i + k]->fb);
+            members[i + k]->step_count += 2;
+        }
+    }
+    return JP_OK;
+}
+
+// The cubes of a set that take two-step passes together: per storage, largest first, planned as one launch;
+// none where the plan is no faster than single steps.  The others are listed in `single`.
+struct PairGroups {
+    std::vector<std::vector<jp_solver*>> members;
+    std::vector<std::vector<PairPlan>> plans;
+    std::vector<jp_solver*> single;
+};
+static PairGroups pair_groups(const std::vector<jp_solver*>& set) {
+    PairGroups g;
+    std::map<int, std::vector<jp_solver*>> by;
+    for (jp_solver* m : set) {
+        if (m->pair_tile.tiles == 0) g.single.push_back(m);
+        else by[m->storage].push_back(m);
+    }
+    for (auto& b : by) {
+        std::vector<jp_solver*>& v = b.second;
+        std::stable_sort(v.begin(), v.end(), [](const jp_solver* x, const jp_solver* y) { return x->n > y->n; });
+        std::vector<PairPlan> plans(v.size());
+        bool use = true;
+        for (size_t i = 0; use && i < v.size(); i += kMaxBatch) {
+            const int cnt = (int)std::min(v.size() - i, (size_t)kMaxBatch);
+            int n[kMaxBatch];
+            for (int k = 0; k < cnt; ++k) {
+                n[k] = v[i + k]->n;
+                plans[i + k] = v[i + k]->pair_tile;
+            }
+            if (cnt == 1) {
+                plans[i] = v[i]->pair;
+                use = v[i]->pair.use;
+            } else {
+                use = pair_plan_batch(b.first, n, cnt, v[i]->sms, plans.data() + i);
+            }
+        }
+        if (use) {
+            g.members.push_back(v);
+            g.plans.push_back(std::move(plans));
+        } else {
+            g.single.insert(g.single.end(), v.begin(), v.end());
+        }
+    }
+    return g;
+}
+
 }  // namespace jp
 
 using namespace jp;
@@ -219,8 +286,17 @@ jp_status jp_ensemble_step(jp_ensemble* e, int64_t nsteps) {
             if (st != JP_OK) return st;
             in_persist[k] = true;
         }
+    const PairGroups pg = pair_groups(nsteps > 1 ? uni : std::vector<jp_solver*>());
     for (int64_t i = 0; i < nsteps; ++i) {
-        jp_status st = batched_step(uni, e->stream);
+        jp_status st = JP_OK;
+        if (nsteps == 1 || (i == nsteps - 1 && nsteps % 2)) {  // the odd step out
+            st = batched_step(uni, e->stream);
+        } else {
+            if (i % 2 == 0)
+                for (size_t k = 0; st == JP_OK && k < pg.members.size(); ++k)
+                    st = batched_pair(pg.members[k], pg.plans[k], e->stream);
+            if (st == JP_OK) st = batched_step(pg.single, e->stream);
+        }
         if (st != JP_OK) return st;
         for (size_t k = 0; k < amr.size(); ++k) {
             if (in_persist[k]) continue;
@@ -996,26 +1072,62 @@ static jp_status server_tick(jp_server* sv, int32_t* n_active, int32_t* n_queued
     std::vector<jp_solver*> members;
     const auto tsb = clk::now();
     bool spanned = false;
-    for (long long t = 0;; ++t) {
+    std::vector<jp_solver*> ahead;
+    for (long long t = 0;;) {
         const jp_status dst = launch_diags();
         if (dst != JP_OK) return dst;
-        if (t == T) break;
+        if (t >= T) break;
         moving.clear();
         members.clear();
+        ahead.clear();
+        // the solves two steps or more from their next diagnostic and their end take a two-step pass where that
+        // is faster; the others two single steps
         for (Job* j : sv->active)
             if (j->error == JP_OK && j->step < j->steps) {
                 moving.push_back(j);
-                members.push_back(j->s);
+                const long long left = std::min(j->steps - j->step, j->diagK - j->step % j->diagK);
+                (t + 2 <= T && left >= 2 ? ahead : members).push_back(j->s);
             }
-        if (members.empty()) break;
+        if (moving.empty()) break;
         if (!spanned) {
             ECK(span_open(sv, sv->uspan, sv->uspan_tick, &jp_server_stats::uniform_gpu_s, sv->stream), "span");
             spanned = true;
         }
-        jp_status st = batched_step(members, sv->stream);
+        const PairGroups pg = pair_groups(ahead);
+        jp_status st = JP_OK;
+        for (size_t k = 0; st == JP_OK && k < pg.members.size(); ++k) st = batched_pair(pg.members[k], pg.plans[k], sv->stream);
         if (st != JP_OK) return st;
-        for (Job* j : moving)
-            if (++j->step % j->diagK == 0) j->need_diag = true;  // launched before the next step
+        members.insert(members.end(), pg.single.begin(), pg.single.end());
+        auto paired = [&pg](const jp_solver* s) {
+            for (const auto& g : pg.members)
+                if (std::find(g.begin(), g.end(), s) != g.end()) return true;
+            return false;
+        };
+        const int sub = pg.members.empty() ? 1 : 2;  // lattice steps of this round
+        for (int u = 0; u < sub; ++u) {
+            if (u) {  // the solves outside the pass: their diagnostics due between its two steps, then a second step
+                const jp_status ds = launch_diags();
+                if (ds != JP_OK) return ds;
+                members.clear();
+                for (size_t k = 0; k < moving.size();) {
+                    if (paired(moving[k]->s) || moving[k]->step >= moving[k]->steps) {
+                        moving.erase(moving.begin() + k);
+                    } else {
+                        members.push_back(moving[k]->s);
+                        ++k;
+                    }
+                }
+            }
+            if (!members.empty()) {
+                st = batched_step(members, sv->stream);
+                if (st != JP_OK) return st;
+            }
+            for (Job* j : moving) {
+                j->step += u == 0 && sub == 2 && paired(j->s) ? 2 : 1;
+                if (j->step % j->diagK == 0) j->need_diag = true;  // launched before the next step
+            }
+        }
+        t += sub;
     }
     if (spanned) {
         ECK(span_close(sv->uspan, sv->uspan_tick, sv->stream), "span");

@@ -67,6 +67,9 @@ struct jp_solver {
     double* diag_dev = nullptr;  // 3 doubles (+ the error word's copy, uniform)
     double* diag_host = nullptr; // 4 doubles, pinned
     int vec = 0, tpb = 0;
+    jp::PairPlan pair{};       // two steps in one pass, where pair.use (uniform_pair.cu)
+    jp::PairPlan pair_tile{};  // the same in a launch of many cubes
+    int sms = 0;               // multiprocessors of the device
     float* outbuf = nullptr;   // device Q / speed / velocity for output frames, allocated on first use
     // populations staged for the next step (jp_stage_populations): uploaded into `staging` on
     // copy_stream while the solver's stream works, swapped in as fa by the next step

@@ -94,6 +94,11 @@ jp_status uniform_create(jp_solver* s) {
         s->vec = pick_vec(c.storage, c.n, c.vec);
         if (!s->vec) return fail(JP_ERR_INVALID, "no vector width fits n=%d (requested vec=%d)", c.n, c.vec);
     }
+    JP_CK(cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, s->device), "cudaDeviceGetAttribute");
+    if (!s->inplace) {
+        s->pair = pair_plan(s->storage, s->n, s->sms);
+        s->pair_tile = pair_tile_plan(s->storage, s->n, s->sms);
+    }
     const size_t bytes = (size_t)Q * s->cells * s->elem;
     s->info.bytes_state = (int64_t)((s->inplace ? 1 : 2) * bytes);
     JP_CK(dev_alloc(s, &s->fa, bytes), "cudaMalloc populations");
@@ -218,7 +223,16 @@ jp_status uniform_step(jp_solver* s, int64_t nsteps) {
         }
         return JP_OK;
     }
-    for (int64_t i = 0; i < nsteps; ++i) {
+    int64_t i = 0;
+    for (; s->pair.use && i + 1 < nsteps; i += 2) {  // two steps in one pass; an odd one out below
+        u.src = s->fa;
+        u.dst = s->fb;
+        cudaError_t e = launch_stream_collide_pair(s->storage, &u, &s->pair, 1, s->sms, s->stream);
+        if (e != cudaSuccess) return cuda_fail(e, "two-step launch");
+        std::swap(s->fa, s->fb);
+        s->step_count += 2;
+    }
+    for (; i < nsteps; ++i) {
         u.src = s->fa;
         u.dst = s->fb;
         cudaError_t e = launch_stream_collide(s->storage, &u, 1, s->vec, s->tpb, s->stream);
