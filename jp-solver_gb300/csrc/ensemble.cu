@@ -52,8 +52,7 @@ static jp_status batched_step(const std::vector<jp_solver*>& members, cudaStream
                 us[k].src = m->fa;
                 us[k].dst = m->inplace ? m->fa : m->fb;
                 us[k].n = m->n;
-                us[k].omega = float(m->info.omega);
-                us[k].omega_d = m->info.omega;
+                us[k].set_omega(m->info.omega);
             }
             if (v[i]->inplace) {
                 ECK(launch_stream_collide_inplace(v[i]->storage, us, (int)cnt, int(v[i]->step_count & 1), v[i]->vec,
@@ -70,8 +69,8 @@ static jp_status batched_step(const std::vector<jp_solver*>& members, cudaStream
     return JP_OK;
 }
 
-// Two lattice steps of `members` in one pass (uniform_pair.cu), one launch per storage and per kMaxBatch
-// cubes; plans[k] belongs to members[k].  Every member shares the storage.
+// Two lattice steps of `members` (FP32) in one pass (uniform_pair.cu), one launch per kMaxBatch cubes; plans[k]
+// belongs to members[k].
 static jp_status batched_pair(const std::vector<jp_solver*>& members, const std::vector<PairPlan>& plans, cudaStream_t st) {
     for (size_t i = 0; i < members.size(); i += kMaxBatch) {
         const size_t cnt = std::min(members.size() - i, (size_t)kMaxBatch);
@@ -82,9 +81,9 @@ static jp_status batched_pair(const std::vector<jp_solver*>& members, const std:
             us[k].src = m->fa;
             us[k].dst = m->fb;
             us[k].n = m->n;
-            us[k].omega = float(m->info.omega);
+            us[k].set_omega(m->info.omega);
         }
-        ECK(launch_stream_collide_pair(members[0]->storage, us, plans.data() + i, (int)cnt, members[0]->sms, st),
+        ECK(launch_stream_collide_pair(us, plans.data() + i, (int)cnt, members[0]->sms, st),
             "batched two-step pass");
         for (size_t k = 0; k < cnt; ++k) {
             std::swap(members[i + k]->fa, members[i + k]->fb);
@@ -94,45 +93,36 @@ static jp_status batched_pair(const std::vector<jp_solver*>& members, const std:
     return JP_OK;
 }
 
-// The cubes of a set that take two-step passes together: per storage, largest first, planned as one launch;
-// none where the plan is no faster than single steps.  The others are listed in `single`.
-struct PairGroups {
-    std::vector<std::vector<jp_solver*>> members;
-    std::vector<std::vector<PairPlan>> plans;
-    std::vector<jp_solver*> single;
+// The cubes of a set that take two-step passes together, largest first, planned as launches of up to kMaxBatch
+// cubes; none where the plan is no faster than single steps.  The others are listed in `single`.
+struct PairGroup {
+    std::vector<jp_solver*> members, single;
+    std::vector<PairPlan> plans;
 };
-static PairGroups pair_groups(const std::vector<jp_solver*>& set) {
-    PairGroups g;
-    std::map<int, std::vector<jp_solver*>> by;
-    for (jp_solver* m : set) {
-        if (m->pair_tile.tiles == 0) g.single.push_back(m);
-        else by[m->storage].push_back(m);
-    }
-    for (auto& b : by) {
-        std::vector<jp_solver*>& v = b.second;
-        std::stable_sort(v.begin(), v.end(), [](const jp_solver* x, const jp_solver* y) { return x->n > y->n; });
-        std::vector<PairPlan> plans(v.size());
-        bool use = true;
-        for (size_t i = 0; use && i < v.size(); i += kMaxBatch) {
-            const int cnt = (int)std::min(v.size() - i, (size_t)kMaxBatch);
-            int n[kMaxBatch];
-            for (int k = 0; k < cnt; ++k) {
-                n[k] = v[i + k]->n;
-                plans[i + k] = v[i + k]->pair_tile;
-            }
-            if (cnt == 1) {
-                plans[i] = v[i]->pair;
-                use = v[i]->pair.use;
-            } else {
-                use = pair_plan_batch(b.first, n, cnt, v[i]->sms, plans.data() + i);
-            }
+static PairGroup pair_group(const std::vector<jp_solver*>& set) {
+    PairGroup g;
+    for (jp_solver* m : set) (m->pair_tile.tiles ? g.members : g.single).push_back(m);
+    std::vector<jp_solver*>& v = g.members;
+    std::stable_sort(v.begin(), v.end(), [](const jp_solver* x, const jp_solver* y) { return x->n > y->n; });
+    g.plans.resize(v.size());
+    bool use = true;
+    for (size_t i = 0; use && i < v.size(); i += kMaxBatch) {
+        const int cnt = (int)std::min(v.size() - i, (size_t)kMaxBatch);
+        int n[kMaxBatch];
+        for (int k = 0; k < cnt; ++k) {
+            n[k] = v[i + k]->n;
+            g.plans[i + k] = v[i + k]->pair_tile;
         }
-        if (use) {
-            g.members.push_back(v);
-            g.plans.push_back(std::move(plans));
+        if (cnt == 1) {
+            g.plans[i] = v[i]->pair;
+            use = v[i]->pair.use;
         } else {
-            g.single.insert(g.single.end(), v.begin(), v.end());
+            use = pair_plan_batch(n, cnt, v[i]->sms, g.plans.data() + i);
         }
+    }
+    if (!use) {
+        g.single.insert(g.single.end(), v.begin(), v.end());
+        v.clear();
     }
     return g;
 }
@@ -286,15 +276,13 @@ jp_status jp_ensemble_step(jp_ensemble* e, int64_t nsteps) {
             if (st != JP_OK) return st;
             in_persist[k] = true;
         }
-    const PairGroups pg = pair_groups(nsteps > 1 ? uni : std::vector<jp_solver*>());
+    const PairGroup pg = pair_group(nsteps > 1 ? uni : std::vector<jp_solver*>());
     for (int64_t i = 0; i < nsteps; ++i) {
         jp_status st = JP_OK;
         if (nsteps == 1 || (i == nsteps - 1 && nsteps % 2)) {  // the odd step out
             st = batched_step(uni, e->stream);
         } else {
-            if (i % 2 == 0)
-                for (size_t k = 0; st == JP_OK && k < pg.members.size(); ++k)
-                    st = batched_pair(pg.members[k], pg.plans[k], e->stream);
+            if (i % 2 == 0) st = batched_pair(pg.members, pg.plans, e->stream);
             if (st == JP_OK) st = batched_step(pg.single, e->stream);
         }
         if (st != JP_OK) return st;
@@ -1093,15 +1081,12 @@ static jp_status server_tick(jp_server* sv, int32_t* n_active, int32_t* n_queued
             ECK(span_open(sv, sv->uspan, sv->uspan_tick, &jp_server_stats::uniform_gpu_s, sv->stream), "span");
             spanned = true;
         }
-        const PairGroups pg = pair_groups(ahead);
-        jp_status st = JP_OK;
-        for (size_t k = 0; st == JP_OK && k < pg.members.size(); ++k) st = batched_pair(pg.members[k], pg.plans[k], sv->stream);
+        const PairGroup pg = pair_group(ahead);
+        jp_status st = batched_pair(pg.members, pg.plans, sv->stream);
         if (st != JP_OK) return st;
         members.insert(members.end(), pg.single.begin(), pg.single.end());
         auto paired = [&pg](const jp_solver* s) {
-            for (const auto& g : pg.members)
-                if (std::find(g.begin(), g.end(), s) != g.end()) return true;
-            return false;
+            return std::find(pg.members.begin(), pg.members.end(), s) != pg.members.end();
         };
         const int sub = pg.members.empty() ? 1 : 2;  // lattice steps of this round
         for (int u = 0; u < sub; ++u) {

@@ -16,8 +16,15 @@ struct UniSolve {
     int n;                   // edge
     int nxs;                 // n / V: x segments per row
     float omega;             // 1/tau (FP32 and shifted storages)
-    int pad;
+    float half_inv;          // 1 / (2 omega)
     double omega_d;          // 1/tau (FP64 storage)
+    double half_inv_d;       // 1 / (2 omega_d)
+    void set_omega(double w) {
+        omega = float(w);
+        half_inv = 0.5f / omega;
+        omega_d = w;
+        half_inv_d = 0.5 / w;
+    }
     long long blk_begin;     // first CUDA block of this cube in the launch
     long long nseg;          // n^3 / V threads
 };
@@ -45,18 +52,18 @@ int inplace_tpb(int storage, int vec, int tpb, int max_n);
 // Two steps of `count` cubes in one pass (uniform_pair.cu): src -> dst holds the state two steps on, the
 // same bits as two launch_stream_collide steps.  A plan gives a cube's tile (tx x ty cells, which a CTA
 // marches along z over chunks of zc planes); us is the model's time per step, use whether that beats
-// the single step.  FP32 and 16-bit storages, even n <= 1600.
+// the single step.  FP32 storage, even n <= 1600.
 struct PairPlan {
     int tx, ty, zc, tiles;
     double us;
     bool use;
 };
-PairPlan pair_plan(int storage, int n, int sms);
+PairPlan pair_plan(int n, int sms);
 // a cube's tile in a launch of many cubes (zc not set), and the chunks of cubes of edges n[0..count) with the
 // tiles plans[] in one launch: whether that beats single steps
-PairPlan pair_tile_plan(int storage, int n, int sms);
-bool pair_plan_batch(int storage, const int* n, int count, int sms, PairPlan* plans);
-cudaError_t launch_stream_collide_pair(int storage, const UniSolve* solves, const PairPlan* plans, int count, int sms,
+PairPlan pair_tile_plan(int n, int sms);
+bool pair_plan_batch(const int* n, int count, int sms, PairPlan* plans);
+cudaError_t launch_stream_collide_pair(const UniSolve* solves, const PairPlan* plans, int count, int sms,
                                        cudaStream_t st);
 
 // Largest supported vec for a storage; a valid vec divides n and keeps n^3/vec a multiple of 32.

@@ -143,6 +143,7 @@ struct StF64 {
 #ifdef __CUDACC__
 template <class T> struct Lanes;
 template <> struct Lanes<float> {
+    using real = float;
     static __device__ __forceinline__ float bc(float s) { return s; }
     static __device__ __forceinline__ float add(float a, float b) { return __fadd_rn(a, b); }
     static __device__ __forceinline__ float sub(float a, float b) { return __fadd_rn(a, -b); }
@@ -150,7 +151,17 @@ template <> struct Lanes<float> {
     static __device__ __forceinline__ float fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
     static __device__ __forceinline__ float rcp(float a) { return __frcp_rn(a); }
 };
+template <> struct Lanes<double> {
+    using real = double;
+    static __device__ __forceinline__ double bc(double s) { return s; }
+    static __device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, b); }
+    static __device__ __forceinline__ double sub(double a, double b) { return __dadd_rn(a, -b); }
+    static __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
+    static __device__ __forceinline__ double fma(double a, double b, double c) { return __fma_rn(a, b, c); }
+    static __device__ __forceinline__ double rcp(double a) { return __drcp_rn(a); }
+};
 template <> struct Lanes<float2> {
+    using real = float;
     static __device__ __forceinline__ float2 bc(float s) { return make_float2(s, s); }
     static __device__ __forceinline__ float2 add(float2 a, float2 b) { return __fadd2_rn(a, b); }
     // a - b as a + (-b): an add is never merged with the product before it (an FMA by -1 can be)

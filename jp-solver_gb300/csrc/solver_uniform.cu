@@ -95,9 +95,9 @@ jp_status uniform_create(jp_solver* s) {
         if (!s->vec) return fail(JP_ERR_INVALID, "no vector width fits n=%d (requested vec=%d)", c.n, c.vec);
     }
     JP_CK(cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, s->device), "cudaDeviceGetAttribute");
-    if (!s->inplace) {
-        s->pair = pair_plan(s->storage, s->n, s->sms);
-        s->pair_tile = pair_tile_plan(s->storage, s->n, s->sms);
+    if (!s->inplace && s->storage == JP_FP32) {
+        s->pair = pair_plan(s->n, s->sms);
+        s->pair_tile = pair_tile_plan(s->n, s->sms);
     }
     const size_t bytes = (size_t)Q * s->cells * s->elem;
     s->info.bytes_state = (int64_t)((s->inplace ? 1 : 2) * bytes);
@@ -211,8 +211,7 @@ jp_status uniform_step(jp_solver* s, int64_t nsteps) {
     UniSolve u;
     std::memset(&u, 0, sizeof u);
     u.n = s->n;
-    u.omega = float(s->info.omega);
-    u.omega_d = s->info.omega;
+    u.set_omega(s->info.omega);
     if (s->inplace) {
         u.src = u.dst = s->fa;
         for (int64_t i = 0; i < nsteps; ++i) {
@@ -227,7 +226,7 @@ jp_status uniform_step(jp_solver* s, int64_t nsteps) {
     for (; s->pair.use && i + 1 < nsteps; i += 2) {  // two steps in one pass; an odd one out below
         u.src = s->fa;
         u.dst = s->fb;
-        cudaError_t e = launch_stream_collide_pair(s->storage, &u, &s->pair, 1, s->sms, s->stream);
+        cudaError_t e = launch_stream_collide_pair(&u, &s->pair, 1, s->sms, s->stream);
         if (e != cudaSuccess) return cuda_fail(e, "two-step launch");
         std::swap(s->fa, s->fb);
         s->step_count += 2;

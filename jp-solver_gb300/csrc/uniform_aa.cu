@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(TPB, (aa_local_min_blocks<ST, V, TPB>())) k_aa
         for (int v = 0; v < V; ++v) f[v][q] = (SA && !SH) ? ST::load(L[q].v[v]) - wgt<R>(q) : ST::load(L[q].v[v]);
 
     const R om = sizeof(R) == 8 ? R(d.omega_d) : R(d.omega);
-    CellBgk<R, V, SA, SA> c(om);
+    typename std::conditional<SH, CellBgk16<V>, CellBgk<R, V, SA>>::type c(om, sizeof(R) == 8 ? R(d.half_inv_d) : R(d.half_inv));
     c.moments(f);
     {
         R o0[V];
@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(TPB, (aa_stream_min_blocks<ST, V, TPB>())) k_a
         }
     // 4. relax in place
     const R om = sizeof(R) == 8 ? R(d.omega_d) : R(d.omega);
-    CellBgk<R, V, SA, SA> c(om);
+    typename std::conditional<SH, CellBgk16<V>, CellBgk<R, V, SA>>::type c(om, sizeof(R) == 8 ? R(d.half_inv_d) : R(d.half_inv));
     c.moments(f);
 #pragma unroll
     for (int v = 0; v < V; ++v) f[v][0] = c.rest(f, v);

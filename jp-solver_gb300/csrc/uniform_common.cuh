@@ -79,109 +79,48 @@ constexpr int min_blocks() {
 }
 
 // ---- BGK relaxation of V cells ------------------------------------------------------------------
-// f[v][q] holds the collision inputs of cell v in the collision type R: the shifts g = f - w_q when SA
-// (FP32 shifts on load, the 16-bit formats store shifts), f itself for FP64.  BGK as
-// out = (1 - omega) f + omega feq with omega*w*rho folded per weight class: with a = c.u,
-// feq_pm = w rho (1 - 1.5|u|^2 + 4.5 a^2) +- 3 w rho a (shifted: the -w part cancels against g).
-// PACK: the FP32 relaxation on pairs of cells (CellBgk<float, V, true, true> below), for the 16-bit
-// storages, whose steps are issue-bound; FP32 and FP64 storage keep this one.
-template <class R, int V, bool SA, bool PACK = false>
-struct CellBgk {
-    R om, omc;
-    R s[V], rho[V], ux[V], uy[V], uz[V], usq[V];
-    // per cell: omega*w*rho and (shifted) omega*w*s for the face (1/18) and edge (1/36) classes, and
-    // the base term 1 - 1.5|u|^2 (or -1.5|u|^2 shifted)
-    R owr1[V], owr2[V], owr3a[V], owr3b[V], ows1[V], ows2[V], base[V];
-
-    __device__ __forceinline__ explicit CellBgk(R omega) : om(omega), omc(R(1) - omega) {}
-
-    // moments per cell (one reciprocal of rho instead of three divisions)
-    __device__ __forceinline__ void moments(const R (&f)[V][Q]) {
-#pragma unroll
-        for (int v = 0; v < V; ++v) {
-            const R* g = f[v];
-            R sm = g[0];
-#pragma unroll
-            for (int q = 1; q < Q; ++q) sm += g[q];
-            const R jx = g[1] - g[2] + g[7] - g[8] + g[9] - g[10] + g[11] - g[12] + g[13] - g[14];
-            const R jy = g[3] - g[4] + g[7] - g[8] - g[9] + g[10] + g[15] - g[16] + g[17] - g[18];
-            const R jz = g[5] - g[6] + g[11] - g[12] - g[13] + g[14] + g[15] - g[16] - g[17] + g[18];
-            const R rh = SA ? R(1) + sm : sm;
-            const R inv = R(1) / rh;
-            s[v] = sm;
-            rho[v] = rh;
-            ux[v] = jx * inv;
-            uy[v] = jy * inv;
-            uz[v] = jz * inv;
-            usq[v] = R(1.5) * (ux[v] * ux[v] + uy[v] * uy[v] + uz[v] * uz[v]);
-        }
-    }
-
-    // relaxed rest population of cell v; sets cell v's folded terms for pair()
-    __device__ __forceinline__ R rest(const R (&f)[V][Q], int v) {
-        const R w0 = wgt<R>(0);
-        const R feq = SA ? w0 * (s[v] - rho[v] * usq[v]) : w0 * rho[v] * (R(1) - usq[v]);
-        const R o = omc * f[v][0] + om * feq;
-        const R orho = om * rho[v];
-        owr1[v] = orho * wgt<R>(1);
-        owr2[v] = orho * wgt<R>(7);
-        owr3a[v] = R(3) * owr1[v];
-        owr3b[v] = R(3) * owr2[v];
-        ows1[v] = SA ? om * wgt<R>(1) * s[v] : R(0);
-        ows2[v] = SA ? om * wgt<R>(7) * s[v] : R(0);
-        base[v] = SA ? -usq[v] : R(1) - usq[v];
-        return o;
-    }
-
-    // relaxed populations q and q+1 = opp(q) (q odd) of every cell; rest() must have run for all cells
-    __device__ __forceinline__ void pair(const R (&f)[V][Q], int q, R (&oa)[V], R (&ob)[V]) const {
-#pragma unroll
-        for (int v = 0; v < V; ++v) {
-            const R a = cdot<R>(q, ux[v], uy[v], uz[v]);
-            const R owr = q < 7 ? owr1[v] : owr2[v];
-            const R t = owr * (R(4.5) * a * a + base[v]);
-            const R osym = SA ? (q < 7 ? ows1[v] : ows2[v]) + t : t;  // omega * symmetric part
-            const R oasym = (q < 7 ? owr3a[v] : owr3b[v]) * a;           // omega * antisymmetric part
-            oa[v] = omc * f[v][q] + (osym + oasym);
-            ob[v] = omc * f[v][q + 1] + (osym - oasym);
-        }
-    }
-};
-
-// ---- the same relaxation in FP32 on pairs of cells ------------------------------------------------
-// Blackwell issues two FP32 adds, multiplies or FMAs in one instruction (f32x2; __fadd2_rn,
+// f[v][q] holds the collision inputs of cell v in the collision type R: the shifts g = f - w_q when SA (FP32
+// shifts on load), f itself for FP64.  half_inv = 1 / (2 omega).
+//
+// FP32: Blackwell issues two FP32 adds, multiplies or FMAs in one instruction (f32x2; __fadd2_rn,
 // __fmul2_rn, __ffma2_rn, each lane rounded to nearest like its scalar op).  The FP32 steps hold V = 2,
 // 4 or 8 cells per thread, so the relaxation runs on pairs of cells and issues half the FP32
-// instructions; an odd V runs the same sequence on single floats.  The 16-bit storages use it (their
-// steps are issue-bound); FP32 storage, bound by HBM, keeps the scalar code above.  Every operation is spelled out
-// (no contraction left to the compiler), so a cell's result does not depend on V, and the pull and
-// in-place steps, which share this code, produce the same bits.  The sequence per cell:
+// instructions; an odd V runs the same sequence on single floats.  FP64 runs it on single doubles.  Every
+// operation is spelled out (no contraction left to the compiler), so a cell's result does not depend on
+// V, and the pull, two-step and in-place steps, which share this code, produce the same bits.  The
+// sequence per cell, 117 operations and a reciprocal (the FP64 step is bound by its FP64 rate):
 //   S_q = g_q + g_opp, D_q = g_q - g_opp; s = g0 + the S, j = the signed sums of the D, in sum_order
-//   inv = 1 / (1 + s) (IEEE), e = s - 1.5 inv (jx jx + jy jy + jz jz) (two FMAs), out0 = (1-om) g0 + om w0 e
+//   rho = 1 + s (s itself in FP64), inv = 1 / rho (IEEE), e = s - 1.5 inv (jx jx + jy jy + jz jz) (two FMAs)
+//   out0 = (1-om) g0 + om w0 e
 //   a = (3 om w) (c_q . j), t = om w e + (inv / (2 om w)) a a   [= om w rho (4.5 (c.u)^2 - 1.5 u.u) + om w s]
 //   u = (1-om)/2 S + t, v = (1-om)/2 D + a; out_q = u + v, out_opp(q) = u - v.
+// Measured against one product chain per population (147 operations; the 16-bit storages keep it, CellBgk16):
+// error against 64 bits of N=64 FP32 after 200 steps 1.4-1.8e-7 -> 1.1-1.5e-7.
 // order in which the pairs enter the sums: those with c_z = 0 first, as a sweep along z has them
 __host__ __device__ constexpr int sum_order(int i) {
     constexpr int t[Q / 2] = {1, 3, 7, 9, 5, 11, 13, 15, 17};
     return t[i];
 }
-// The opposite pairs enter as sums S = g_q + g_opp and differences D = g_q - g_opp.
-template <class T>
+// One lane set T (a float, a double, a pair of floats) of the sequence.  SA: the inputs are shifts.
+template <class T, bool SA>
 struct LaneBgk {
     using L = Lanes<T>;
-    float om;
-    T s, jx, jy, jz;  // sum and momentum; finish() turns s into e = s - 1.5 j.j / rho
+    using R = typename L::real;
+    R om;
+    T s, jx, jy, jz;  // sum and momentum; finish() turns s into e
     T inv;            // 1 / rho
     T k, b, ax, ay, az;  // of the class at hand (faces, edges)
 
     // 3 om w of the classes.  A momentum component is relaxed by 2 a1 + 8 a2 in all, which has to be om: the
     // faces take what the edges' rounding leaves (a common factor off by 3e-8 in every step would be a
     // systematic gain of momentum).
-    float a1, a2;
+    R a1, a2;
 
-    __device__ __forceinline__ explicit LaneBgk(float omega) : om(omega) {
-        a2 = __fmul_rn(omega, 1.f / 12.f);
-        a1 = 0.5f * __fmaf_rn(-8.f, a2, omega);
+    R kc;  // 1 / (2 om)
+
+    __device__ __forceinline__ LaneBgk(R omega, R half_inv) : om(omega), kc(half_inv) {
+        a2 = omega * (R(1) / R(12));
+        a1 = R(0.5) * fma(R(-8), a2, omega);
     }
 
     __device__ __forceinline__ void add_rest(T g0) { s = g0; }
@@ -196,19 +135,21 @@ struct LaneBgk {
         gb = D;
     }
     __device__ __forceinline__ void finish() {
-        inv = L::rcp(L::add(L::bc(1.f), s));
+        inv = L::rcp(SA ? L::add(L::bc(R(1)), s) : s);
         T t = L::mul(jx, jx);
         t = L::fma(jy, jy, t);
         t = L::fma(jz, jz, t);
-        s = L::fma(L::mul(L::bc(-1.5f), inv), t, s);
+        s = L::fma(L::mul(L::bc(R(-1.5)), inv), t, s);
     }
-    __device__ __forceinline__ T rest(T g0) const { return L::fma(L::bc(1.f - om), g0, L::mul(L::bc(om * wf(0)), s)); }
+    __device__ __forceinline__ T rest(T g0) const {
+        return L::fma(L::bc(R(1) - om), g0, L::mul(L::bc(om * wgt<R>(0)), s));
+    }
     // relaxed populations q and q+1 = opp(q) (q odd, ascending from 1) from S and D
     __device__ __forceinline__ void pair(int q, T S, T D, T& oa, T& ob) {
         if (q == 1 || q == 7) {
-            const float w = q == 1 ? a1 : a2;
-            b = L::mul(L::bc(om * wf(q)), s);
-            k = L::mul(L::bc(0.5f / (om * wf(q))), inv);
+            const R w = q == 1 ? a1 : a2;
+            b = L::mul(L::bc(om * wgt<R>(q)), s);
+            k = L::mul(L::bc(kc * R(q == 1 ? 18 : 36)), inv);
             ax = L::mul(L::bc(w), jx);
             ay = L::mul(L::bc(w), jy);
             az = L::mul(L::bc(w), jz);
@@ -218,32 +159,32 @@ struct LaneBgk {
         if (cx(q) != 0 && cy(q) != 0) a = cy(q) > 0 ? L::add(a, ay) : L::sub(a, ay);
         if ((cx(q) != 0 || cy(q) != 0) && cz(q) != 0) a = cz(q) > 0 ? L::add(a, az) : L::sub(a, az);
         const T t = L::fma(L::mul(k, a), a, b);  // om times the symmetric part
-        const T h = L::bc(0.5f * (1.f - om));
+        const T h = L::bc(R(0.5) * (R(1) - om));
         const T u = L::fma(h, S, t), v = L::fma(h, D, a);
         oa = L::add(u, v);
         ob = L::sub(u, v);
     }
 };
 
-template <int V>
-struct CellBgk<float, V, true, true> {
-    static constexpr bool PAIR = V % 2 == 0;
+template <class R, int V, bool SA>
+struct CellBgk {
+    static constexpr bool PAIR = sizeof(R) == 4 && V % 2 == 0;
     static constexpr int NP = PAIR ? V / 2 : V;  // lane sets
-    using T = typename std::conditional<PAIR, float2, float>::type;
-    float om;
-    LaneBgk<T> c[NP];
+    using T = typename std::conditional<PAIR, float2, R>::type;
+    LaneBgk<T, SA> c[NP];
     T orest[NP];
+    T S[NP][Q / 2], D[NP][Q / 2];
 
     template <int... I>
-    __device__ __forceinline__ CellBgk(float omega, std::integer_sequence<int, I...>)
-        : om(omega), c{((void)I, LaneBgk<T>(omega))...} {}
-    __device__ __forceinline__ explicit CellBgk(float omega) : CellBgk(omega, std::make_integer_sequence<int, NP>{}) {}
+    __device__ __forceinline__ CellBgk(R omega, R half_inv, std::integer_sequence<int, I...>)
+        : c{((void)I, LaneBgk<T, SA>(omega, half_inv))...} {}
+    __device__ __forceinline__ CellBgk(R omega, R half_inv) : CellBgk(omega, half_inv, std::make_integer_sequence<int, NP>{}) {}
 
-    static __device__ __forceinline__ T get(const float (&f)[V][Q], int p, int q) {
+    static __device__ __forceinline__ T get(const R (&f)[V][Q], int p, int q) {
         if constexpr (PAIR) return make_float2(f[2 * p][q], f[2 * p + 1][q]);
         else return f[p][q];
     }
-    static __device__ __forceinline__ void put(float (&o)[V], int p, T v) {
+    static __device__ __forceinline__ void put(R (&o)[V], int p, T v) {
         if constexpr (PAIR) {
             o[2 * p] = v.x;
             o[2 * p + 1] = v.y;
@@ -252,9 +193,7 @@ struct CellBgk<float, V, true, true> {
         }
     }
 
-    T S[NP][Q / 2], D[NP][Q / 2];
-
-    __device__ __forceinline__ void moments(const float (&f)[V][Q]) {
+    __device__ __forceinline__ void moments(const R (&f)[V][Q]) {
 #pragma unroll
         for (int p = 0; p < NP; ++p) {
             c[p].add_rest(get(f, p, 0));
@@ -271,19 +210,126 @@ struct CellBgk<float, V, true, true> {
     }
 
     // relaxed rest population of cell v (moments() computed it)
-    __device__ __forceinline__ float rest(const float (&)[V][Q], int v) const {
+    __device__ __forceinline__ R rest(const R (&)[V][Q], int v) const {
         if constexpr (PAIR) return (v & 1) ? orest[v / 2].y : orest[v / 2].x;
         else return orest[v];
     }
 
-    // relaxed populations q and q+1 = opp(q) (q odd) of every cell
-    __device__ __forceinline__ void pair(const float (&)[V][Q], int q, float (&oa)[V], float (&ob)[V]) {
+    // relaxed populations q and q+1 = opp(q) (q odd, ascending from 1) of every cell
+    __device__ __forceinline__ void pair(const R (&)[V][Q], int q, R (&oa)[V], R (&ob)[V]) {
 #pragma unroll
         for (int p = 0; p < NP; ++p) {
             T a, b;
             c[p].pair(q, S[p][q / 2], D[p][q / 2], a, b);
             put(oa, p, a);
             put(ob, p, b);
+        }
+    }
+};
+
+// ---- the relaxation of the 16-bit storages ------------------------------------------------------------
+// A state rounded to 16 bits after every step keeps the last bit of its relaxation: another order of the
+// same operations moves whole populations by 2^-11 (FP16) or 2^-8 (BF16) of their shift (2e-5 and 1e-4 of the
+// state's norm after 15 steps), so these storages keep one product chain per population, on pairs of cells:
+//   s = g0 + g1 + ... + g18, j = the signed sums in q order, rho = 1 + s, inv = 1/rho (IEEE), u = j inv
+//   t = ux ux + uy uy + uz uz (two FMAs), base = -1.5 t, feq0 = w0 (s + rho base)
+//   out0 = (1 - om) g0 + om feq0, and per odd q with a = c_q . u (two terms at most):
+//   sym = fma(om w, s, om w rho (4.5 a a + base)), asym = 3 om w rho a, out_q = (1 - om) g_q + (sym + asym),
+//   out_opp(q) = (1 - om) g_opp(q) + (sym - asym).
+template <int V>
+struct CellBgk16 {
+    static constexpr bool PAIR = V % 2 == 0;
+    static constexpr int NP = PAIR ? V / 2 : V;  // lanes
+    using T = typename std::conditional<PAIR, float2, float>::type;
+    using L = Lanes<T>;
+    float om, omc;
+    T s[NP], rho[NP], ux[NP], uy[NP], uz[NP], base[NP];
+    T owr1[NP], owr2[NP], owr3a[NP], owr3b[NP];
+    T orest[NP];
+
+    __device__ __forceinline__ explicit CellBgk16(float omega, float) : om(omega), omc(1.f - omega) {}
+
+    static __device__ __forceinline__ T get(const float (&f)[V][Q], int p, int q) {
+        if constexpr (PAIR) return make_float2(f[2 * p][q], f[2 * p + 1][q]);
+        else return f[p][q];
+    }
+    static __device__ __forceinline__ void put(float (&o)[V], int p, T v) {
+        if constexpr (PAIR) {
+            o[2 * p] = v.x;
+            o[2 * p + 1] = v.y;
+        } else {
+            o[p] = v;
+        }
+    }
+    // c_q . u for odd q (its first non-zero component is positive)
+    __device__ __forceinline__ T cdot_odd(int q, int p) const {
+        T a = cx(q) != 0 ? ux[p] : (cy(q) != 0 ? uy[p] : uz[p]);
+        if (cx(q) != 0 && cy(q) != 0) a = cy(q) > 0 ? L::add(a, uy[p]) : L::sub(a, uy[p]);
+        if ((cx(q) != 0 || cy(q) != 0) && cz(q) != 0) a = cz(q) > 0 ? L::add(a, uz[p]) : L::sub(a, uz[p]);
+        return a;
+    }
+
+    __device__ __forceinline__ void moments(const float (&f)[V][Q]) {
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+            T g[Q];
+#pragma unroll
+            for (int q = 0; q < Q; ++q) g[q] = get(f, p, q);
+            T sm = g[0];
+#pragma unroll
+            for (int q = 1; q < Q; ++q) sm = L::add(sm, g[q]);
+            // j in q order: a signed sum of the populations with that velocity component
+            constexpr int kx[10] = {1, 2, 7, 8, 9, 10, 11, 12, 13, 14}, ky[10] = {3, 4, 7, 8, 9, 10, 15, 16, 17, 18},
+                          kz[10] = {5, 6, 11, 12, 13, 14, 15, 16, 17, 18};
+            T jx = g[1], jy = g[3], jz = g[5];
+#pragma unroll
+            for (int i = 1; i < 10; ++i) {
+                jx = cx(kx[i]) > 0 ? L::add(jx, g[kx[i]]) : L::sub(jx, g[kx[i]]);
+                jy = cy(ky[i]) > 0 ? L::add(jy, g[ky[i]]) : L::sub(jy, g[ky[i]]);
+                jz = cz(kz[i]) > 0 ? L::add(jz, g[kz[i]]) : L::sub(jz, g[kz[i]]);
+            }
+            const T rh = L::add(L::bc(1.f), sm);
+            const T inv = L::rcp(rh);
+            s[p] = sm;
+            rho[p] = rh;
+            ux[p] = L::mul(jx, inv);
+            uy[p] = L::mul(jy, inv);
+            uz[p] = L::mul(jz, inv);
+            T t = L::mul(ux[p], ux[p]);
+            t = L::fma(uy[p], uy[p], t);
+            t = L::fma(uz[p], uz[p], t);
+            base[p] = L::mul(L::bc(-1.5f), t);
+            // the folded per-class terms and the rest population
+            const T feq0 = L::mul(L::bc(wf(0)), L::fma(rh, base[p], sm));
+            orest[p] = L::fma(L::bc(omc), g[0], L::mul(L::bc(om), feq0));
+            const T orho = L::mul(L::bc(om), rh);
+            owr1[p] = L::mul(orho, L::bc(wf(1)));
+            owr2[p] = L::mul(orho, L::bc(wf(7)));
+            owr3a[p] = L::mul(L::bc(3.f), owr1[p]);
+            owr3b[p] = L::mul(L::bc(3.f), owr2[p]);
+
+        }
+    }
+
+    // relaxed rest population of cell v (moments() computed it)
+    __device__ __forceinline__ float rest(const float (&)[V][Q], int v) const {
+        if constexpr (PAIR) return (v & 1) ? orest[v / 2].y : orest[v / 2].x;
+        else return orest[v];
+    }
+
+    // relaxed populations q and q+1 = opp(q) (q odd) of every cell
+    __device__ __forceinline__ void pair(const float (&f)[V][Q], int q, float (&oa)[V], float (&ob)[V]) const {
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+            const T a = cdot_odd(q, p);
+            const T owr = q < 7 ? owr1[p] : owr2[p];
+            const T t = L::mul(owr, L::fma(L::mul(L::bc(4.5f), a), a, base[p]));
+            // + omega w s as one FMA (a product by a broadcast constant then an add is not compiled
+            // alike in every kernel; an FMA is)
+            const T osym = L::fma(L::bc(om * wf(q)), s[p], t);
+            const T oasym = L::mul(q < 7 ? owr3a[p] : owr3b[p], a);
+            put(oa, p, L::fma(L::bc(omc), get(f, p, q), L::add(osym, oasym)));
+            put(ob, p, L::fma(L::bc(omc), get(f, p, q + 1), L::sub(osym, oasym)));
         }
     }
 };

@@ -12,19 +12,19 @@
 // three planes, 0 for two, -1 for one; the populations with c_x = c_y = 0 never leave their thread.
 // The next plane's loads are issued before the second step, whose arithmetic they fly across.
 //
-// Every cell goes through pair_unpack, LaneBgk and the rounding of its storage format exactly as in the
-// single step, in both of the two steps, so the two paths give the same bits.
+// Every cell goes through LaneBgk and the rounding of FP32 storage exactly as in the single step, in both of
+// the two steps, so the two paths give the same bits.
 //
-// What bounds it (N=256 FP32, ncu): 2.56 GB of DRAM traffic per pass (the populations once each way) at
-// 70 % of the copy rate; the rest is the alternation of its phases (loads, FP32 pipe, shared memory) at
-// 12 warps per SM, 39 % issue.  Measured per step, single / two in one pass: N=512 FP32 2917 / 1897 us
-// (46.0 / 70.8 GLUPS), N=256 367 / 256, N=128 51.0 / 35.3, N=96 21.0 / 18.4, N=64 8.2 / 8.2, N=32 6.1 / 4.1 (one
-// launch less per step).  16-bit at N=512 1497 / 1482 us, N=96 12.4 / 11.5, N=32 5.8 / 4.1: issue-bound both
-// ways, so there it pays for its launches on small cubes only.  Shapes measured and left: 512 threads (128 registers: spills, and
-// 155 KB of ring leave the loads in flight too little L1) 2315 us at N=512, 320 threads 2080, two CTAs of 256
-// or 192 threads (more halo) 2447 and 2262; planes staged by 16-byte cp.async in shared memory 2583; the two
-// steps on two groups of warps with named barriers 2866 (each plane's chain of load, relax and hand-over
-// is longer than its share of bandwidth).
+// What bounds it (N=256, ncu): 2.56 GB of DRAM traffic per pass (the populations once each way) at 70 % of the
+// copy rate; the rest is the alternation of its phases (loads, FP32 pipe, shared memory) at 12 warps per
+// SM, 39 % issue.  Measured per step, single / two in one pass: N=512 2915 / 1890 us (46.0 / 71.0 GLUPS), N=256
+// 367 / 256, N=128 51.1 / 35.4, N=96 21.0 / 18.4, N=64 8.2 / 8.2, N=32 6.2 / 4.1 (one launch less per step).  Shapes
+// measured and left: 512 threads (128 registers: spills, and 155 KB of ring leave the loads in flight too
+// little L1) 2315 us at N=512, 320 threads 2080, two CTAs of 256 or 192 threads (more halo) 2447 and 2262; a
+// ring one plane longer, with one barrier per plane, 2333; planes staged by 16-byte cp.async in shared memory
+// 2583; the two steps on two groups of warps with named barriers 2866 (each plane's chain of load, relax and
+// hand-over is longer than its share of bandwidth).  16-bit storage gains nothing (N=512 FP16 1588 to 1462 us in
+// the same forms, issue-bound, against 1507 for its single step).
 #include "kernels.h"
 #include "lattice.cuh"
 #include "uniform_common.cuh"
@@ -33,21 +33,12 @@
 
 namespace jp {
 
-// Threads of a CTA (pairs of cells of a tile plane with its halo).  FP32: 12 warps of 168 registers; the
-// ring leaves 156 KB of L1 for a plane's loads in flight.  16-bit: 14 warps of 128 registers.
-// deep: the ring holds one plane more of every class, so that the first step of the next plane never
-// overwrites what a second step still reads and one barrier per plane is enough (16-bit: N=512 FP16 1588 ->
-// 1513 us; in FP32 the longer ring takes the loads' L1: 2006 -> 2333 us).
-template <int ELEM> struct PairCfg;
-template <> struct PairCfg<4> {
-    static constexpr int NT = 384;
-    static constexpr bool deep = false;
-};
-template <> struct PairCfg<2> {
-    static constexpr int NT = 448;
-    static constexpr bool deep = true;
-};
-template <int ELEM> constexpr int pair_smem_bytes() { return (PairCfg<ELEM>::deep ? 48 : 32) * PairCfg<ELEM>::NT * 2 * ELEM; }
+// Threads of a CTA (pairs of cells of a tile plane with its halo): 12 warps of 168 registers; the ring leaves
+// 156 KB of L1 for a plane's loads in flight.
+constexpr int kPairThreads = 384;
+constexpr int kSlotBytes = kPairThreads * 8;      // one ring slot: a pair of floats per thread
+constexpr int kRing0 = 0, kRingP = 2 * 8 * kSlotBytes, kRingM = kRingP + 3 * 4 * kSlotBytes;  // c_z = 0, +1, -1
+constexpr int kPairSmem = kRingM + 4 * kSlotBytes;  // 32 slots, 96 KB
 
 // index of population q within its class of c_z (+1, 0, -1), ascending q; 0, 5 and 6 (c_x = c_y = 0) stay
 // in the thread's registers
@@ -62,7 +53,7 @@ struct PairSolve {
     void* dst;
     int n, tx, ty, ntx, ntiles, zc;
     int begin;  // first item of the cube in the launch
-    float omega;
+    float omega, half_inv;
 };
 template <int MAXB>
 struct PairBatch {
@@ -81,44 +72,16 @@ __device__ __forceinline__ uint2 lds_words(const char* p) {
     return v;
 }
 
-// The collision inputs of a pair's two cells from the words of population q.  FP32: one word per cell.
-// 16-bit: c_x = 0 the pair's word, else the two neighbouring pair words that the pulled cells straddle.
-template <class ST>
+// the collision inputs of a pair's two cells from the words of population q, and the relaxed values as stored
 __device__ __forceinline__ float2 pair_unpack(int q, unsigned w0, unsigned w1) {
-    if constexpr (sizeof(typename ST::raw) == 4) {
-        return __fadd2_rn(make_float2(__uint_as_float(w0), __uint_as_float(w1)), make_float2(-wgt<float>(q), -wgt<float>(q)));
-    } else {
-        const unsigned w = cx(q) == 0 ? w0 : __funnelshift_r(w0, w1, 16);
-        if constexpr (ST::id == 1) return __half22float2(*reinterpret_cast<const __half2*>(&w));
-        else return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w));
-    }
+    return __fadd2_rn(make_float2(__uint_as_float(w0), __uint_as_float(w1)), make_float2(-wf(q), -wf(q)));
 }
-// relaxed values as stored (FP32 shifts back by w_q)
-template <class ST>
-__device__ __forceinline__ Pack<typename ST::raw, 2> pair_pack(int q, float2 o) {
-    Pack<typename ST::raw, 2> pk;
-    if constexpr (sizeof(typename ST::raw) == 4) {
-        const float2 v = __fadd2_rn(o, make_float2(wgt<float>(q), wgt<float>(q)));
-        pk.v[0] = v.x;
-        pk.v[1] = v.y;
-    } else {
-        pk.u32[0] = ST::store2(o.x, o.y);
-    }
-    return pk;
-}
+__device__ __forceinline__ float2 pair_pack(int q, float2 o) { return __fadd2_rn(o, make_float2(wf(q), wf(q))); }
 
-template <class ST, int MAXB>
-__global__ void __launch_bounds__(PairCfg<sizeof(typename ST::raw)>::NT, 1)
-    k_stream_collide_pair(const __grid_constant__ PairBatch<MAXB> b) {
-    using raw = typename ST::raw;
-    using word = typename Pack<raw, 2>::word;
-    constexpr int E = (int)sizeof(raw);
-    constexpr int NT = PairCfg<E>::NT;
-    constexpr bool DEEP = PairCfg<E>::deep;
-    constexpr int SB = NT * 2 * E;                // bytes of one ring slot: a pair per thread
-    constexpr int N0 = DEEP ? 3 : 2, NP = DEEP ? 4 : 3;  // planes held of c_z = 0, +1 (and N0 - 1 of -1)
-    constexpr int B1 = N0 * 8 * SB, B2 = B1 + NP * 4 * SB;
-    extern __shared__ __align__(16) char ring[];  // [N0][8], [NP][4], [N0 - 1][4] slots
+template <int MAXB>
+__global__ void __launch_bounds__(kPairThreads, 1) k_stream_collide_pair(const __grid_constant__ PairBatch<MAXB> b) {
+    constexpr int NT = kPairThreads, SB = kSlotBytes;
+    extern __shared__ __align__(16) char ring[];
     const int t = threadIdx.x;
     for (int it = blockIdx.x; it < b.items; it += gridDim.x) {
         int si = 0;
@@ -131,8 +94,8 @@ __global__ void __launch_bounds__(PairCfg<sizeof(typename ST::raw)>::NT, 1)
         const int row = t / P, col = t - row * P;
         const bool active = row < d.ty + 2;
         const bool inner = row >= 1 && row < d.ty + 1 && col >= 1 && col < P - 1;
-        const raw* __restrict__ src = static_cast<const raw*>(d.src);
-        raw* __restrict__ dst = static_cast<raw*>(d.dst);
+        const float* __restrict__ src = static_cast<const float*>(d.src);
+        float* __restrict__ dst = static_cast<float*>(d.dst);
         const size_t qs = (size_t)n * n * n;
         const unsigned n2 = (unsigned)n * n;
         auto wrap = [n](int a) {
@@ -147,56 +110,46 @@ __global__ void __launch_bounds__(PairCfg<sizeof(typename ST::raw)>::NT, 1)
         const bool valid = inner && ox < n && oy < n;
         const unsigned row0 = (unsigned)gy * n, rowm = (unsigned)(gy == 0 ? n - 1 : gy - 1) * n,
                        rowp = (unsigned)(gy + 1 == n ? 0 : gy + 1) * n;
-        // FP32 pulls cells x-1 .. x+2, 16-bit the pairs at x-2, x, x+2
-        const unsigned xm = E == 4 ? (gx == 0 ? n - 1 : gx - 1) : (gx == 0 ? n - 2 : gx - 2);
-        const unsigned xp = gx + 2 == n ? 0 : gx + 2;
+        const unsigned xm = gx == 0 ? n - 1 : gx - 1, xp = gx + 2 == n ? 0 : gx + 2;
         unsigned a0[Q], a1[Q];
         auto load_plane = [&](int z) {
             const unsigned zo[3] = {(unsigned)(z == 0 ? n - 1 : z - 1) * n2, (unsigned)z * n2,
                                     (unsigned)(z + 1 == n ? 0 : z + 1) * n2};
 #pragma unroll
             for (int q = 0; q < Q; ++q) {
-                const raw* p = src + q * qs + zo[1 - cz(q)];
+                const float* p = src + q * qs + zo[1 - cz(q)];
                 const unsigned ro = cy(q) > 0 ? rowm : cy(q) < 0 ? rowp : row0;
                 auto one = [&](unsigned x) { return __ldg(reinterpret_cast<const unsigned*>(p + (ro + x))); };
                 if (cx(q) == 0) {
-                    if constexpr (E == 4) {
-                        const uint2 v = __ldg(reinterpret_cast<const uint2*>(p + (ro + gx)));
-                        a0[q] = v.x;
-                        a1[q] = v.y;
-                    } else {
-                        a0[q] = one(gx);
-                    }
-                } else if (cx(q) > 0) {
-                    a0[q] = one(xm);
-                    a1[q] = one(gx);
+                    const uint2 v = __ldg(reinterpret_cast<const uint2*>(p + (ro + gx)));
+                    a0[q] = v.x;
+                    a1[q] = v.y;
                 } else {
-                    a0[q] = one(E == 4 ? gx + 1 : gx);
-                    a1[q] = one(xp);
+                    a0[q] = cx(q) > 0 ? one(xm) : one(gx + 1);
+                    a1[q] = cx(q) > 0 ? one(gx) : one(xp);
                 }
             }
         };
         __syncthreads();  // the last item's reads of the ring are done
         if (active) load_plane(zs == 0 ? n - 1 : zs - 1);
-        word h0{}, h0n{}, h5{}, h5n{}, h5nn{}, h6{};  // own column: 0 of plane r - 1, 5 of r - 2, 6 of r
-        int s3 = 0;                                   // r mod 3
+        // own column, as stored: 0 of plane r - 1, 5 of r - 2, 6 of r
+        float2 h0{}, h0n{}, h5{}, h5n{}, h5nn{}, h6{};
+        int s3 = 0;                         // r mod 3
         for (int r = 0; r <= m + 1; ++r) {  // first step of plane zs - 1 + r, second of zs + r - 2
-            // slots: c_z = +1 written for r, read for r - 2; 0 for r and r - 1; -1 for r and r
-            const int wp = DEEP ? (r & 3) : s3, rp = DEEP ? ((r + 2) & 3) : (s3 == 2 ? 0 : s3 + 1);
-            const int w0 = DEEP ? s3 : (r & 1), rz = DEEP ? (s3 == 0 ? 2 : s3 - 1) : ((r & 1) ^ 1);
-            char* const wr0 = ring + w0 * 8 * SB;
-            char* const wr1 = ring + B1 + wp * 4 * SB;
-            char* const wr2 = ring + B2 + (DEEP ? (r & 1) : 0) * 4 * SB;
+            // slots: c_z = 0 written for r, read for r - 1; +1 for r and r - 2; -1 for r and r
+            char* const wr0 = ring + kRing0 + (r & 1) * 8 * SB;
+            char* const wr1 = ring + kRingP + s3 * 4 * SB;
+            char* const wr2 = ring + kRingM;
             if (active) {
                 float2 g[Q];
-                LaneBgk<float2> c(d.omega);
-                g[0] = pair_unpack<ST>(0, a0[0], a1[0]);
+                LaneBgk<float2, true> c(d.omega, d.half_inv);
+                g[0] = pair_unpack(0, a0[0], a1[0]);
                 c.add_rest(g[0]);
 #pragma unroll
                 for (int i = 0; i < Q / 2; ++i) {
                     const int q = sum_order(i);
-                    g[q] = pair_unpack<ST>(q, a0[q], a1[q]);
-                    g[q + 1] = pair_unpack<ST>(q + 1, a0[q + 1], a1[q + 1]);
+                    g[q] = pair_unpack(q, a0[q], a1[q]);
+                    g[q + 1] = pair_unpack(q + 1, a0[q + 1], a1[q + 1]);
                     c.add(q, g[q], g[q + 1]);
                 }
                 c.finish();
@@ -204,7 +157,7 @@ __global__ void __launch_bounds__(PairCfg<sizeof(typename ST::raw)>::NT, 1)
                 h5 = h5n;
                 h5n = h5nn;
                 auto put = [&](int q, float2 o) {
-                    const word w = pair_pack<ST>(q, o).w;
+                    const float2 w = pair_pack(q, o);
                     if (own_column(q)) {
                         if (q == 0) h0n = w;
                         else if (q == 5) h5nn = w;
@@ -212,17 +165,13 @@ __global__ void __launch_bounds__(PairCfg<sizeof(typename ST::raw)>::NT, 1)
                         return;
                     }
                     char* slot = (cz(q) == 0 ? wr0 : cz(q) > 0 ? wr1 : wr2) + zrank(q) * SB;
-                    if constexpr (E == 4) {
-                        // c_x != 0: the pairs' cells in two separate rows, which the shifted reads take
-                        // without bank conflicts
-                        if (cx(q) == 0) {
-                            reinterpret_cast<uint2*>(slot)[t] = w;
-                        } else {
-                            reinterpret_cast<unsigned*>(slot)[t] = w.x;
-                            reinterpret_cast<unsigned*>(slot)[NT + t] = w.y;
-                        }
+                    // c_x != 0: the pairs' cells in two separate rows, which the shifted reads take without
+                    // bank conflicts
+                    if (cx(q) == 0) {
+                        reinterpret_cast<float2*>(slot)[t] = w;
                     } else {
-                        reinterpret_cast<unsigned*>(slot)[t] = w;
+                        reinterpret_cast<float*>(slot)[t] = w.x;
+                        reinterpret_cast<float*>(slot)[NT + t] = w.y;
                     }
                 };
                 put(0, c.rest(g[0]));
@@ -235,84 +184,67 @@ __global__ void __launch_bounds__(PairCfg<sizeof(typename ST::raw)>::NT, 1)
                 }
                 if (r <= m) load_plane(zs + r == n ? 0 : zs + r);
             }
-            const bool second = r >= 2 && valid;
-            const char* const rd0 = ring + rz * 8 * SB;
-            const char* const rd1 = ring + B1 + rp * 4 * SB;
-            // the pulled pair of population q, from the first step's planes
-            auto get = [&](int q) -> float2 {
-                if (own_column(q)) {
-                    const word w = q == 0 ? h0 : q == 5 ? h5 : h6;
-                    if constexpr (E == 4) return pair_unpack<ST>(q, w.x, w.y);
-                    else return pair_unpack<ST>(q, w, 0);
-                }
-                const char* slot = (cz(q) == 0 ? rd0 : cz(q) > 0 ? rd1 : wr2) + zrank(q) * SB;
-                const int i = t - cy(q) * P;
-                if constexpr (E == 4) {
+            __syncthreads();
+            if (r >= 2 && valid) {
+                const char* const rd0 = ring + kRing0 + ((r & 1) ^ 1) * 8 * SB;
+                const char* const rd1 = ring + kRingP + (s3 == 2 ? 0 : s3 + 1) * 4 * SB;
+                // the pulled pair of population q, from the first step's planes
+                auto get = [&](int q) -> float2 {
+                    if (own_column(q)) {
+                        const float2 w = q == 0 ? h0 : q == 5 ? h5 : h6;
+                        return pair_unpack(q, __float_as_uint(w.x), __float_as_uint(w.y));
+                    }
+                    const char* slot = (cz(q) == 0 ? rd0 : cz(q) > 0 ? rd1 : wr2) + zrank(q) * SB;
+                    const int i = t - cy(q) * P;
                     if (cx(q) == 0) {
                         const uint2 v = lds_words(slot + i * 8);
-                        return pair_unpack<ST>(q, v.x, v.y);
+                        return pair_unpack(q, v.x, v.y);
                     }
-                    return cx(q) > 0 ? pair_unpack<ST>(q, lds_word(slot + (NT + i - 1) * 4), lds_word(slot + i * 4))
-                                     : pair_unpack<ST>(q, lds_word(slot + (NT + i) * 4), lds_word(slot + (i + 1) * 4));
-                } else {
-                    return cx(q) == 0  ? pair_unpack<ST>(q, lds_word(slot + i * 4), 0)
-                           : cx(q) > 0 ? pair_unpack<ST>(q, lds_word(slot + (i - 1) * 4), lds_word(slot + i * 4))
-                                       : pair_unpack<ST>(q, lds_word(slot + i * 4), lds_word(slot + (i + 1) * 4));
-                }
-            };
-            LaneBgk<float2> c(d.omega);
-            auto sum = [&](int i0, int i1) {
+                    return cx(q) > 0 ? pair_unpack(q, lds_word(slot + (NT + i - 1) * 4), lds_word(slot + i * 4))
+                                     : pair_unpack(q, lds_word(slot + (NT + i) * 4), lds_word(slot + (i + 1) * 4));
+                };
+                LaneBgk<float2, true> c(d.omega, d.half_inv);
+                c.add_rest(get(0));
 #pragma unroll
-                for (int i = i0; i < i1; ++i) {
+                for (int i = 0; i < Q / 2; ++i) {
                     const int q = sum_order(i);
                     float2 ga = get(q), gb = get(q + 1);
                     c.add(q, ga, gb);
                 }
-            };
-            // the c_z = 0 pairs were in the ring before this plane: summed ahead of the barrier when the
-            // ring is deep
-            if (DEEP && second) {
-                c.add_rest(get(0));
-                sum(0, 4);
-            }
-            __syncthreads();
-            if (second) {
-                if (!DEEP) {
-                    c.add_rest(get(0));
-                    sum(0, 4);
-                }
-                sum(4, Q / 2);
                 c.finish();
                 const unsigned o0 = (unsigned)(zs + r - 2) * n2 + row0 + gx;
-                st_pack<raw, 2>(dst + o0, pair_pack<ST>(0, c.rest(get(0))));
+                auto store = [&](int q, float2 o) {
+                    Pack<float, 2> pk;
+                    const float2 w = pair_pack(q, o);
+                    pk.v[0] = w.x;
+                    pk.v[1] = w.y;
+                    st_pack<float, 2>(dst + q * qs + o0, pk);
+                };
+                store(0, c.rest(get(0)));
 #pragma unroll
                 for (int q = 1; q < Q; q += 2) {
                     const float2 ga = get(q), gb = get(q + 1);
                     float2 oa, ob;
                     c.pair(q, __fadd2_rn(ga, gb), __fadd2_rn(ga, make_float2(-gb.x, -gb.y)), oa, ob);
-                    st_pack<raw, 2>(dst + q * qs + o0, pair_pack<ST>(q, oa));
-                    st_pack<raw, 2>(dst + (q + 1) * qs + o0, pair_pack<ST>(q + 1, ob));
+                    store(q, oa);
+                    store(q + 1, ob);
                 }
             }
-            if (!DEEP) __syncthreads();  // the second step has read what the next plane overwrites
+            __syncthreads();  // the second step has read what the next plane overwrites
             s3 = s3 == 2 ? 0 : s3 + 1;
         }
     }
 }
 
 // Time model of the plans, in microseconds per step.  A CTA walks its items' planes (chunk + 2 halo planes
-// each) and a plane takes plane_us whatever the tile's share of the threads: measured 2.4-2.6 us FP32 and
-// 2.2-2.3 us 16-bit for tiles of 56 to 128 cells along x at N=128..512, a third more for narrower tiles, whose
-// rows are mostly halo.
-static double plane_us(int storage, int tx) { return (storage == 0 ? 2.45 : 2.3) * (tx < 48 ? 1.33 : 1.0); }
-// The single step: 21.7 ps per cell FP32, 11.3 ps 16-bit where HBM sets its time, 5 us and 12 (7) ps per cell
-// where the state stays in L2 (measured N=32 6.1, N=48 6.2, N=64 8.2 us FP32).
-static double single_us(int storage, double cells) {
-    return std::max(cells * (storage == 0 ? 21.7e-6 : 11.3e-6), 5.0 + cells * (storage == 0 ? 12e-6 : 7e-6));
-}
-static bool pair_tile(int storage, int n, int tx, PairPlan& p) {
-    const int NT = storage == 0 ? PairCfg<4>::NT : PairCfg<2>::NT;
-    const int P = tx / 2 + 2, tymax = std::min(n, NT / P - 2);
+// each) and a plane takes plane_us whatever the tile's share of the threads: measured 2.4-2.6 us for tiles of 56
+// to 128 cells along x at N=128..512, a third more for narrower tiles, whose rows are mostly halo.
+static double plane_us(int tx) { return tx < 48 ? 3.26 : 2.45; }
+// The single step: 21.7 ps per cell where HBM sets its time, 5 us and 12 ps per cell where the state stays in
+// L2 (measured N=32 6.1, N=48 6.2, N=64 8.2 us).
+static double single_us(double cells) { return std::max(cells * 21.7e-6, 5.0 + cells * 12e-6); }
+static bool pair_tile(int n, int tx, PairPlan& p) {
+    const int P = tx / 2 + 2, tymax = std::min(n, kPairThreads / P - 2);
     if (tymax < 1) return false;
     const int nty = (n + tymax - 1) / tymax;
     p.tx = tx;
@@ -320,19 +252,17 @@ static bool pair_tile(int storage, int n, int tx, PairPlan& p) {
     p.tiles = (n + tx - 1) / tx * ((n + p.ty - 1) / p.ty);
     return true;
 }
-static int pair_align(int storage) { return storage == 0 ? 8 : 16; }  // x tiles start at 32-byte sectors
-static bool pair_ok(int storage, int n, int sms) {
-    return storage >= 0 && storage <= 2 && n >= 2 && n % 2 == 0 && n <= 1600 && sms > 0;
-}
+constexpr int kPairAlign = 8;  // x tiles start at 32-byte sectors
+// pairs of cells at even x need an even n; cell indices are 32-bit
+static bool pair_ok(int n, int sms) { return n >= 2 && n % 2 == 0 && n <= 1600 && sms > 0; }
 
 // One cube: every tile width, and the chunks that fill 1 to 16 rounds of CTAs.  The two-step pass is used where the model puts it 3 % ahead.
-PairPlan pair_plan(int storage, int n, int sms) {
+PairPlan pair_plan(int n, int sms) {
     PairPlan best{};
-    if (!pair_ok(storage, n, sms)) return best;
-    const int al = pair_align(storage);
-    for (int tx = al; tx <= 128 && tx < n + al; tx += al) {
+    if (!pair_ok(n, sms)) return best;
+    for (int tx = kPairAlign; tx <= 128 && tx < n + kPairAlign; tx += kPairAlign) {
         PairPlan p{};
-        if (!pair_tile(storage, n, tx, p)) break;
+        if (!pair_tile(n, tx, p)) break;
         int last = 0;
         for (int rounds = 1; rounds <= 16; ++rounds) {  // the shortest chunk that fits each number of rounds
             const int nzc = std::min((long long)n, (long long)rounds * sms / p.tiles);
@@ -340,35 +270,34 @@ PairPlan pair_plan(int storage, int n, int sms) {
             last = nzc;
             p.zc = (n + nzc - 1) / nzc;
             const long long items = (long long)p.tiles * ((n + p.zc - 1) / p.zc);
-            p.us = double((items + sms - 1) / sms) * (p.zc + 2) * plane_us(storage, tx) / 2;
+            p.us = double((items + sms - 1) / sms) * (p.zc + 2) * plane_us(tx) / 2;
             if (best.us == 0 || p.us < best.us) best = p;
         }
         if (best.us == 0) {  // more tiles than 16 rounds hold: whole columns
             p.zc = n;
-            p.us = double((p.tiles + sms - 1) / sms) * (n + 2) * plane_us(storage, tx) / 2;
+            p.us = double((p.tiles + sms - 1) / sms) * (n + 2) * plane_us(tx) / 2;
             best = p;
         }
     }
-    best.use = best.us < 0.97 * single_us(storage, double(n) * n * n);
+    best.use = best.us < 0.97 * single_us(double(n) * n * n);
     return best;
 }
 
 // In a launch of many cubes a cube takes the tile with the fewest CTA planes ...
-PairPlan pair_tile_plan(int storage, int n, int sms) {
+PairPlan pair_tile_plan(int n, int sms) {
     PairPlan best{};
-    if (!pair_ok(storage, n, sms)) return best;
-    const int al = pair_align(storage);
-    for (int tx = al; tx <= 128 && tx < n + al; tx += al) {
+    if (!pair_ok(n, sms)) return best;
+    for (int tx = kPairAlign; tx <= 128 && tx < n + kPairAlign; tx += kPairAlign) {
         PairPlan p{};
-        if (!pair_tile(storage, n, tx, p)) break;
-        p.us = p.tiles * plane_us(storage, tx);
+        if (!pair_tile(n, tx, p)) break;
+        p.us = p.tiles * plane_us(tx);
         if (best.us == 0 || p.us < best.us) best = p;
     }
     return best;
 }
 
 // ... and all of them one chunk length: the one with the least mean load of a CTA plus its longest item.
-bool pair_plan_batch(int storage, const int* n, int count, int sms, PairPlan* plans) {
+bool pair_plan_batch(const int* n, int count, int sms, PairPlan* plans) {
     double cells = 0, best = 0;
     int best_zc = 0;
     for (int i = 0; i < count; ++i) {
@@ -379,7 +308,7 @@ bool pair_plan_batch(int storage, const int* n, int count, int sms, PairPlan* pl
         double sum = 0, longest = 0;
         for (int i = 0; i < count; ++i) {
             const int nzc = (n[i] + zc - 1) / zc, z = (n[i] + nzc - 1) / nzc;
-            const double us = (z + 2) * plane_us(storage, plans[i].tx) / 2;
+            const double us = (z + 2) * plane_us(plans[i].tx) / 2;
             sum += double(plans[i].tiles) * ((n[i] + z - 1) / z) * us;
             longest = std::max(longest, us);
         }
@@ -393,15 +322,13 @@ bool pair_plan_batch(int storage, const int* n, int count, int sms, PairPlan* pl
         const int nzc = (n[i] + best_zc - 1) / best_zc;
         plans[i].zc = (n[i] + nzc - 1) / nzc;
     }
-    return best < 0.97 * single_us(storage, cells);
+    return best < 0.97 * single_us(cells);
 }
 
-template <class ST, int MAXB>
+template <int MAXB>
 static cudaError_t launch_pair_t(const UniSolve* u, const PairPlan* plans, int count, int sms, cudaStream_t st) {
-    constexpr int E = (int)sizeof(typename ST::raw);
-    auto kern = k_stream_collide_pair<ST, MAXB>;
-    const int smem = pair_smem_bytes<E>();
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    auto kern = k_stream_collide_pair<MAXB>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem);
     if (e != cudaSuccess) return e;
     PairBatch<MAXB> b;
     b.count = count;
@@ -409,13 +336,14 @@ static cudaError_t launch_pair_t(const UniSolve* u, const PairPlan* plans, int c
     for (int i = 0; i < count; ++i) {
         PairSolve& s = b.s[i];
         const PairPlan& p = plans[i];
-        if (p.tx <= 0 || p.tx % 2 || p.ty <= 0 || p.zc <= 0 || (p.tx / 2 + 2) * (p.ty + 2) > PairCfg<E>::NT ||
-            u[i].n < 2 || u[i].n % 2 || u[i].n > 1600)
+        if (p.tx <= 0 || p.tx % 2 || p.ty <= 0 || p.zc <= 0 || (p.tx / 2 + 2) * (p.ty + 2) > kPairThreads ||
+            !pair_ok(u[i].n, sms))
             return cudaErrorInvalidValue;
         s.src = u[i].src;
         s.dst = u[i].dst;
         s.n = u[i].n;
         s.omega = u[i].omega;
+        s.half_inv = u[i].half_inv;
         s.tx = p.tx;
         s.ty = p.ty;
         s.zc = p.zc;
@@ -424,26 +352,15 @@ static cudaError_t launch_pair_t(const UniSolve* u, const PairPlan* plans, int c
         s.begin = b.items;
         b.items += s.ntiles * ((s.n + p.zc - 1) / p.zc);
     }
-    kern<<<std::min(b.items, sms), PairCfg<E>::NT, smem, st>>>(b);
+    kern<<<std::min(b.items, sms), kPairThreads, kPairSmem, st>>>(b);
     note_launch();
     return cudaGetLastError();
 }
 
-template <class ST>
-static cudaError_t launch_pair(const UniSolve* u, const PairPlan* plans, int count, int sms, cudaStream_t st) {
-    return count == 1 ? launch_pair_t<ST, 1>(u, plans, count, sms, st) : launch_pair_t<ST, kMaxBatch>(u, plans, count, sms, st);
-}
-
-cudaError_t launch_stream_collide_pair(int storage, const UniSolve* solves, const PairPlan* plans, int count, int sms,
-                                       cudaStream_t st) {
+cudaError_t launch_stream_collide_pair(const UniSolve* solves, const PairPlan* plans, int count, int sms, cudaStream_t st) {
     if (count <= 0) return cudaSuccess;
     if (count > kMaxBatch || sms <= 0) return cudaErrorInvalidValue;
-    switch (storage) {
-        case 0: return launch_pair<StF32>(solves, plans, count, sms, st);
-        case 1: return launch_pair<StF16>(solves, plans, count, sms, st);
-        case 2: return launch_pair<StBF16>(solves, plans, count, sms, st);
-        default: return cudaErrorInvalidValue;
-    }
+    return count == 1 ? launch_pair_t<1>(solves, plans, count, sms, st) : launch_pair_t<kMaxBatch>(solves, plans, count, sms, st);
 }
 
 }  // namespace jp
