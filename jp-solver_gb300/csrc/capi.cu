@@ -45,42 +45,6 @@ size_t storage_bytes(int storage) {
     return 0;
 }
 
-// host-side conversion of one stored element to double (unshifted)
-double stored_to_double(int storage, const void* base, size_t idx, int q) {
-    switch (storage) {
-        case JP_FP32: return double(static_cast<const float*>(base)[idx]);
-        case JP_FP64: return static_cast<const double*>(base)[idx];
-        case JP_FP16: {
-            __half_raw r;
-            r.x = static_cast<const uint16_t*>(base)[idx];
-            return double(wf(q)) + double(__half2float(__half(r)));
-        }
-        case JP_BF16: {
-            __nv_bfloat16_raw r;
-            r.x = static_cast<const uint16_t*>(base)[idx];
-            return double(wf(q)) + double(__bfloat162float(__nv_bfloat16(r)));
-        }
-    }
-    return 0.0;
-}
-
-void double_to_stored(int storage, void* base, size_t idx, int q, double v) {
-    switch (storage) {
-        case JP_FP32: static_cast<float*>(base)[idx] = float(v); break;
-        case JP_FP64: static_cast<double*>(base)[idx] = v; break;
-        case JP_FP16: {
-            __half h = __float2half_rn(float(v - double(wf(q))));
-            static_cast<uint16_t*>(base)[idx] = __half_raw(h).x;
-            break;
-        }
-        case JP_BF16: {
-            __nv_bfloat16 h = __float2bfloat16_rn(float(v - double(wf(q))));
-            static_cast<uint16_t*>(base)[idx] = __nv_bfloat16_raw(h).x;
-            break;
-        }
-    }
-}
-
 }  // namespace jp
 
 using namespace jp;

@@ -75,10 +75,11 @@ bool vec_supported(int storage, int vec);
 cudaError_t launch_init_tgv(int storage, void* f, int n, double u0, double kf, double* axis_tab, cudaStream_t st,
                             bool aa = false);
 
-// Macroscopic field (rho, ux, uy, uz) per cell, linear (z*n+y)*n+x.  FP64 storage writes double4,
-// every other storage float4 (k_macro, src/tgv3d_uniform.cu:80-90).  layout: 0 flat [q][x]; 1, 2 the
+// Macroscopic field (rho, ux, uy, uz) per cell, linear (z*n+y)*n+x.  FP64 storage writes double4 (float4
+// when as_float), every other storage float4 (k_macro, src/tgv3d_uniform.cu:80-90).  layout: 0 flat [q][x]; 1, 2 the
 // in-place layouts after an even / odd step count (aa_layout()).
-cudaError_t launch_macro(int storage, const void* f, void* field, int n, cudaStream_t st, int layout = 0);
+cudaError_t launch_macro(int storage, const void* f, void* field, int n, cudaStream_t st, int layout = 0,
+                         bool as_float = false);
 
 // Energy, enstrophy, mass of a macro field, reduced deterministically to out_dev[3] (device).
 // partials_dev holds kDiagBlocks*3 doubles.  float_diff=true takes the velocity differences in

@@ -38,8 +38,6 @@ jp_status create_solver(const jp_config* cfg, cudaMemPool_t pool, jp_solver** ou
 cudaError_t wait_stream(jp_solver* s);
 // wait for an event without spinning on a core (yield, then sleep between polls)
 cudaError_t wait_event(cudaEvent_t ev);
-double stored_to_double(int storage, const void* base, size_t idx, int q);
-void double_to_stored(int storage, void* base, size_t idx, int q, double v);
 }  // namespace jp
 
 struct jp_solver {
@@ -70,6 +68,7 @@ struct jp_solver {
     jp::PairPlan pair{};       // two steps in one pass, where pair.use (uniform_pair.cu)
     jp::PairPlan pair_tile{};  // the same in a launch of many cubes
     int sms = 0;               // multiprocessors of the device
+    void* io = nullptr;        // population conversion scratch of an in-place cube, allocated on first use
     float* outbuf = nullptr;   // device Q / speed / velocity for output frames, allocated on first use
     // populations staged for the next step (jp_stage_populations): uploaded into `staging` on
     // copy_stream while the solver's stream works, swapped in as fa by the next step
@@ -86,6 +85,17 @@ struct jp_solver {
 };
 
 namespace jp {
+// How a host's population array maps onto a state (convert.cu): `units` contiguous runs of `len` values.
+struct PopMap {
+    enum Kind { LINEAR, FLAT, BLOCKED } kind;  // state in the host's order / a uniform cube's flat / blocked order
+    int n, mb, aa;                             // cube edge, block edge, state layout (jp_solver::aa_layout)
+    int len;                                   // a row of n cells (FLAT), else the mb^3 cells of a block's population
+    long long units;
+};
+// Convert all populations between `state` (the solver's storage) and `host` (dtype JP_F32 / JP_F64) through
+// the device scratch, in chunks of whole units; synchronous.
+jp_status convert_populations(jp_solver* s, int storage, int dtype, const PopMap& m, void* state, void* scratch,
+                              size_t scratch_bytes, void* host, bool to_host_order);
 // uniform (solver_uniform.cu)
 jp_status uniform_create(jp_solver* s);
 void uniform_free(jp_solver* s);
@@ -105,8 +115,6 @@ jp_status output_fields_from(jp_solver* s, const void* field, bool field_is_doub
 jp_status common_setup(jp_solver* s);
 // drop populations staged for the next step, after their copy has finished reading the host buffer
 jp_status uniform_discard_staged(jp_solver* s);
-// element of fa that holds population q of cell (x, y, z) at the current step count
-size_t uniform_slot(const jp_solver* s, int q, int x, int y, int z);
 // fa as stored <-> the flat [q][z][y][x] order of the two-array step (host copies; identity unless in place)
 void uniform_raw_to_flat(const jp_solver* s, const unsigned char* raw, unsigned char* flat);
 void uniform_flat_to_raw(const jp_solver* s, const unsigned char* flat, unsigned char* raw);

@@ -1336,15 +1336,7 @@ jp_status amr_get_populations(jp_solver* s, int level, int layout, int dtype, vo
         ACK(cudaStreamSynchronize(s->stream), "D2H");
         return JP_OK;
     }
-    std::vector<unsigned char> raw((size_t)count * a->elem);
-    ACK(cudaMemcpyAsync(raw.data(), p, raw.size(), cudaMemcpyDeviceToHost, s->stream), "D2H");
-    ACK(cudaStreamSynchronize(s->stream), "D2H");
-    for (int64_t i = 0; i < count; ++i) {
-        const double v = stored_to_double(a->storage, raw.data(), (size_t)i, int((i / a->MB3) % Q));
-        if (dtype == JP_F32) static_cast<float*>(host)[i] = float(v);
-        else static_cast<double*>(host)[i] = v;
-    }
-    return JP_OK;
+    return amr_convert(s, level, p, nb, dtype, host, true);
 }
 
 jp_status amr_set_populations(jp_solver* s, int level, int layout, int dtype, const void* host, int64_t count) {
@@ -1360,14 +1352,21 @@ jp_status amr_set_populations(jp_solver* s, int level, int layout, int dtype, co
         ACK(cudaStreamSynchronize(s->stream), "H2D");
         return JP_OK;
     }
-    std::vector<unsigned char> raw((size_t)count * a->elem);
-    for (int64_t i = 0; i < count; ++i) {
-        const double v = dtype == JP_F32 ? double(static_cast<const float*>(host)[i]) : static_cast<const double*>(host)[i];
-        double_to_stored(a->storage, raw.data(), (size_t)i, int((i / a->MB3) % Q), v);
-    }
-    ACK(cudaMemcpyAsync(p, raw.data(), raw.size(), cudaMemcpyHostToDevice, s->stream), "H2D");
-    ACK(cudaStreamSynchronize(s->stream), "H2D");
-    return JP_OK;
+// A level's populations in another type than the storage's, converted on the device through the level's
+// other array, which the next substep overwrites.
+static jp_status amr_convert(jp_solver* s, int level, void* p, long long nb, int dtype, void* host, bool to_host_order) {
+    AmrState* a = s->amr;
+    PopMap m{};
+    m.kind = PopMap::LINEAR;
+    m.mb = a->MB;
+    m.len = a->MB3;
+    m.units = nb * Q;
+    void* const scratch = level == 0 ? a->c0b : level == 1 ? a->f1b : a->f2b;
+    const long long cap = level == 0 ? a->cnb0 : level == 1 ? a->cap1 : a->cap2;
+    return convert_populations(s, a->storage, dtype, m, p, scratch, (size_t)cap * Q * a->MB3 * a->elem, host, to_host_order);
+}
+
+    return amr_convert(s, level, p, nb, dtype, const_cast<void*>(host), false);
 }
 
 // ---- state files (jp_save_state / jp_load_state) ---------------------------------------------------

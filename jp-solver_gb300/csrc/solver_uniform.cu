@@ -6,6 +6,7 @@
 #include "lattice.cuh"
 #include "solver.h"
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -129,6 +130,8 @@ void uniform_free(jp_solver* s) {
     dev_free(s, s->diag_dev);
     pinned_slot_free(s->diag_host);
     dev_free(s, s->outbuf);
+    dev_free(s, s->io);
+    s->io = nullptr;
     s->outbuf = nullptr;
     s->fa = s->fb = s->field = nullptr;
     s->partials = s->diag_dev = s->diag_host = nullptr;
@@ -274,15 +277,8 @@ jp_status uniform_diag(jp_solver* s, double out[3]) {
     return JP_OK;
 }
 
-// index of population q of cell (x,y,z) in the blocked layout [block][q][cell] of edge mb
-static inline size_t blocked_index(int n, int mb, int q, int x, int y, int z) {
-    const int gx = n / mb;
-    const size_t b = ((size_t)(z / mb) * gx + (y / mb)) * gx + (x / mb);
-    const size_t cell = ((size_t)(z % mb) * mb + (y % mb)) * mb + (x % mb);
-    return (b * Q + q) * (size_t)mb * mb * mb + cell;
-}
-
-size_t uniform_slot(const jp_solver* s, int q, int x, int y, int z) {
+// element of fa that holds population q of cell (x, y, z) at the current step count
+static size_t uniform_slot(const jp_solver* s, int q, int x, int y, int z) {
     const int n = s->n;
     if (s->inplace) {
         if (s->step_count & 1) {
@@ -326,6 +322,34 @@ void uniform_flat_to_raw(const jp_solver* s, const unsigned char* flat, unsigned
                                 flat + e * ((size_t)q * s->cells + ((size_t)z * n + y) * n + x), e);
 }
 
+// Populations in another type or order than the state's, converted on the device.  The scratch is the next
+// step's target array, whose contents nothing reads between steps; an in-place cube takes an allocation of
+// at most 64 MiB on first use.
+static jp_status uniform_convert(jp_solver* s, int layout, int dtype, void* host, bool to_host_order) {
+    PopMap m{};
+    m.n = s->n;
+    m.mb = s->cfg.mb;
+    m.aa = s->aa_layout();
+    if (layout == JP_LAYOUT_FLAT) {
+        m.kind = PopMap::FLAT;
+        m.len = s->n;
+        m.units = (long long)Q * s->n * s->n;
+    } else {
+        const long long g = s->n / m.mb;
+        m.kind = PopMap::BLOCKED;
+        m.len = m.mb * m.mb * m.mb;
+        m.units = Q * g * g * g;
+    }
+    void* scratch = s->fb;
+    size_t bytes = (size_t)Q * s->cells * s->elem;
+    if (s->inplace) {
+        bytes = std::min(bytes, (size_t)64 << 20);
+        if (!s->io) JP_CK(dev_alloc(s, &s->io, bytes), "cudaMalloc population scratch");
+        scratch = s->io;
+    }
+    return convert_populations(s, s->storage, dtype, m, s->fa, scratch, bytes, host, to_host_order);
+}
+
 jp_status uniform_get_populations(jp_solver* s, int level, int layout, int dtype, void* host, int64_t count) {
     if (level != 0) return fail(JP_ERR_INVALID, "uniform solver has only level 0");
     if (count != (int64_t)Q * s->cells) return fail(JP_ERR_INVALID, "count %lld != 19*n^3", (long long)count);
@@ -338,22 +362,7 @@ jp_status uniform_get_populations(jp_solver* s, int level, int layout, int dtype
         JP_CK(cudaStreamSynchronize(s->stream), "populations D2H");
         return JP_OK;
     }
-    std::vector<unsigned char> raw(bytes);
-    JP_CK(cudaMemcpyAsync(raw.data(), s->fa, bytes, cudaMemcpyDeviceToHost, s->stream), "populations D2H");
-    JP_CK(cudaStreamSynchronize(s->stream), "populations D2H");
-    const int n = s->n, mb = s->cfg.mb;
-    for (int q = 0; q < Q; ++q)
-        for (int z = 0; z < n; ++z)
-            for (int y = 0; y < n; ++y)
-                for (int x = 0; x < n; ++x) {
-                    const size_t src = uniform_slot(s, q, x, y, z);
-                    const size_t dst = layout == JP_LAYOUT_FLAT ? (size_t)q * s->cells + ((size_t)z * n + y) * n + x
-                                                                : blocked_index(n, mb, q, x, y, z);
-                    const double v = stored_to_double(s->storage, raw.data(), src, q);
-                    if (dtype == JP_F32) static_cast<float*>(host)[dst] = float(v);
-                    else static_cast<double*>(host)[dst] = v;
-                }
-    return JP_OK;
+    return uniform_convert(s, layout, dtype, host, true);
 }
 
 jp_status uniform_set_populations(jp_solver* s, int level, int layout, int dtype, const void* host, int64_t count) {
@@ -372,22 +381,7 @@ jp_status uniform_set_populations(jp_solver* s, int level, int layout, int dtype
         JP_CK(cudaMemcpyAsync(s->fa, host, bytes, cudaMemcpyHostToDevice, s->stream), "populations H2D");
         return JP_OK;
     }
-    std::vector<unsigned char> raw(bytes);
-    const int n = s->n, mb = s->cfg.mb;
-    for (int q = 0; q < Q; ++q)
-        for (int z = 0; z < n; ++z)
-            for (int y = 0; y < n; ++y)
-                for (int x = 0; x < n; ++x) {
-                    const size_t dst = uniform_slot(s, q, x, y, z);
-                    const size_t src = layout == JP_LAYOUT_FLAT ? (size_t)q * s->cells + ((size_t)z * n + y) * n + x
-                                                                : blocked_index(n, mb, q, x, y, z);
-                    const double v = dtype == JP_F32 ? double(static_cast<const float*>(host)[src])
-                                                     : static_cast<const double*>(host)[src];
-                    double_to_stored(s->storage, raw.data(), dst, q, v);
-                }
-    JP_CK(cudaMemcpyAsync(s->fa, raw.data(), bytes, cudaMemcpyHostToDevice, s->stream), "populations H2D");
-    JP_CK(cudaStreamSynchronize(s->stream), "populations H2D");
-    return JP_OK;
+    return uniform_convert(s, layout, dtype, const_cast<void*>(host), false);
 }
 
 // Q / speed / velocity of a device macro field of edge n, copied to host arrays of n^3 (vel: 3 n^3).
@@ -419,14 +413,7 @@ jp_status uniform_get_macro(jp_solver* s, float* host, int64_t count) {
     if (count != 4 * (int64_t)s->cells) return fail(JP_ERR_INVALID, "count %lld != 4*n^3", (long long)count);
     jp_status st = ensure_field(s);
     if (st != JP_OK) return st;
-    JP_CK(launch_macro(s->storage, s->fa, s->field, s->n, s->stream, s->aa_layout()), "macro");
-    if (s->storage == JP_FP64) {
-        std::vector<double> tmp((size_t)count);
-        JP_CK(cudaMemcpyAsync(tmp.data(), s->field, (size_t)count * 8, cudaMemcpyDeviceToHost, s->stream), "macro D2H");
-        JP_CK(cudaStreamSynchronize(s->stream), "macro D2H");
-        for (int64_t i = 0; i < count; ++i) host[i] = float(tmp[(size_t)i]);
-        return JP_OK;
-    }
+    JP_CK(launch_macro(s->storage, s->fa, s->field, s->n, s->stream, s->aa_layout(), true), "macro");
     JP_CK(cudaMemcpyAsync(host, s->field, (size_t)count * 4, cudaMemcpyDeviceToHost, s->stream), "macro D2H");
     JP_CK(cudaStreamSynchronize(s->stream), "macro D2H");
     return JP_OK;

@@ -323,14 +323,17 @@ __global__ void k_macro(const typename ST::raw* __restrict__ f, FT* __restrict__
     o[3] = FT(uz);
 }
 
-cudaError_t launch_macro(int storage, const void* f, void* field, int n, cudaStream_t st, int layout) {
+cudaError_t launch_macro(int storage, const void* f, void* field, int n, cudaStream_t st, int layout, bool as_float) {
     const long long cells = (long long)n * n * n;
     const unsigned blocks = (unsigned)((cells + 255) / 256);
     switch (storage) {
         case 0: k_macro<StF32, float><<<blocks, 256, 0, st>>>((const float*)f, (float*)field, n, layout); break;
         case 1: k_macro<StF16, float><<<blocks, 256, 0, st>>>((const uint16_t*)f, (float*)field, n, layout); break;
         case 2: k_macro<StBF16, float><<<blocks, 256, 0, st>>>((const uint16_t*)f, (float*)field, n, layout); break;
-        case 3: k_macro<StF64, double><<<blocks, 256, 0, st>>>((const double*)f, (double*)field, n, layout); break;
+        case 3:
+            if (as_float) k_macro<StF64, float><<<blocks, 256, 0, st>>>((const double*)f, (float*)field, n, layout);
+            else k_macro<StF64, double><<<blocks, 256, 0, st>>>((const double*)f, (double*)field, n, layout);
+            break;
         default: return cudaErrorInvalidValue;
     }
     note_launch();
