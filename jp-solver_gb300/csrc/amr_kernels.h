@@ -56,6 +56,16 @@ struct AmrLaunch {
     double u0 = 0.0, kf = 0.0;
 };
 
+// The block tables of a grid that the diagnostics walk.
+struct AmrGrid {
+    const int *ref0, *ref1, *f1pos, *l1grid, *fof1, *l2pl1, *l2oct;
+    int cgx, l1gx, cnb0, nf1, nf2, N2;
+};
+// Energy, enstrophy and mass of the state into out[3] (device): macro holds the leaf blocks' values, 16 bytes
+// for each of the (cnb0 + nf1 + nf2) mb^3 cells; partials as launch_diag_field (amr_diag.cu).
+cudaError_t launch_amr_diag(int storage, int mb, const AmrGrid& g, const void* c0, const void* f1, const void* f2,
+                            void* macro, double* partials, double* out, cudaStream_t st);
+
 // One member of a batched launch: the fields of AmrLaunch a per-block stage reads, and the first
 // CTA of the member in the batched grid (members follow each other; a member gets as many CTAs as
 // its single launch would).

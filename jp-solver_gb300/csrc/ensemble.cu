@@ -350,8 +350,7 @@ long long estimate_bytes(const jp_config& c) {
     const long long cap2 = 8 * cap_nref1;
     const long long elem = c.storage == JP_FP32 ? 4 : 2;
     const long long blk = Qn * mb3 * elem, gh = Qn * sh * elem;
-    const long long n2 = 4 * n;
-    return 3 * cnb0 * blk + cap1 * (3 * blk + gh) + cap2 * (2 * blk + gh) + 16 * n2 * n2 * n2 + (8 << 20);
+    return 3 * cnb0 * blk + cap1 * (3 * blk + gh) + cap2 * (2 * blk + gh) + 16 * (cnb0 + cap1 + cap2) * mb3 + (8 << 20);
 }
 
 }  // namespace

@@ -93,6 +93,9 @@ inline int* diag_err_word(double* partials) { return reinterpret_cast<int*>(part
 cudaError_t launch_diag_field(bool field_is_double, bool float_diff, const void* field, int n,
                               double* partials_dev, double* out_dev, cudaStream_t st);
 
+// sum of `nparts` partial triples in a fixed order, scaled by inv_cells, into out_dev[3]
+cudaError_t launch_diag_finish(const double* partials_dev, int nparts, double inv_cells, double* out_dev, cudaStream_t st);
+
 // Energy, enstrophy, mass of a float-storage cube (storage 0 FP32, 1 FP16, 2 BF16) straight from its
 // populations f in layout 0 / 1 / 2 (as launch_macro), with no macro field: the per-cell terms of
 // launch_macro + launch_diag_field(float_diff=true), summed another way (double-float partials in a

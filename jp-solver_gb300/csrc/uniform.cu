@@ -812,4 +812,10 @@ cudaError_t launch_diag_field(bool field_is_double, bool float_diff, const void*
     return cudaGetLastError();
 }
 
+cudaError_t launch_diag_finish(const double* partials_dev, int nparts, double inv_cells, double* out_dev, cudaStream_t st) {
+    k_diag_finish<<<1, 256, 0, st>>>(partials_dev, nparts, inv_cells, out_dev);
+    note_launch();
+    return cudaGetLastError();
+}
+
 }  // namespace jp
