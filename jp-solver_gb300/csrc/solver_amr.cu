@@ -63,9 +63,9 @@ struct AmrState {
     int* step_cnt_host = nullptr;  // pinned staging of the upload
     // captured base_step graphs, one per combination of the ping-pong parities of the three levels
     // (a coarse step swaps level 0 once and the fine levels an even number of times; a regrid's
-    // seeding swaps a fine level once).  Dropped only when buffers move (pool growth, new initial
-    // build) or the launch shape changes.
-    cudaGraphExec_t graph[8] = {};
+    // seeding swaps a fine level once) and of whether there is a level 2.  Dropped only when buffers
+    // move (pool growth, new initial build) or the launch shape changes.
+    cudaGraphExec_t graph[16] = {};
     float *c0_home = nullptr, *f1_home = nullptr, *f2_home = nullptr;
     AmrFork fk;  // a coarse step's level-0 chain runs on fk.side, beside the first level-2 pair (base_step)
 };
@@ -667,20 +667,26 @@ static jp_status base_step(jp_solver* s) {
     // restrictions fused into the last substep of each fine level (same values, one pass less)
     const bool fuse = !skip_restrict && can_fuse_restrict(a->MB);
     const int* cnt = a->step_cnt;
-    ACK(cudaEventRecord(a->fk.fork, s->stream), "fork");
-    ACK(cudaStreamWaitEvent(a->fk.side, a->fk.fork, 0), "fork");
-    const jp_status st0 = level0_chain(s, a->fk.side);
-    ACK(cudaEventRecord(a->fk.join, a->fk.side), "join");
-    JoinOnExit join{s->stream, a->fk.join};
+    // Without level-2 blocks (the host knows the grid) the step is the level-0 chain and two level-1 substeps, in
+    // one stream: eight launches over nothing and four events less.  Per coarse step, with / without them: N0=16
+    // graph 26.7 / 23.5 us, N0=48 FP16 direct launches 81.7 / 66 us.
+    const bool l2 = a->nf2 > 0;
+    if (l2) {
+        ACK(cudaEventRecord(a->fk.fork, s->stream), "fork");
+        ACK(cudaStreamWaitEvent(a->fk.side, a->fk.fork, 0), "fork");
+    }
+    const jp_status st0 = level0_chain(s, l2 ? a->fk.side : s->stream);
+    if (l2) ACK(cudaEventRecord(a->fk.join, a->fk.side), "join");
+    JoinOnExit join{s->stream, a->fk.join, l2};
     TRY(st0);
     // The first level-1 substep in two parts: its skin blocks (the only ones the next level-2 pair
     // reads, through the prep cells, and the only ones that pair restricts into), then the others on
     // the side branch, beside the whole second level-2 pair; they join before the last level-1
     // substep.  Each block is stepped as in one launch (rows mapping).
-    const bool split = a->MB >= 8 && (a->vec ? a->vec : default_step_vec(a->MB)) == 4;
+    const bool split = l2 && a->MB >= 8 && (a->vec ? a->vec : default_step_vec(a->MB)) == 4;
     JoinOnExit join2{s->stream, a->fk.join2, false};
     for (int s1 = 0; s1 < 2; ++s1) {
-        if (!skip_prep) {
+        if (l2 && !skip_prep) {
             AmrLaunch L;
             L.nblocks = interface_cells(a->MB) * a->cap1;
             L.nlim = cnt + SC_PREP1;
@@ -704,7 +710,7 @@ static jp_status base_step(jp_solver* s) {
             F.n1 = a->N1;
             TRY(launch(s, OP_FILL_L2, F));
         }
-        for (int s2 = 0; s2 < 2; ++s2) {
+        for (int s2 = 0; l2 && s2 < 2; ++s2) {
             AmrLaunch S;
             S.nblocks = a->cap2;
             S.nlim = cnt + SC_NF2;
@@ -724,7 +730,7 @@ static jp_status base_step(jp_solver* s) {
             TRY(launch(s, OP_STEP_L2, S));
             std::swap(a->f2a, a->f2b);
         }
-        if (!skip_restrict && !fuse) {
+        if (l2 && !skip_restrict && !fuse) {
             AmrLaunch R;
             R.nblocks = (a->cap2 + 7) / 8;
             R.nlim = cnt + SC_NREF1;
@@ -735,7 +741,7 @@ static jp_status base_step(jp_solver* s) {
             R.scale = float(a->nqi21);
             TRY(launch(s, OP_RESTRICT, R));
         }
-        if (s1 == 0) TRY(join.now());
+        if (join.pending) TRY(join.now());
         if (s1 == 1 && join2.pending) TRY(join2.now());
         AmrLaunch S;
         S.nblocks = a->cap1;
@@ -816,7 +822,11 @@ jp_status amr_batch_step(const std::vector<jp_solver*>& ms, cudaStream_t st, con
     };
     auto run = [&](int op, bool fused, auto fill) { return run_on(st, op, fused, fill); };
     // the level-0 chain, on the side stream when there is one (base_step: it shares no array with
-    // the first level-2 pair and joins before the first level-1 substep)
+    // the first level-2 pair and joins before the first level-1 substep); with no level 2 anywhere
+    // there is nothing beside it
+    bool l2 = false;
+    for (const jp_solver* m : ms) l2 = l2 || m->amr->nf2 > 0;
+    if (!l2) fk = nullptr;
     const cudaStream_t s0 = fk ? fk->side : st;
     if (fk) {
         ACK(cudaEventRecord(fk->fork, st), "fork");
@@ -858,8 +868,9 @@ jp_status amr_batch_step(const std::vector<jp_solver*>& ms, cudaStream_t st, con
     JoinOnExit join{st, fk ? fk->join : nullptr, fk != nullptr};
     TRY(st0);
     for (int s1 = 0; s1 < 2; ++s1) {
-        if (!skip_prep) {
+        if (l2 && !skip_prep) {
             TRY(run(OP_PREP, false, [](AmrState* a, AmrItem& it) {
+                if (a->nf2 == 0) return 0;
                 it.in = a->f1a;
                 it.out = a->prep1;
                 it.list = a->pc1;
@@ -869,6 +880,7 @@ jp_status amr_batch_step(const std::vector<jp_solver*>& ms, cudaStream_t st, con
                 return std::min((interface_cells(a->MB) * a->cap1 + 255) / 256, kBatchPrepCtas);
             }));
             TRY(run(OP_FILL_L2, false, [](AmrState* a, AmrItem& it) {
+                if (a->nf2 == 0) return 0;
                 it.in = a->prep1;
                 it.out = a->gh2;
                 it.t0 = a->l2pl1;
@@ -882,7 +894,7 @@ jp_status amr_batch_step(const std::vector<jp_solver*>& ms, cudaStream_t st, con
                 return std::min((a->SH * a->cap2 + 255) / 256, kBatchPrepCtas);
             }));
         }
-        for (int s2 = 0; s2 < 2; ++s2) {
+        for (int s2 = 0; l2 && s2 < 2; ++s2) {
             const bool f = s2 == 1 && fuse;  // last level-2 substep restricts itself into level 1
             TRY(run(OP_STEP_L2, f, [f](AmrState* a, AmrItem& it) {
                 it.in = a->f2a;
@@ -897,11 +909,11 @@ jp_status amr_batch_step(const std::vector<jp_solver*>& ms, cudaStream_t st, con
                     it.out2 = a->f1a;
                     it.scale = float(a->nqi21);
                 }
-                return a->cap2;
+                return a->nf2;
             }));
             for (jp_solver* m : ms) std::swap(m->amr->f2a, m->amr->f2b);
         }
-        if (!skip_restrict && !fuse) {
+        if (l2 && !skip_restrict && !fuse) {
             TRY(run(OP_RESTRICT, false, [](AmrState* a, AmrItem& it) {
                 it.out = a->f1a;
                 it.in = a->f2a;
@@ -909,7 +921,7 @@ jp_status amr_batch_step(const std::vector<jp_solver*>& ms, cudaStream_t st, con
                 it.t0 = a->fof1;
                 it.scale = float(a->nqi21);
                 it.nlim = a->step_cnt + SC_NREF1;
-                return (a->cap2 + 7) / 8;
+                return (a->nf2 + 7) / 8;
             }));
         }
         if (s1 == 0 && join.pending) TRY(join.now());
@@ -927,7 +939,7 @@ jp_status amr_batch_step(const std::vector<jp_solver*>& ms, cudaStream_t st, con
                 it.out2 = a->c0a;
                 it.scale = float(a->nqi10);
             }
-            return a->cap1;
+            return a->nf1;
         }));
         for (jp_solver* m : ms) std::swap(m->amr->f1a, m->amr->f1b);
     }
@@ -939,7 +951,7 @@ jp_status amr_batch_step(const std::vector<jp_solver*>& ms, cudaStream_t st, con
             it.t0 = a->fof0;
             it.scale = float(a->nqi10);
             it.nlim = a->step_cnt + SC_NREF0;
-            return (a->cap1 + 7) / 8;
+            return (a->nf1 + 7) / 8;
         }));
     }
     for (jp_solver* m : ms) ++m->step_count;
@@ -1043,7 +1055,8 @@ bool amr_batch_compatible(const jp_solver* a, const jp_solver* b) {
 // base_step replayed from a captured graph (captured on first use for each parity combination)
 static jp_status graph_step(jp_solver* s, cudaStream_t on = nullptr) {
     AmrState* a = s->amr;
-    const int key = (a->c0a == a->c0_home ? 0 : 1) | (a->f1a == a->f1_home ? 0 : 2) | (a->f2a == a->f2_home ? 0 : 4);
+    const int key = (a->c0a == a->c0_home ? 0 : 1) | (a->f1a == a->f1_home ? 0 : 2) | (a->f2a == a->f2_home ? 0 : 4) |
+                    (a->nf2 > 0 ? 0 : 8);
     if (!a->graph[key]) {
         float *c0a = a->c0a, *c0b = a->c0b, *f1a = a->f1a, *f1b = a->f1b, *f2a = a->f2a, *f2b = a->f2b;
         ACK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal), "begin capture");
@@ -1347,6 +1360,20 @@ jp_status amr_population_count(const jp_solver* s, int level, int64_t* count) {
 
 // Populations cross the boundary as unshifted values in the blocked layout [blk][q][MB^3]
 // (FP32 storage read as float: the stored bits; shifted formats converted, f = w_q + g).
+// A level's populations in another type than the storage's, converted on the device through the level's
+// other array, which the next substep overwrites.
+static jp_status amr_convert(jp_solver* s, int level, void* p, long long nb, int dtype, void* host, bool to_host_order) {
+    AmrState* a = s->amr;
+    PopMap m{};
+    m.kind = PopMap::LINEAR;
+    m.mb = a->MB;
+    m.len = a->MB3;
+    m.units = nb * Q;
+    void* const scratch = level == 0 ? a->c0b : level == 1 ? a->f1b : a->f2b;
+    const long long cap = level == 0 ? a->cnb0 : level == 1 ? a->cap1 : a->cap2;
+    return convert_populations(s, a->storage, dtype, m, p, scratch, (size_t)cap * Q * a->MB3 * a->elem, host, to_host_order);
+}
+
 jp_status amr_get_populations(jp_solver* s, int level, int layout, int dtype, void* host, int64_t count) {
     AmrState* a = s->amr;
     long long nb;
@@ -1376,20 +1403,6 @@ jp_status amr_set_populations(jp_solver* s, int level, int layout, int dtype, co
         ACK(cudaStreamSynchronize(s->stream), "H2D");
         return JP_OK;
     }
-// A level's populations in another type than the storage's, converted on the device through the level's
-// other array, which the next substep overwrites.
-static jp_status amr_convert(jp_solver* s, int level, void* p, long long nb, int dtype, void* host, bool to_host_order) {
-    AmrState* a = s->amr;
-    PopMap m{};
-    m.kind = PopMap::LINEAR;
-    m.mb = a->MB;
-    m.len = a->MB3;
-    m.units = nb * Q;
-    void* const scratch = level == 0 ? a->c0b : level == 1 ? a->f1b : a->f2b;
-    const long long cap = level == 0 ? a->cnb0 : level == 1 ? a->cap1 : a->cap2;
-    return convert_populations(s, a->storage, dtype, m, p, scratch, (size_t)cap * Q * a->MB3 * a->elem, host, to_host_order);
-}
-
     return amr_convert(s, level, p, nb, dtype, const_cast<void*>(host), false);
 }
 
