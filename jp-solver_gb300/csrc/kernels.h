@@ -88,7 +88,8 @@ cudaError_t launch_macro(int storage, const void* f, void* field, int n, cudaStr
 // be 16-byte aligned (every solver's own field is).
 constexpr int kDiagBlocks = 1216;   // 152 SMs x 8
 constexpr int kDiagThreads = 256;
-constexpr int kDiagPartials = kDiagBlocks * 3 + 1;  // block partials + the error word of launch_diag_pop
+// block partials + launch_diag_pop's error word and count of finished CTAs (both zero between launches)
+constexpr int kDiagPartials = kDiagBlocks * 3 + 1;
 inline int* diag_err_word(double* partials) { return reinterpret_cast<int*>(partials + kDiagBlocks * 3); }
 cudaError_t launch_diag_field(bool field_is_double, bool float_diff, const void* field, int n,
                               double* partials_dev, double* out_dev, cudaStream_t st);
@@ -101,9 +102,10 @@ cudaError_t launch_diag_finish(const double* partials_dev, int nparts, double in
 // launch_macro + launch_diag_field(float_diff=true), summed another way (double-float partials in a
 // fixed order) to ~1e-13 of the result.
 // Cubes it takes: even n (pairs of cells), n <= 1600 (32-bit cell indices).  partials_dev holds
-// kDiagPartials doubles: the last is the kernel's error word (zero when allocated; set if a bounded
-// wait between its warps gave up, cleared by the launch's final sum, which copies it to *flag_out
-// when flag_out is given and then writes NaN diagnostics).
+// kDiagPartials doubles: the last is the kernel's error word and its count of finished CTAs (zero when
+// allocated; the error word is set if a bounded wait between its warps gave up, and cleared by the launch's
+// final sum, which copies it to *flag_out when flag_out is given and then writes NaN diagnostics).
+// out_dev and flag_out may be pinned host memory.
 cudaError_t launch_diag_pop(int storage, int layout, const void* f, int n, double* partials_dev, double* out_dev,
                             double* flag_out, cudaStream_t st);
 inline bool diag_pop_ok(int storage, int n) { return storage >= 0 && storage <= 2 && n % 2 == 0 && n <= 1600; }

@@ -62,8 +62,7 @@ struct jp_solver {
     bool inplace = false;      // JP_FLAG_INPLACE: one array, AA steps (uniform_aa.cu)
     void* field = nullptr;     // macro field (float4 or double4 per cell), allocated on first use
     double* partials = nullptr;  // diagnostic block partials + error word (kDiagPartials)
-    double* diag_dev = nullptr;  // 3 doubles (+ the error word's copy, uniform)
-    double* diag_host = nullptr; // 4 doubles, pinned
+    double* diag_host = nullptr; // 3 doubles (+ the error word's copy, uniform), pinned: the kernels write it
     int vec = 0, tpb = 0;
     jp::PairPlan pair{};       // two steps in one pass, where pair.use (uniform_pair.cu)
     jp::PairPlan pair_tile{};  // the same in a launch of many cubes

@@ -1183,7 +1183,6 @@ jp_status amr_create(jp_solver* s) {
     s->diag_host = (double*)pinned_slot_alloc();
     if (!a->cnt_host || !s->diag_host) return fail(JP_ERR_NOMEM, "pinned host slot");
     ACK(dev_alloc(s, (void**)&s->partials, sizeof(double) * kDiagPartials), "cudaMalloc partials");
-    ACK(dev_alloc(s, (void**)&s->diag_dev, sizeof(double) * 3), "cudaMalloc diag");
     ACK(a->fk.create(s->stream), "side stream");
     ACK(cudaMemsetAsync(a->fof1, 0xFF, sizeof(int) * a->cap1, s->stream), "memset");
     ACK(cudaMemsetAsync(a->ref1, 0, sizeof(int) * a->cap1, s->stream), "memset");
@@ -1287,7 +1286,8 @@ static jp_status ensure_macro(jp_solver* s) {
     return dalloc(a, &a->macro, 4 * ((size_t)a->cnb0 + a->cap1 + a->cap2) * a->MB3, "cudaMalloc leaf macro values");
 }
 
-static jp_status launch_diag(jp_solver* s, cudaStream_t st) {
+// out[3]: device or pinned host memory
+static jp_status launch_diag(jp_solver* s, cudaStream_t st, double* out) {
     AmrState* a = s->amr;
     AmrGrid g{};
     g.ref0 = a->ref0;
@@ -1303,7 +1303,7 @@ static jp_status launch_diag(jp_solver* s, cudaStream_t st) {
     g.nf1 = a->nf1;
     g.nf2 = a->nf2;
     g.N2 = a->N2;
-    ACK(launch_amr_diag(a->storage, a->MB, g, a->c0a, a->f1a, a->f2a, a->macro, s->partials, s->diag_dev, st), "diag");
+    ACK(launch_amr_diag(a->storage, a->MB, g, a->c0a, a->f1a, a->f2a, a->macro, s->partials, out, st), "diag");
     return JP_OK;
 }
 
@@ -1316,9 +1316,7 @@ jp_status amr_prepare_diag(jp_solver* s) {
 // the diagnostics of the current state on another stream, into pinned host_out[3]; buffers prepared before
 jp_status amr_diag_async(jp_solver* s, cudaStream_t st, double* host_out) {
     if (!s->amr->macro) return fail(JP_ERR_STATE, "amr_diag_async: buffers not prepared");
-    TRY(launch_diag(s, st));
-    ACK(cudaMemcpyAsync(host_out, s->diag_dev, 3 * sizeof(double), cudaMemcpyDeviceToHost, st), "diag D2H");
-    return JP_OK;
+    return launch_diag(s, st, host_out);
 }
 
 jp_status amr_diag(jp_solver* s, double out[3]) {
@@ -1328,12 +1326,11 @@ jp_status amr_diag(jp_solver* s, double out[3]) {
     // leaves, 1087 and 222).
     if ((double)a->nf2 * a->MB3 > 0.9 * (double)a->N2 * a->N2 * a->N2) {
         TRY(composite(s));
-        ACK(launch_diag_field(false, false, a->field, a->N2, s->partials, s->diag_dev, s->stream), "diag");
+        ACK(launch_diag_field(false, false, a->field, a->N2, s->partials, s->diag_host, s->stream), "diag");
     } else {
         TRY(ensure_macro(s));
-        TRY(launch_diag(s, s->stream));
+        TRY(launch_diag(s, s->stream, s->diag_host));
     }
-    ACK(cudaMemcpyAsync(s->diag_host, s->diag_dev, 3 * sizeof(double), cudaMemcpyDeviceToHost, s->stream), "diag D2H");
     ACK(wait_stream(s), "diag");
     out[0] = s->diag_host[0];
     out[1] = s->diag_host[1];

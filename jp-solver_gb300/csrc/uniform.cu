@@ -410,35 +410,35 @@ __global__ void __launch_bounds__(kDiagThreads) k_diag_field(const FT* __restric
     }
 }
 
-// Sum `nparts` partial triples in a fixed order and scale by 1/cells.  err (optional): the error word
-// of the kernel that wrote the partials, copied to *flag_out (when given) and cleared for the next one.
-__global__ void __launch_bounds__(256) k_diag_finish(const double* __restrict__ partials, int nparts,
-                                                     double inv_cells, double* __restrict__ out,
-                                                     int* __restrict__ err = nullptr,
-                                                     double* __restrict__ flag_out = nullptr) {
-    double a[3] = {0.0, 0.0, 0.0};
-    for (int p = threadIdx.x; p < nparts; p += 256) {
-        a[0] += partials[p * 3 + 0];
-        a[1] += partials[p * 3 + 1];
-        a[2] += partials[p * 3 + 2];
-    }
+// Sum `nparts` partial triples in a fixed order and scale by 1/cells: the CTA's first 256 threads, every thread
+// of the CTA calls it.  `volatile`: the partials may come from other CTAs of the same launch.
+__device__ __forceinline__ void diag_total(const volatile double* partials, int nparts, double inv_cells,
+                                           double* __restrict__ out) {
     __shared__ double sh[3][8];
-    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int t = threadIdx.x;
+    if (t < 256) {
+        double a[3] = {0.0, 0.0, 0.0};
+        for (int p = t; p < nparts; p += 256) {
+            a[0] += partials[p * 3 + 0];
+            a[1] += partials[p * 3 + 1];
+            a[2] += partials[p * 3 + 2];
+        }
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const double t = warp_sum(a[k]);
-        if (lane == 0) sh[k][wid] = t;
+        for (int k = 0; k < 3; ++k) {
+            const double v = warp_sum(a[k]);
+            if ((t & 31) == 0) sh[k][t >> 5] = v;
+        }
     }
     __syncthreads();
-    if (threadIdx.x < 3) {
-        double t = 0.0;
-        for (int i = 0; i < 8; ++i) t += sh[threadIdx.x][i];
-        out[threadIdx.x] = t * inv_cells;
+    if (t < 3) {
+        double v = 0.0;
+        for (int i = 0; i < 8; ++i) v += sh[t][i];
+        out[t] = v * inv_cells;
     }
-    if (threadIdx.x == 0 && err) {
-        if (flag_out) *flag_out = double(*err);
-        *err = 0;
-    }
+}
+__global__ void __launch_bounds__(256) k_diag_finish(const double* __restrict__ partials, int nparts, double inv_cells,
+                                                     double* __restrict__ out) {
+    diag_total(partials, nparts, inv_cells, out);
 }
 
 // ---- energy / enstrophy / mass straight from the populations ---------------------------------------
@@ -556,7 +556,8 @@ __device__ __forceinline__ void pop_unpack(typename PopPair<typename ST::raw>::w
 template <class ST, bool SHIFTED>
 __global__ void __launch_bounds__(kPopThreads, 1)
     k_diag_pop(const PopPtrs<typename ST::raw> P, int n, int ntx, int ntiles, int zc, int items,
-               double* __restrict__ partials, int* __restrict__ err) {
+               double* __restrict__ partials, int* __restrict__ err, double inv_cells, double* __restrict__ out,
+               double* __restrict__ flag_out) {
     using RAW = typename ST::raw;
     using PP = PopPair<RAW>;
     using W = typename PP::word;
@@ -690,8 +691,26 @@ __global__ void __launch_bounds__(kPopThreads, 1)
         double sum = 0.0;
         for (int i = 0; i < kPopThreads / 32; ++i) sum += sh[t][i];
         partials[blockIdx.x * 3 + t] = *abort ? __longlong_as_double(0x7ff8000000000000ll) : sum;
+        __threadfence();
     }
     if (t == 0 && *abort) atomicExch(err, 1);
+    // the last CTA to get here adds the partials up (a launch less than a kernel of its own: 4 us of a small
+    // cube's diagnostic); err[1] counts the CTAs and goes back to zero for the next launch
+    __shared__ int last;
+    __syncthreads();
+    if (t == 0) {
+        __threadfence();
+        last = atomicAdd(err + 1, 1) == (int)gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    diag_total(partials, gridDim.x, inv_cells, out);
+    if (t == 0) {
+        if (flag_out) *flag_out = double(atomicExch(err, 0));
+        else *err = 0;
+        err[1] = 0;
+    }
 }
 
 template <class ST>
@@ -711,10 +730,11 @@ static cudaError_t launch_diag_pop_t(int layout, const void* f, int n, double* p
     const long long cap = std::min<long long>(kDiagBlocks, std::max(1, sms * std::max(1, per_sm)));
     const int ntx = (n + kPopTx - 1) / kPopTx, nty = (n + kPopTy - 1) / kPopTy, ntiles = ntx * nty;
     // z chunk: a CTA walks rounds x (chunk + 2 halo planes) planes, rounds = items over the resident
-    // CTA slots; take the chunk with the fewest (the longest on a tie)
+    // CTA slots; take the chunk with the fewest (the longest on a tie).  Small cubes go down to single planes:
+    // N=32 walks 3 planes instead of 6
     int best_zc = n;
     long long best = -1;
-    for (int zc = n; zc >= 4; --zc) {
+    for (int zc = n; zc >= 1; --zc) {
         const long long items = (long long)ntiles * ((n + zc - 1) / zc);
         const long long planes = (items + cap - 1) / cap * (zc + 2);
         if (best < 0 || planes < best) {
@@ -724,9 +744,9 @@ static cudaError_t launch_diag_pop_t(int layout, const void* f, int n, double* p
     }
     const long long nzc = (n + best_zc - 1) / best_zc, items = (long long)ntiles * nzc;
     const int grid = (int)std::min(items, cap);
-    kern<<<grid, kPopThreads, kPopRingBytes, st>>>(P, n, ntx, ntiles, best_zc, (int)items, partials_dev, err_dev);
-    k_diag_finish<<<1, 256, 0, st>>>(partials_dev, grid, 1.0 / double(cells), out_dev, err_dev, flag_out);
-    note_launch(2);
+    kern<<<grid, kPopThreads, kPopRingBytes, st>>>(P, n, ntx, ntiles, best_zc, (int)items, partials_dev, err_dev,
+                                                   1.0 / double(cells), out_dev, flag_out);
+    note_launch();
     return cudaGetLastError();
 }
 
