@@ -29,11 +29,13 @@ struct UniSolve {
     long long nseg;          // n^3 / V threads
 };
 constexpr int kMaxBatch = 48;
-struct UniBatch {
+template <int MAXB>
+struct UniBatchOf {
     int count;
     int pad;
-    UniSolve s[kMaxBatch];
+    UniSolve s[MAXB];
 };
+using UniBatch = UniBatchOf<kMaxBatch>;
 
 // Launch one stream-collide over `count` cubes of the same storage format (storage id of jp_storage).
 // vec: cells per thread along x (0 = default), tpb: threads per block (0 = default).

@@ -23,8 +23,15 @@ static std::atomic<long long> g_launches{0};
 void note_launch(int k) { g_launches.fetch_add(k, std::memory_order_relaxed); }
 long long launch_count() { return g_launches.load(std::memory_order_relaxed); }
 
-template <class ST, int V, int TPB>
-__global__ void __launch_bounds__(TPB, (min_blocks<ST, V, TPB>())) k_stream_collide(const __grid_constant__ UniBatch b) {
+template <class ST, int V, int TPB, int MAXB>
+__global__ void __launch_bounds__(TPB, (min_blocks<ST, V, TPB>())) k_stream_collide(const __grid_constant__ UniBatchOf<MAXB> b) {
+    // An FP64 CTA keeps its SM's FP64 pipe busy: the successor's CTAs come only when it is done relaxing, or they
+    // would be dealt two to an SM (N=32, 128 CTAs: 28.6 us per step released at once, 11.5 released late)
+    constexpr bool LATE = sizeof(typename ST::real) == 8;
+    if (MAXB == 1) {
+        if (!LATE) step_release();
+        step_wait();
+    }
     using raw = typename ST::raw;
     using R = typename ST::real;
     constexpr bool SH = ST::shifted;
@@ -35,8 +42,10 @@ __global__ void __launch_bounds__(TPB, (min_blocks<ST, V, TPB>())) k_stream_coll
 
     // which cube this CUDA block belongs to (uniform over the block)
     int si = 0;
+    if (MAXB > 1) {
 #pragma unroll 1
-    for (int i = 1; i < b.count; ++i) si = (b.s[i].blk_begin <= (long long)blockIdx.x) ? i : si;
+        for (int i = 1; i < b.count; ++i) si = (b.s[i].blk_begin <= (long long)blockIdx.x) ? i : si;
+    }
     const UniSolve& d = b.s[si];
     const long long seg = ((long long)blockIdx.x - d.blk_begin) * TPB + threadIdx.x;
     if (seg >= d.nseg) return;  // whole warps: nseg is a multiple of 32
@@ -107,6 +116,7 @@ __global__ void __launch_bounds__(TPB, (min_blocks<ST, V, TPB>())) k_stream_coll
     const R om = sizeof(R) == 8 ? R(d.omega_d) : R(d.omega);
     typename std::conditional<SH, CellBgk16<V>, CellBgk<R, V, SA>>::type c(om, sizeof(R) == 8 ? R(d.half_inv_d) : R(d.half_inv));
     c.moments(f);
+    if (MAXB == 1 && LATE) step_release();
     const size_t orow = ((size_t)z * n + y) * n + x0;
     {
         R o[V];
@@ -146,9 +156,9 @@ bool vec_supported(int storage, int vec) {
     return false;
 }
 
-template <class ST, int V, int TPB>
+template <class ST, int V, int TPB, int MAXB>
 static cudaError_t launch_sc(const UniSolve* solves, int count, cudaStream_t st) {
-    UniBatch b;
+    UniBatchOf<MAXB> b;
     b.count = count;
     b.pad = 0;
     long long blocks = 0;
@@ -161,18 +171,22 @@ static cudaError_t launch_sc(const UniSolve* solves, int count, cudaStream_t st)
     }
     if (blocks <= 0) return cudaSuccess;
     if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    k_stream_collide<ST, V, TPB><<<(unsigned)blocks, TPB, 0, st>>>(b);
     note_launch();
+    if constexpr (MAXB == 1) return launch_step(k_stream_collide<ST, V, TPB, 1>, (unsigned)blocks, TPB, 0, st, b);
+    k_stream_collide<ST, V, TPB, MAXB><<<(unsigned)blocks, TPB, 0, st>>>(b);
     return cudaGetLastError();
 }
 
 template <class ST, int V>
 static cudaError_t launch_sc_tpb(int tpb, const UniSolve* s, int c, cudaStream_t st) {
+    // one cube in the default mapping: a kernel with one cube's parameters (72 bytes instead of 3.5 KB), launched
+    // as its predecessor drains
+    if (c == 1 && tpb == 128) return launch_sc<ST, V, 128, 1>(s, c, st);
     switch (tpb) {
-        case 64: return launch_sc<ST, V, 64>(s, c, st);
-        case 128: return launch_sc<ST, V, 128>(s, c, st);
-        case 512: return launch_sc<ST, V, 512>(s, c, st);
-        default: return launch_sc<ST, V, 256>(s, c, st);
+        case 64: return launch_sc<ST, V, 64, kMaxBatch>(s, c, st);
+        case 128: return launch_sc<ST, V, 128, kMaxBatch>(s, c, st);
+        case 512: return launch_sc<ST, V, 512, kMaxBatch>(s, c, st);
+        default: return launch_sc<ST, V, 256, kMaxBatch>(s, c, st);
     }
 }
 

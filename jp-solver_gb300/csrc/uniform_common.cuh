@@ -69,6 +69,28 @@ template <> __device__ __forceinline__ uint16_t shfl_from<uint16_t>(uint16_t v, 
     return (uint16_t)__shfl_sync(0xffffffffu, (unsigned)v, lane);
 }
 
+// Programmatic dependent launch: a step launched with launch_step below may start while its predecessor in the
+// stream drains.  Every thread waits for the predecessor's completion (and its writes) before it touches a
+// state array (step_wait), and step_release lets the successor's CTAs take their places once every CTA of
+// this grid has called it or ended.  Both are no-ops in a plain launch.
+__device__ __forceinline__ void step_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void step_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// launch with programmatic stream serialization
+template <class K, class A>
+static cudaError_t launch_step(K kern, unsigned grid, int threads, int smem, cudaStream_t st, const A& arg) {
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = at;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kern, arg);
+}
+
 // Occupancy floor per SM for a variant: the wide-vector variants need warps (to keep 19 vector
 // loads per thread in flight, and for the issue-bound 16-bit collision) more than registers:
 // FP32 V=4 and 16-bit V=4 to 128 registers, 16-bit V=8 to 168.

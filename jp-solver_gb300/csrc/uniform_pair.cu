@@ -18,7 +18,7 @@
 // What bounds it (N=256, ncu): 2.56 GB of DRAM traffic per pass (the populations once each way) at 70 % of the
 // copy rate; the rest is the alternation of its phases (loads, FP32 pipe, shared memory) at 12 warps per
 // SM, 39 % issue.  Measured per step, single / two in one pass: N=512 2915 / 1890 us (46.0 / 71.0 GLUPS), N=256
-// 367 / 256, N=128 51.1 / 35.4, N=96 21.0 / 18.4, N=64 8.2 / 8.2, N=32 6.2 / 4.1 (one launch less per step).  Shapes
+// 367 / 256, N=128 48.0 / 36.2, N=96 17.5 / 17.8, N=32 3.4 / 3.0 (one launch less per two steps).  Shapes
 // measured and left: 512 threads (128 registers: spills, and 155 KB of ring leave the loads in flight too
 // little L1) 2315 us at N=512, 320 threads 2080, two CTAs of 256 or 192 threads (more halo) 2447 and 2262; a
 // ring one plane longer, with one barrier per plane, 2333; planes staged by 16-byte cp.async in shared memory
@@ -83,6 +83,10 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_stream_collide_pair(const _
     constexpr int NT = kPairThreads, SB = kSlotBytes;
     extern __shared__ __align__(16) char ring[];
     const int t = threadIdx.x;
+    if (MAXB == 1) {
+        step_release();
+        step_wait();
+    }
     for (int it = blockIdx.x; it < b.items; it += gridDim.x) {
         int si = 0;
         if (MAXB > 1) {
@@ -236,13 +240,18 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_stream_collide_pair(const _
     }
 }
 
-// Time model of the plans, in microseconds per step.  A CTA walks its items' planes (chunk + 2 halo planes
-// each) and a plane takes plane_us whatever the tile's share of the threads: measured 2.4-2.6 us for tiles of 56
-// to 128 cells along x at N=128..512, a third more for narrower tiles, whose rows are mostly halo.
-static double plane_us(int tx) { return tx < 48 ? 3.26 : 2.45; }
-// The single step: 21.7 ps per cell where HBM sets its time, 5 us and 12 ps per cell where the state stays in
-// L2 (measured N=32 6.1, N=48 6.2, N=64 8.2 us).
-static double single_us(double cells) { return std::max(cells * 21.7e-6, 5.0 + cells * 12e-6); }
+// Time model of the plans, in microseconds.  A CTA walks its items' planes (chunk + 2 halo planes each).  A
+// plane of a tile of 56 to 128 cells along x takes 2.4-2.6 us at N=128..512 whatever the tile's share of the
+// threads, a third more for narrower tiles, whose rows are mostly halo; where both states fit L2 (up to 600,000
+// cells) it takes 1.4-2.3 us with the share of threads at work.
+constexpr double kL2Cells = 6e5;
+static double plane_us(double cells, int tx, int ty) {
+    if (cells <= kL2Cells) return 2.3 * (0.5 + 0.5 * (tx / 2 + 2) * (ty + 2) / kPairThreads);
+    return tx < 48 ? 3.26 : 2.45;
+}
+// The single step: 21.7 ps per cell from HBM, 2.7 us and 12 ps per cell in L2 (measured N=16 2.8, N=32 3.4, N=64
+// 5.9, N=80 8.2, N=128 48.0, N=192 154.6 us; the two-step pass 2.2, 3.0, 7.0, 11.0, 36.2, 118.1).
+static double single_us(double cells) { return cells <= kL2Cells ? 2.7 + cells * 12e-6 : cells * 21.7e-6; }
 static bool pair_tile(int n, int tx, PairPlan& p) {
     const int P = tx / 2 + 2, tymax = std::min(n, kPairThreads / P - 2);
     if (tymax < 1) return false;
@@ -256,13 +265,15 @@ constexpr int kPairAlign = 8;  // x tiles start at 32-byte sectors
 // pairs of cells at even x need an even n; cell indices are 32-bit
 static bool pair_ok(int n, int sms) { return n >= 2 && n % 2 == 0 && n <= 1600 && sms > 0; }
 
-// One cube: every tile width, and the chunks that fill 1 to 16 rounds of CTAs.  The two-step pass is used where the model puts it 3 % ahead.
+// One cube: every tile width, and the chunks that fill 1 to 16 rounds of CTAs.  The two-step pass is used where the model puts it 5 % ahead.
 PairPlan pair_plan(int n, int sms) {
     PairPlan best{};
     if (!pair_ok(n, sms)) return best;
+    const double cells = double(n) * n * n;
     for (int tx = kPairAlign; tx <= 128 && tx < n + kPairAlign; tx += kPairAlign) {
         PairPlan p{};
         if (!pair_tile(n, tx, p)) break;
+        const double plane = plane_us(cells, tx, p.ty);
         int last = 0;
         for (int rounds = 1; rounds <= 16; ++rounds) {  // the shortest chunk that fits each number of rounds
             const int nzc = std::min((long long)n, (long long)rounds * sms / p.tiles);
@@ -270,16 +281,16 @@ PairPlan pair_plan(int n, int sms) {
             last = nzc;
             p.zc = (n + nzc - 1) / nzc;
             const long long items = (long long)p.tiles * ((n + p.zc - 1) / p.zc);
-            p.us = double((items + sms - 1) / sms) * (p.zc + 2) * plane_us(tx) / 2;
+            p.us = double((items + sms - 1) / sms) * (p.zc + 2) * plane / 2;
             if (best.us == 0 || p.us < best.us) best = p;
         }
         if (best.us == 0) {  // more tiles than 16 rounds hold: whole columns
             p.zc = n;
-            p.us = double((p.tiles + sms - 1) / sms) * (n + 2) * plane_us(tx) / 2;
+            p.us = double((p.tiles + sms - 1) / sms) * (n + 2) * plane / 2;
             best = p;
         }
     }
-    best.use = best.us < 0.97 * single_us(double(n) * n * n);
+    best.use = best.us < 0.95 * single_us(cells);
     return best;
 }
 
@@ -290,7 +301,7 @@ PairPlan pair_tile_plan(int n, int sms) {
     for (int tx = kPairAlign; tx <= 128 && tx < n + kPairAlign; tx += kPairAlign) {
         PairPlan p{};
         if (!pair_tile(n, tx, p)) break;
-        p.us = p.tiles * plane_us(tx);
+        p.us = p.tiles * plane_us(2 * kL2Cells, tx, p.ty);
         if (best.us == 0 || p.us < best.us) best = p;
     }
     return best;
@@ -308,7 +319,7 @@ bool pair_plan_batch(const int* n, int count, int sms, PairPlan* plans) {
         double sum = 0, longest = 0;
         for (int i = 0; i < count; ++i) {
             const int nzc = (n[i] + zc - 1) / zc, z = (n[i] + nzc - 1) / nzc;
-            const double us = (z + 2) * plane_us(plans[i].tx) / 2;
+            const double us = (z + 2) * plane_us(cells, plans[i].tx, plans[i].ty) / 2;
             sum += double(plans[i].tiles) * ((n[i] + z - 1) / z) * us;
             longest = std::max(longest, us);
         }
@@ -322,7 +333,7 @@ bool pair_plan_batch(const int* n, int count, int sms, PairPlan* plans) {
         const int nzc = (n[i] + best_zc - 1) / best_zc;
         plans[i].zc = (n[i] + nzc - 1) / nzc;
     }
-    return best < 0.97 * single_us(cells);
+    return best < 0.95 * single_us(cells);
 }
 
 template <int MAXB>
@@ -352,8 +363,9 @@ static cudaError_t launch_pair_t(const UniSolve* u, const PairPlan* plans, int c
         s.begin = b.items;
         b.items += s.ntiles * ((s.n + p.zc - 1) / p.zc);
     }
-    kern<<<std::min(b.items, sms), kPairThreads, kPairSmem, st>>>(b);
     note_launch();
+    if constexpr (MAXB == 1) return launch_step(kern, std::min(b.items, sms), kPairThreads, kPairSmem, st, b);
+    kern<<<std::min(b.items, sms), kPairThreads, kPairSmem, st>>>(b);
     return cudaGetLastError();
 }
 
