@@ -71,7 +71,8 @@ static jp_status batched_step(const std::vector<jp_solver*>& members, cudaStream
 
 // Two lattice steps of `members` (FP32) in one pass (uniform_pair.cu), one launch per kMaxBatch cubes; plans[k]
 // belongs to members[k].
-static jp_status batched_pair(const std::vector<jp_solver*>& members, const std::vector<PairPlan>& plans, cudaStream_t st) {
+static jp_status batched_pair(const std::vector<jp_solver*>& members, const std::vector<PairPlan>& plans, cudaStream_t st,
+                              int sms) {
     for (size_t i = 0; i < members.size(); i += kMaxBatch) {
         const size_t cnt = std::min(members.size() - i, (size_t)kMaxBatch);
         UniSolve us[kMaxBatch];
@@ -83,7 +84,7 @@ static jp_status batched_pair(const std::vector<jp_solver*>& members, const std:
             us[k].n = m->n;
             us[k].set_omega(m->info.omega);
         }
-        ECK(launch_stream_collide_pair(us, plans.data() + i, (int)cnt, members[0]->sms, st),
+        ECK(launch_stream_collide_pair(us, plans.data() + i, (int)cnt, sms, st),
             "batched two-step pass");
         for (size_t k = 0; k < cnt; ++k) {
             std::swap(members[i + k]->fa, members[i + k]->fb);
@@ -93,13 +94,19 @@ static jp_status batched_pair(const std::vector<jp_solver*>& members, const std:
     return JP_OK;
 }
 
+// SMs a two-step pass may fill while AMR coarse steps run on other streams: its CTAs hold an SM for a whole
+// chunk of planes, so the short AMR kernels would wait for them.  A ninth (16 of 152) is left free.  Measured, SMs
+// left free: an ensemble of 2 x {32..128} cubes and 6 AMR solves, 24 steps, 8: 4743, 16: 4545, 24 and more (the pass is
+// not used) 5300 us; 300 served requests 0 (single steps): 42.9, 16: 45.3, 32 and more: 42.9 solves/s.
+static int beside_amr(int sms) { return sms - sms / 9; }
+
 // The cubes of a set that take two-step passes together, largest first, planned as launches of up to kMaxBatch
 // cubes; none where the plan is no faster than single steps.  The others are listed in `single`.
 struct PairGroup {
     std::vector<jp_solver*> members, single;
     std::vector<PairPlan> plans;
 };
-static PairGroup pair_group(const std::vector<jp_solver*>& set) {
+static PairGroup pair_group(const std::vector<jp_solver*>& set, int sms) {
     PairGroup g;
     for (jp_solver* m : set) (m->pair_tile.tiles ? g.members : g.single).push_back(m);
     std::vector<jp_solver*>& v = g.members;
@@ -117,7 +124,7 @@ static PairGroup pair_group(const std::vector<jp_solver*>& set) {
             g.plans[i] = v[i]->pair;
             use = v[i]->pair.use;
         } else {
-            use = pair_plan_batch(n, cnt, v[i]->sms, g.plans.data() + i);
+            use = pair_plan_batch(n, cnt, sms, g.plans.data() + i);
         }
     }
     if (!use) {
@@ -138,6 +145,10 @@ struct jp_ensemble {
     int device = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t done = nullptr;
+    // mixed ensembles: the uniform members' steps run beside the AMR members' coarse steps
+    cudaStream_t uni = nullptr;
+    cudaEvent_t uni_fork = nullptr, uni_join = nullptr;
+    int sms = 0;
     AmrFork fk;  // the level-0 branch of the AMR members' coarse steps
     std::vector<jp_solver*> members;
     // persistent AMR coarse steps (jp_ensemble_set_persistent): barrier state of each launch of a
@@ -159,7 +170,14 @@ jp_status jp_ensemble_create(int32_t device, jp_ensemble** out) {
     jp_ensemble* e = new (std::nothrow) jp_ensemble();
     if (!e) return fail(JP_ERR_NOMEM, "host allocation");
     e->device = device;
-    cudaError_t err = cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking);
+    // the coarse steps' short kernels go first where uniform steps run beside them
+    int lo = 0, hi = 0;
+    cudaError_t err = cudaDeviceGetStreamPriorityRange(&lo, &hi);
+    if (err == cudaSuccess) err = cudaStreamCreateWithPriority(&e->stream, cudaStreamNonBlocking, hi);
+    if (err == cudaSuccess) err = cudaStreamCreateWithPriority(&e->uni, cudaStreamNonBlocking, lo);
+    if (err == cudaSuccess) err = cudaEventCreateWithFlags(&e->uni_fork, cudaEventDisableTiming);
+    if (err == cudaSuccess) err = cudaEventCreateWithFlags(&e->uni_join, cudaEventDisableTiming);
+    if (err == cudaSuccess) err = cudaDeviceGetAttribute(&e->sms, cudaDevAttrMultiProcessorCount, device);
     if (err == cudaSuccess) err = cudaEventCreateWithFlags(&e->done, cudaEventDisableTiming);
     if (err == cudaSuccess) err = e->fk.create(e->stream);
     if (err != cudaSuccess) {
@@ -177,6 +195,9 @@ void jp_ensemble_destroy(jp_ensemble* e) {
         cudaStreamDestroy(e->stream);
     }
     e->fk.destroy();
+    if (e->uni) cudaStreamDestroy(e->uni);  // always joined into e->stream, which has drained
+    if (e->uni_fork) cudaEventDestroy(e->uni_fork);
+    if (e->uni_join) cudaEventDestroy(e->uni_join);
     if (e->done) cudaEventDestroy(e->done);
     if (e->sync) cudaFree(e->sync);
     if (e->sync_host) cudaFreeHost(e->sync_host);
@@ -276,20 +297,42 @@ jp_status jp_ensemble_step(jp_ensemble* e, int64_t nsteps) {
             if (st != JP_OK) return st;
             in_persist[k] = true;
         }
-    const PairGroup pg = pair_group(nsteps > 1 ? uni : std::vector<jp_solver*>());
-    for (int64_t i = 0; i < nsteps; ++i) {
-        jp_status st = JP_OK;
-        if (nsteps == 1 || (i == nsteps - 1 && nsteps % 2)) {  // the odd step out
-            st = batched_step(uni, e->stream);
-        } else {
-            if (i % 2 == 0) st = batched_pair(pg.members, pg.plans, e->stream);
-            if (st == JP_OK) st = batched_step(pg.single, e->stream);
+    // Uniform and AMR members share nothing: the uniform steps run on a stream of their own beside the coarse
+    // steps, whose chains of short kernels leave most of the GPU idle (the ensemble of beside_amr: 6182 us one after
+    // the other).
+    bool stepwise = false;
+    for (size_t k = 0; k < amr.size(); ++k) stepwise = stepwise || !in_persist[k];
+    const bool beside = nsteps > 0 && !uni.empty() && stepwise;
+    const cudaStream_t us = beside ? e->uni : e->stream;
+    const int sms = beside ? beside_amr(e->sms) : e->sms;
+    struct Join {  // on every return
+        jp_ensemble* e;
+        bool on;
+        ~Join() {
+            if (on && cudaEventRecord(e->uni_join, e->uni) == cudaSuccess) cudaStreamWaitEvent(e->stream, e->uni_join, 0);
         }
-        if (st != JP_OK) return st;
-        for (size_t k = 0; k < amr.size(); ++k) {
-            if (in_persist[k]) continue;
-            st = amr_batch_step(amr[k], e->stream, &e->fk);
+    };
+    {
+        if (beside) {
+            ECK(cudaEventRecord(e->uni_fork, e->stream), "fork");
+            ECK(cudaStreamWaitEvent(e->uni, e->uni_fork, 0), "fork");
+        }
+        Join join{e, beside};
+        const PairGroup pg = pair_group(nsteps > 1 ? uni : std::vector<jp_solver*>(), sms);
+        for (int64_t i = 0; i < nsteps; ++i) {
+            jp_status st = JP_OK;
+            if (nsteps == 1 || (i == nsteps - 1 && nsteps % 2)) {  // the odd step out
+                st = batched_step(uni, us);
+            } else {
+                if (i % 2 == 0) st = batched_pair(pg.members, pg.plans, us, sms);
+                if (st == JP_OK) st = batched_step(pg.single, us);
+            }
             if (st != JP_OK) return st;
+            for (size_t k = 0; k < amr.size(); ++k) {
+                if (in_persist[k]) continue;
+                st = amr_batch_step(amr[k], e->stream, &e->fk);
+                if (st != JP_OK) return st;
+            }
         }
     }
     ECK(cudaEventRecord(e->done, e->stream), "event");
@@ -358,6 +401,7 @@ long long estimate_bytes(const jp_config& c) {
 struct jp_server {
     jp_server_config cfg{};
     cudaStream_t stream = nullptr;     // batched uniform launches and their diagnostics
+    int sms = 0;
     cudaMemPool_t pool = nullptr;      // device memory of every served solve (stream-ordered)
     std::deque<Job*> queue;            // submitted, not admitted
     std::vector<Job*> active;          // admitted uniform solves
@@ -787,6 +831,7 @@ jp_status jp_server_create(const jp_server_config* cfg, jp_server** out) {
     // with uniform_first the uniform batches share it and the AMR lanes take the lowest
     int lo = 0, hi = 0;
     cudaError_t e = cudaDeviceGetStreamPriorityRange(&lo, &hi);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sv->sms, cudaDevAttrMultiProcessorCount, cfg->device);
     if (e == cudaSuccess)
         e = cudaStreamCreateWithPriority(&sv->stream, cudaStreamNonBlocking, sv->cfg.uniform_first ? hi : lo);
     for (int l = 0; l < jp_server::kLanes && e == cudaSuccess; ++l) {
@@ -1080,8 +1125,9 @@ static jp_status server_tick(jp_server* sv, int32_t* n_active, int32_t* n_queued
             ECK(span_open(sv, sv->uspan, sv->uspan_tick, &jp_server_stats::uniform_gpu_s, sv->stream), "span");
             spanned = true;
         }
-        const PairGroup pg = pair_group(ahead);
-        jp_status st = batched_pair(pg.members, pg.plans, sv->stream);
+        const int sms = sv->amr_live > 0 ? beside_amr(sv->sms) : sv->sms;
+        const PairGroup pg = pair_group(ahead, sms);
+        jp_status st = batched_pair(pg.members, pg.plans, sv->stream, sms);
         if (st != JP_OK) return st;
         members.insert(members.end(), pg.single.begin(), pg.single.end());
         auto paired = [&pg](const jp_solver* s) {
