@@ -17,12 +17,12 @@
 //
 // What bounds it (N=256, ncu): 2.56 GB of DRAM traffic per pass (the populations once each way) at 70 % of the
 // copy rate; the rest is the alternation of its phases (loads, FP32 pipe, shared memory) at 12 warps per
-// SM, 39 % issue.  Measured per step, single / two in one pass: N=512 2915 / 1890 us (46.0 / 71.0 GLUPS), N=256
-// 367 / 256, N=128 48.0 / 36.2, N=96 17.5 / 17.8, N=32 3.4 / 3.0 (one launch less per two steps).  Shapes
+// SM, 39 % issue.  Measured per step, single / two in one pass: N=512 2915 / 1889 us (46.0 / 71.0 GLUPS), N=256
+// 364 / 259, N=128 48.0 / 34.6, N=96 17.5 / 16.9, N=32 3.4 / 3.0 (one launch less per two steps).  Shapes
 // measured and left: 512 threads (128 registers: spills, and 155 KB of ring leave the loads in flight too
 // little L1) 2315 us at N=512, 320 threads 2080, two CTAs of 256 or 192 threads (more halo) 2447 and 2262; a
 // ring one plane longer, with one barrier per plane, 2333; planes staged by 16-byte cp.async in shared memory
-// 2583; the two steps on two groups of warps with named barriers 2866 (each plane's chain of load, relax and
+// 2583; the second step's pulls read twice from the ring instead of held 1930; the two steps on two groups of warps with named barriers 2866 (each plane's chain of load, relax and
 // hand-over is longer than its share of bandwidth).  16-bit storage gains nothing (N=512 FP16 1588 to 1462 us in
 // the same forms, issue-bound, against 1507 for its single step).
 #include "kernels.h"
@@ -60,17 +60,6 @@ struct PairBatch {
     int count, items;
     PairSolve s[MAXB];
 };
-
-__device__ __forceinline__ unsigned lds_word(const char* p) {  // volatile: read twice rather than held in a register
-    unsigned v;
-    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"((unsigned)__cvta_generic_to_shared(p)));
-    return v;
-}
-__device__ __forceinline__ uint2 lds_words(const char* p) {
-    uint2 v;
-    asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"((unsigned)__cvta_generic_to_shared(p)));
-    return v;
-}
 
 // the collision inputs of a pair's two cells from the words of population q, and the relaxed values as stored
 __device__ __forceinline__ float2 pair_unpack(int q, unsigned w0, unsigned w1) {
@@ -199,21 +188,21 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_stream_collide_pair(const _
                         return pair_unpack(q, __float_as_uint(w.x), __float_as_uint(w.y));
                     }
                     const char* slot = (cz(q) == 0 ? rd0 : cz(q) > 0 ? rd1 : wr2) + zrank(q) * SB;
+                    const unsigned* w = reinterpret_cast<const unsigned*>(slot);
                     const int i = t - cy(q) * P;
-                    if (cx(q) == 0) {
-                        const uint2 v = lds_words(slot + i * 8);
-                        return pair_unpack(q, v.x, v.y);
-                    }
-                    return cx(q) > 0 ? pair_unpack(q, lds_word(slot + (NT + i - 1) * 4), lds_word(slot + i * 4))
-                                     : pair_unpack(q, lds_word(slot + (NT + i) * 4), lds_word(slot + (i + 1) * 4));
+                    if (cx(q) == 0) return pair_unpack(q, w[2 * i], w[2 * i + 1]);
+                    return cx(q) > 0 ? pair_unpack(q, w[NT + i - 1], w[i]) : pair_unpack(q, w[NT + i], w[i + 1]);
                 };
                 LaneBgk<float2, true> c(d.omega, d.half_inv);
-                c.add_rest(get(0));
+                float2 g[Q];
+                g[0] = get(0);
+                c.add_rest(g[0]);
 #pragma unroll
                 for (int i = 0; i < Q / 2; ++i) {
                     const int q = sum_order(i);
-                    float2 ga = get(q), gb = get(q + 1);
-                    c.add(q, ga, gb);
+                    g[q] = get(q);
+                    g[q + 1] = get(q + 1);
+                    c.add(q, g[q], g[q + 1]);
                 }
                 c.finish();
                 const unsigned o0 = (unsigned)(zs + r - 2) * n2 + row0 + gx;
@@ -224,12 +213,11 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_stream_collide_pair(const _
                     pk.v[1] = w.y;
                     st_pack<float, 2>(dst + q * qs + o0, pk);
                 };
-                store(0, c.rest(get(0)));
+                store(0, c.rest(g[0]));
 #pragma unroll
                 for (int q = 1; q < Q; q += 2) {
-                    const float2 ga = get(q), gb = get(q + 1);
                     float2 oa, ob;
-                    c.pair(q, __fadd2_rn(ga, gb), __fadd2_rn(ga, make_float2(-gb.x, -gb.y)), oa, ob);
+                    c.pair(q, g[q], g[q + 1], oa, ob);
                     store(q, oa);
                     store(q + 1, ob);
                 }
@@ -243,14 +231,14 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_stream_collide_pair(const _
 // Time model of the plans, in microseconds.  A CTA walks its items' planes (chunk + 2 halo planes each).  A
 // plane of a tile of 56 to 128 cells along x takes 2.4-2.6 us at N=128..512 whatever the tile's share of the
 // threads, a third more for narrower tiles, whose rows are mostly halo; where both states fit L2 (up to 600,000
-// cells) it takes 1.4-2.3 us with the share of threads at work.
+// cells) it takes 1.4-2.2 us with the share of threads at work.
 constexpr double kL2Cells = 6e5;
 static double plane_us(double cells, int tx, int ty) {
-    if (cells <= kL2Cells) return 2.3 * (0.5 + 0.5 * (tx / 2 + 2) * (ty + 2) / kPairThreads);
+    if (cells <= kL2Cells) return 2.2 * (0.5 + 0.5 * (tx / 2 + 2) * (ty + 2) / kPairThreads);
     return tx < 48 ? 3.26 : 2.45;
 }
 // The single step: 21.7 ps per cell from HBM, 2.7 us and 12 ps per cell in L2 (measured N=16 2.8, N=32 3.4, N=64
-// 5.9, N=80 8.2, N=128 48.0, N=192 154.6 us; the two-step pass 2.2, 3.0, 7.0, 11.0, 36.2, 118.1).
+// 5.9, N=80 8.2, N=128 48.0, N=192 154.6 us; the two-step pass 2.2, 3.0, 7.0, 11.0, 34.6, 112.5).
 static double single_us(double cells) { return cells <= kL2Cells ? 2.7 + cells * 12e-6 : cells * 21.7e-6; }
 static bool pair_tile(int n, int tx, PairPlan& p) {
     const int P = tx / 2 + 2, tymax = std::min(n, kPairThreads / P - 2);
