@@ -34,7 +34,7 @@ extern "C" jp_status jp_autotune(jp_config* cfg, int32_t steps, double* best) {
             if (!vec_supported(s->storage, v) || s->n % v || ((long long)s->cells / v) % 32) continue;
             if (s->inplace && v != s->vec) continue;  // the in-place steps run the storage's default width
             for (int t : tpbs) {
-                s->vec = v;
+                s->vec = s->solo_vec = v;
                 s->tpb = t;
                 float ms = 0.f;
                 st = jp_step(s, 2);
@@ -53,7 +53,7 @@ extern "C" jp_status jp_autotune(jp_config* cfg, int32_t steps, double* best) {
         }
         if (two) {
             s->pair.use = true;
-            s->vec = bv;
+            s->vec = s->solo_vec = bv;
             s->tpb = bt;
             float ms = 0.f;
             st = jp_step(s, 2);

@@ -64,6 +64,7 @@ struct jp_solver {
     double* partials = nullptr;  // diagnostic block partials + error word (kDiagPartials)
     double* diag_host = nullptr; // 3 doubles (+ the error word's copy, uniform), pinned: the kernels write it
     int vec = 0, tpb = 0;
+    int solo_vec = 0;          // vec of the cube stepped on its own (small cubes: narrower vectors, more threads)
     jp::PairPlan pair{};       // two steps in one pass, where pair.use (uniform_pair.cu)
     jp::PairPlan pair_tile{};  // the same in a launch of many cubes
     int sms = 0;               // multiprocessors of the device

@@ -73,6 +73,15 @@ static int pick_vec(int storage, int n, int want) {
     return 0;
 }
 
+// A small cube stepped on its own has fewer threads than the GPU holds: half the vector width doubles them.
+// Measured per step at widths 4 / 2 with 128 threads per CTA: FP32 N=48 4.9 / 4.0, N=64 6.1 / 5.5, N=80 8.2 / 8.6 us (216, 512,
+// 1000 CTAs of width 4); FP16 N=48 4.2 / 3.1, N=64 4.3 / 4.7.  (Launches of many cubes keep one width for all.)
+static int pick_solo_vec(const jp_solver* s) {
+    if (s->cfg.vec || s->inplace || s->vec != 4 || s->storage == JP_FP64) return s->vec;
+    const long long ctas = s->cells / 4 / 128;
+    return ctas < (s->storage == JP_FP32 ? 4 : 2) * s->sms ? 2 : 4;
+}
+
 jp_status uniform_create(jp_solver* s) {
     jp_status st = common_setup(s);
     if (st != JP_OK) return st;
@@ -96,6 +105,7 @@ jp_status uniform_create(jp_solver* s) {
         if (!s->vec) return fail(JP_ERR_INVALID, "no vector width fits n=%d (requested vec=%d)", c.n, c.vec);
     }
     JP_CK(cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, s->device), "cudaDeviceGetAttribute");
+    s->solo_vec = pick_solo_vec(s);
     if (!s->inplace && s->storage == JP_FP32) {
         s->pair = pair_plan(s->n, s->sms);
         s->pair_tile = pair_tile_plan(s->n, s->sms);
@@ -235,7 +245,7 @@ jp_status uniform_step(jp_solver* s, int64_t nsteps) {
     for (; i < nsteps; ++i) {
         u.src = s->fa;
         u.dst = s->fb;
-        cudaError_t e = launch_stream_collide(s->storage, &u, 1, s->vec, s->tpb, s->stream);
+        cudaError_t e = launch_stream_collide(s->storage, &u, 1, s->solo_vec, s->tpb, s->stream);
         if (e != cudaSuccess) return cuda_fail(e, "stream_collide launch");
         std::swap(s->fa, s->fb);
         ++s->step_count;

@@ -22,7 +22,8 @@
 // measured and left: 512 threads (128 registers: spills, and 155 KB of ring leave the loads in flight too
 // little L1) 2315 us at N=512, 320 threads 2080, two CTAs of 256 or 192 threads (more halo) 2447 and 2262; a
 // ring one plane longer, with one barrier per plane, 2333; planes staged by 16-byte cp.async in shared memory
-// 2583; the second step's pulls read twice from the ring instead of held 1930; the two steps on two groups of warps with named barriers 2866 (each plane's chain of load, relax and
+// 2583; the second step's pulls read twice from the ring instead of held 1930; the two steps on two groups of
+// warps with named barriers 2866 (each plane's chain of load, relax and
 // hand-over is longer than its share of bandwidth).  16-bit storage gains nothing (N=512 FP16 1588 to 1462 us in
 // the same forms, issue-bound, against 1507 for its single step).
 #include "kernels.h"
@@ -237,9 +238,9 @@ static double plane_us(double cells, int tx, int ty) {
     if (cells <= kL2Cells) return 2.2 * (0.5 + 0.5 * (tx / 2 + 2) * (ty + 2) / kPairThreads);
     return tx < 48 ? 3.26 : 2.45;
 }
-// The single step: 21.7 ps per cell from HBM, 2.7 us and 12 ps per cell in L2 (measured N=16 2.8, N=32 3.4, N=64
-// 5.9, N=80 8.2, N=128 48.0, N=192 154.6 us; the two-step pass 2.2, 3.0, 7.0, 11.0, 34.6, 112.5).
-static double single_us(double cells) { return cells <= kL2Cells ? 2.7 + cells * 12e-6 : cells * 21.7e-6; }
+// The single step: 21.7 ps per cell from HBM, 2.7 us and 11 ps per cell in L2 (measured N=16 2.8, N=32 3.1, N=48 4.0,
+// N=64 5.5, N=80 8.2, N=128 48.0, N=192 154.6 us; the two-step pass 2.2, 3.0, 4.9, 7.0, 11.0, 34.6, 112.5).
+static double single_us(double cells) { return cells <= kL2Cells ? 2.7 + cells * 11e-6 : cells * 21.7e-6; }
 static bool pair_tile(int n, int tx, PairPlan& p) {
     const int P = tx / 2 + 2, tymax = std::min(n, kPairThreads / P - 2);
     if (tymax < 1) return false;
