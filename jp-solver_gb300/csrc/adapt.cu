@@ -253,7 +253,8 @@ __global__ void k_dilate(const int* __restrict__ ref0, int cnb0, int cgx, const 
 // ordered compaction of the two flag ranges into the skin lists (copy_if over a counting iterator)
 __global__ void __launch_bounds__(kScanThreads) k_compact_skins(const int* __restrict__ flags, int cnb0, int nf1,
                                                                int* __restrict__ skin0, int* __restrict__ skin1,
-                                                               int* __restrict__ rest1, AdaptCounts* __restrict__ counts) {
+                                                               int* __restrict__ rest1, AdaptCounts* __restrict__ counts,
+                                                               int* __restrict__ nskin, int* __restrict__ nrest) {
     for (int part = 0; part < 2; ++part) {
         const int* fl = part == 0 ? flags : flags + cnb0;
         const int n = part == 0 ? cnb0 : nf1;
@@ -269,10 +270,13 @@ __global__ void __launch_bounds__(kScanThreads) k_compact_skins(const int* __res
             carry += tot;
         }
         if (threadIdx.x == 0) {
-            if (part == 0) counts->n_skin0 = carry;
-            else {
+            nskin[part] = carry;
+            if (part == 0) {
+                counts->n_skin0 = carry;
+            } else {
                 counts->n_skin1 = carry;
                 counts->n_rest1 = n - carry;
+                *nrest = n - carry;
             }
         }
     }
@@ -415,10 +419,10 @@ cudaError_t adapt_scatter_l2(const int* ref1, const int* rank, int nf1, int cap2
     return cudaGetLastError();
 }
 cudaError_t adapt_skins(const int* ref0, int cnb0, int cgx, const int* ref1, const int* f1pos, const int* l1grid,
-                        int nf1, int l1gx, int* flags, int* skin0, int* skin1, AdaptCounts* counts, cudaStream_t st,
-                        int* rest1) {
+                        int nf1, int l1gx, int* flags, int* skin0, int* skin1, int* rest1, AdaptCounts* counts, int* nskin,
+                        int* nrest, cudaStream_t st) {
     k_dilate<<<grid_for(cnb0 + nf1, 256), 256, 0, st>>>(ref0, cnb0, cgx, ref1, f1pos, l1grid, nf1, l1gx, flags);
-    k_compact_skins<<<1, kScanThreads, 0, st>>>(flags, cnb0, nf1, skin0, skin1, rest1, counts);
+    k_compact_skins<<<1, kScanThreads, 0, st>>>(flags, cnb0, nf1, skin0, skin1, rest1, counts, nskin, nrest);
     note_launch(2);
     return cudaGetLastError();
 }
@@ -455,8 +459,7 @@ cudaError_t adapt_dilate_marks(int* ref, int* tmp, int n, int gx, const int* pos
 }
 
 cudaError_t adapt_fill_list(const int* nb, int nf, int mb, int* list, int* count, cudaStream_t st) {
-    cudaError_t e = cudaMemsetAsync(count, 0, sizeof(int), st);
-    if (e != cudaSuccess || nf <= 0) return e;
+    if (nf <= 0) return cudaSuccess;
     switch (mb) {
         case 4: k_fill_list<4><<<nf, 160, 0, st>>>(nb, list, count); break;
         case 8: k_fill_list<8><<<nf, 256, 0, st>>>(nb, list, count); break;
@@ -469,8 +472,7 @@ cudaError_t adapt_fill_list(const int* nb, int nf, int mb, int* list, int* count
 
 cudaError_t adapt_prep_list(const int* skin, const int* nskin_dev, int cap, const int* ref, const int* pos,
                             const int* grid, int gx, int* list, int* count, cudaStream_t st) {
-    cudaError_t e = cudaMemsetAsync(count, 0, sizeof(int), st);
-    if (e != cudaSuccess || cap <= 0) return e;
+    if (cap <= 0) return cudaSuccess;
     k_prep_list<<<grid_for(cap, 256), 256, 0, st>>>(skin, nskin_dev, ref, pos, grid, gx, reinterpret_cast<int2*>(list),
                                                      count);
     note_launch();
@@ -479,11 +481,37 @@ cudaError_t adapt_prep_list(const int* skin, const int* nskin_dev, int cap, cons
 
 cudaError_t adapt_prep_cells(const int* plist, const int* pcount, int max_entries, int mb, int* cells, int* ncells,
                              cudaStream_t st) {
-    cudaError_t e = cudaMemsetAsync(ncells, 0, sizeof(int), st);
-    if (e != cudaSuccess || max_entries <= 0) return e;
+    if (max_entries <= 0) return cudaSuccess;
     const int mb3 = mb * mb * mb;
     k_prep_cells<<<max_entries, mb3 < 256 ? ((mb3 + 31) / 32) * 32 : 256, 0, st>>>(
         reinterpret_cast<const int2*>(plist), pcount, mb, cells, ncells);
+    note_launch();
+    return cudaGetLastError();
+}
+
+// The tables a regrid keeps of the previous grid, and its counts cleared, in one launch.
+__global__ void k_snapshot(const int* __restrict__ a0, const int* __restrict__ a1, int* __restrict__ b0, int* __restrict__ b1,
+                           int na, const int* __restrict__ g, int* __restrict__ gb, int ng, const int* __restrict__ c0,
+                           const int* __restrict__ c1, int* __restrict__ d0, int* __restrict__ d1, int nc,
+                           AdaptCounts* __restrict__ counts) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < na) {
+        b0[i] = a0[i];
+        b1[i] = a1[i];
+    }
+    if (i < ng) gb[i] = g[i];
+    if (i < nc) {
+        d0[i] = c0[i];
+        d1[i] = c1[i];
+    }
+    if (i == 0) *counts = AdaptCounts{};
+}
+cudaError_t adapt_snapshot(const int* ref0, const int* fof0, int* o_ref0, int* o_fof0, int cnb0, const int* l1grid,
+                           int* o_l1grid, int ng1, const int* ref1, const int* fof1, int* o_ref1, int* o_fof1, int cap1,
+                           AdaptCounts* counts, cudaStream_t st) {
+    const int n = std::max(std::max(cnb0, ng1), cap1);
+    k_snapshot<<<grid_for(n, 256), 256, 0, st>>>(ref0, fof0, o_ref0, o_fof0, cnb0, l1grid, o_l1grid, ng1, ref1, fof1, o_ref1,
+                                                 o_fof1, cap1, counts);
     note_launch();
     return cudaGetLastError();
 }

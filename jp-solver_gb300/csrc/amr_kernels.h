@@ -178,27 +178,33 @@ cudaError_t adapt_scan_l2(const int* ref1, int nf1, int* rank, AdaptCounts* coun
 cudaError_t adapt_scatter_l2(const int* ref1, const int* rank, int nf1, int cap2, int* fof1, int* rl1, int* l2pl1,
                              int* l2oct, AdaptCounts* counts, cudaStream_t st);
 // skin lists: blocks that are refined or have a refined 26-neighbour, ascending (k_dilate + copy_if);
-// rest1 (optional): the other level-1 blocks, ascending, their count in counts->n_rest1
+// rest1: the other level-1 blocks, ascending, their count in counts->n_rest1.  The two skin counts
+// also go to nskin[0..1] and the rest count to *nrest, where the coarse steps read them.
 cudaError_t adapt_skins(const int* ref0, int cnb0, int cgx, const int* ref1, const int* f1pos, const int* l1grid,
-                        int nf1, int l1gx, int* flags, int* skin0, int* skin1, AdaptCounts* counts, cudaStream_t st,
-                        int* rest1 = nullptr);
+                        int nf1, int l1gx, int* flags, int* skin0, int* skin1, int* rest1, AdaptCounts* counts, int* nskin,
+                        int* nrest, cudaStream_t st);
+// copies of the tables a regrid compares the new grid with, and *counts cleared: one launch for five
+// copies and a fill, whose launches took longer than the bytes (cnb0, ng1 and cap1 ints)
+cudaError_t adapt_snapshot(const int* ref0, const int* fof0, int* o_ref0, int* o_fof0, int cnb0, const int* l1grid,
+                           int* o_l1grid, int ng1, const int* ref1, const int* fof1, int* o_ref1, int* o_fof1, int cap1,
+                           AdaptCounts* counts, cudaStream_t st);
 // set n ints to v
 cudaError_t adapt_fill(int* p, int v, long long n, cudaStream_t st);
 // fill list of a fine level: the ghost-shell cells (faces, edges) of the nf blocks whose slot of the
 // neighbour table nb (27 per block) is on another level (-1), as b * SH + shell cell (SH = shell
-// cells of edge mb; at most SH per block); *count is set.  The list's order is not fixed: each
+// cells of edge mb; at most SH per block); *count, 0 before, is added to.  The list's order is not fixed: each
 // cell is filled independently.
 cudaError_t adapt_fill_list(const int* nb, int nf, int mb, int* list, int* count, cudaStream_t st);
 // prep list of a level: the skin blocks whose 27 neighbour blocks (periodic) mix refined and
 // unrefined, as pairs {block, mask of the refined neighbours (bit = slot)}; level 0: pos null and
 // gx = cgx; level 1: pos = f1pos, grid = l1grid, gx = l1gx (absent blocks unrefined).  The skin
 // count is read on the device (*nskin_dev, at most cap: the grid), so no read-back precedes the
-// list.  *count is set.
+// list.  *count, 0 before, is added to.
 cudaError_t adapt_prep_list(const int* skin, const int* nskin_dev, int cap, const int* ref, const int* pos,
                             const int* grid, int gx, int* list, int* count, cudaStream_t st);
 // interface cells of the (at most max_entries, *pcount) blocks of a prep list: the cells whose 3x3x3
 // neighbourhood reaches refined and unrefined blocks, as b * mb^3 + cell (at most
-// mb^3 - (mb-2)^3 per block); *ncells is set.  The order is not fixed.
+// mb^3 - (mb-2)^3 per block); *ncells, 0 before, is added to.  The order is not fixed.
 cudaError_t adapt_prep_cells(const int* plist, const int* pcount, int max_entries, int mb, int* cells, int* ncells,
                              cudaStream_t st);
 // interface cells a block can hold (its cells within one of a face)

@@ -178,7 +178,7 @@ static jp_status step_l0(jp_solver* s, cudaStream_t st = nullptr) {
 }
 
 // the host's block counts of the current grid to the device copy the step kernels read
-static jp_status upload_counts(jp_solver* s) {
+static jp_status upload_counts(jp_solver* s, cudaStream_t st) {
     AmrState* a = s->amr;
     int* h = a->step_cnt_host;
     h[SC_NF1] = a->nf1;
@@ -187,46 +187,47 @@ static jp_status upload_counts(jp_solver* s) {
     h[SC_SKIN1] = a->n_skin1;
     h[SC_NREF0] = a->nref0;
     h[SC_NREF1] = a->nref1;
-    ACK(cudaMemcpyAsync(a->step_cnt, h, sizeof(int) * SC_COUNT, cudaMemcpyHostToDevice, s->stream), "counts H2D");
+    ACK(cudaMemcpyAsync(a->step_cnt, h, sizeof(int) * SC_COUNT, cudaMemcpyHostToDevice, st), "counts H2D");
     return JP_OK;
 }
 
 // prep lists of both levels from their skin lists and refinement marks, lengths into the device counts;
 // the skin counts are read on the device (step_cnt[SC_SKIN0/1]), the grids sized by capacity
-static jp_status prep_lists(jp_solver* s) {
+static jp_status prep_lists(jp_solver* s, cudaStream_t st) {
     AmrState* a = s->amr;
     ACK(adapt_prep_list(a->skin0, a->step_cnt + SC_SKIN0, a->cnb0, a->ref0, nullptr, nullptr, a->cgx, a->pl0,
-                        a->step_cnt + SC_PBLK0, s->stream), "prep list 0");
+                        a->step_cnt + SC_PBLK0, st), "prep list 0");
     ACK(adapt_prep_list(a->skin1, a->step_cnt + SC_SKIN1, a->cap1, a->ref1, a->f1pos, a->l1grid, a->l1gx, a->pl1,
-                        a->step_cnt + SC_PBLK1, s->stream), "prep list 1");
-    ACK(adapt_prep_cells(a->pl0, a->step_cnt + SC_PBLK0, a->cnb0, a->MB, a->pc0, a->step_cnt + SC_PREP0, s->stream),
+                        a->step_cnt + SC_PBLK1, st), "prep list 1");
+    ACK(adapt_prep_cells(a->pl0, a->step_cnt + SC_PBLK0, a->cnb0, a->MB, a->pc0, a->step_cnt + SC_PREP0, st),
         "prep cells 0");
-    ACK(adapt_prep_cells(a->pl1, a->step_cnt + SC_PBLK1, a->cap1, a->MB, a->pc1, a->step_cnt + SC_PREP1, s->stream),
+    ACK(adapt_prep_cells(a->pl1, a->step_cnt + SC_PBLK1, a->cap1, a->MB, a->pc1, a->step_cnt + SC_PREP1, st),
         "prep cells 1");
     return JP_OK;
 }
 
-static_assert(offsetof(AdaptCounts, n_skin1) == offsetof(AdaptCounts, n_skin0) + sizeof(int) &&
-                  SC_SKIN1 == SC_SKIN0 + 1,
-              "the two skin counts are copied as one pair");
-
-// Skin lists of the current grid and the prep lists built from them.  Their lengths stay on the
-// device: the host's block counts go up first, then the two skin counts are copied over theirs
-// from the adaptation counts, and the prep lists read them there.  The host's copy of the skin
-// counts arrives with a read-back queued here and is taken after the caller's wait (skins_landed):
-// a regrid needs no read-back for its skins.
-static jp_status skins(jp_solver* s) {
+// Skin lists of the current grid and the prep lists built from them, on st.  Their lengths stay on
+// the device: the host's block counts go up first, then k_compact_skins writes the skin counts over
+// theirs, and the prep lists read them there.  The host's copy of the skin counts arrives with the
+// read-back of skins_readback and is taken after the caller's wait (skins_landed): a regrid needs no
+// read-back for its skins.  The list counts of the device are 0 before (clear_lists).
+static jp_status skins(jp_solver* s, cudaStream_t st) {
     AmrState* a = s->amr;
+    TRY(upload_counts(s, st));
     ACK(adapt_skins(a->ref0, a->cnb0, a->cgx, a->ref1, a->f1pos, a->l1grid, a->nf1, a->l1gx, a->flags, a->skin0,
-                    a->skin1, a->cnt_dev, s->stream, a->rest1), "skins");
-    TRY(upload_counts(s));
-    ACK(cudaMemcpyAsync(a->step_cnt + SC_SKIN0, &a->cnt_dev->n_skin0, 2 * sizeof(int), cudaMemcpyDeviceToDevice,
-                        s->stream), "skin counts");
-    ACK(cudaMemcpyAsync(a->step_cnt + SC_REST1, &a->cnt_dev->n_rest1, sizeof(int), cudaMemcpyDeviceToDevice,
-                        s->stream), "rest count");
-    TRY(prep_lists(s));
+                    a->skin1, a->rest1, a->cnt_dev, a->step_cnt + SC_SKIN0, a->step_cnt + SC_REST1, st), "skins");
+    return prep_lists(s, st);
+}
+static jp_status skins_readback(jp_solver* s) {
+    AmrState* a = s->amr;
     ACK(cudaMemcpyAsync(a->cnt_host, a->cnt_dev, sizeof(AdaptCounts), cudaMemcpyDeviceToHost, s->stream), "counts D2H");
     a->skins_pending = true;
+    return JP_OK;
+}
+
+// the lengths of the lists built from the neighbour tables and the skins: each list adds to its own
+static jp_status clear_lists(jp_solver* s, cudaStream_t st) {
+    ACK(cudaMemsetAsync(s->amr->step_cnt + SC_FILL1, 0, sizeof(int) * (SC_ALL - SC_FILL1), st), "list counts");
     return JP_OK;
 }
 
@@ -388,16 +389,20 @@ static jp_status build_l1(jp_solver* s, bool restore_marks) {
     return JP_OK;
 }
 
-// fill lists of both fine levels from their neighbour tables, lengths into the device counts
-static jp_status fill_lists(jp_solver* s) {
+// fill list of a fine level from its neighbour table, its length into the device counts
+static jp_status fill_list1(jp_solver* s, cudaStream_t st) {
     AmrState* a = s->amr;
-    ACK(adapt_fill_list(a->nb1, a->nf1, a->MB, a->fl1, a->step_cnt + SC_FILL1, s->stream), "fill list 1");
-    ACK(adapt_fill_list(a->nb2, a->nf2, a->MB, a->fl2, a->step_cnt + SC_FILL2, s->stream), "fill list 2");
+    ACK(adapt_fill_list(a->nb1, a->nf1, a->MB, a->fl1, a->step_cnt + SC_FILL1, st), "fill list 1");
+    return JP_OK;
+}
+static jp_status fill_list2(jp_solver* s, cudaStream_t st) {
+    AmrState* a = s->amr;
+    ACK(adapt_fill_list(a->nb2, a->nf2, a->MB, a->fl2, a->step_cnt + SC_FILL2, st), "fill list 2");
     return JP_OK;
 }
 
-// same-level neighbour tables of both fine levels for the current grid
-static jp_status neighbour_tables(jp_solver* s) {
+// same-level neighbour table and fill list of a fine level for the current grid
+static jp_status neighbours1(jp_solver* s, cudaStream_t st) {
     AmrState* a = s->amr;
     AmrLaunch L;
     L.nblocks = a->nf1;
@@ -407,7 +412,11 @@ static jp_status neighbour_tables(jp_solver* s) {
     L.t2 = a->ref0;
     L.t3 = a->fof0;
     L.cgx = a->cgx;
-    TRY(launch(s, OP_NBTAB_L1, L));
+    TRY(launch(s, OP_NBTAB_L1, L, st));
+    return fill_list1(s, st);
+}
+static jp_status neighbours2(jp_solver* s, cudaStream_t st) {
+    AmrState* a = s->amr;
     AmrLaunch M;
     M.nblocks = a->nf2;
     M.iout = a->nb2;
@@ -418,8 +427,8 @@ static jp_status neighbour_tables(jp_solver* s) {
     M.t4 = a->ref1;
     M.t5 = a->fof1;
     M.l1gx = a->l1gx;
-    TRY(launch(s, OP_NBTAB_L2, M));
-    return fill_lists(s);
+    TRY(launch(s, OP_NBTAB_L2, M, st));
+    return fill_list2(s, st);
 }
 
 // gpurce_init (src/tgv3d_amr.cu:776-815)
@@ -509,23 +518,53 @@ static jp_status initial_build(jp_solver* s) {
         L.scale = float(a->nqs12);
         TRY(launch(s, OP_SEED_L2, L));
     }
-    TRY(neighbour_tables(s));
-    TRY(skins(s));
-    return JP_OK;
+    TRY(clear_lists(s, s->stream));
+    TRY(neighbours1(s, s->stream));
+    TRY(neighbours2(s, s->stream));
+    TRY(skins(s, s->stream));
+    return skins_readback(s);
 }
 
+// Takes a side branch back into a stream (or a capture) on every return, errors included.
+struct JoinOnExit {
+    cudaStream_t st;
+    cudaEvent_t ev;
+    bool pending = true;
+    jp_status now() {
+        pending = false;
+        ACK(cudaStreamWaitEvent(st, ev, 0), "join");
+        return JP_OK;
+    }
+    ~JoinOnExit() {
+        if (pending) cudaStreamWaitEvent(st, ev, 0);
+    }
+};
+
+// The adaptation's tail runs on two streams: the level-1 tables and the skin lists need the marks
+// only, so they are built on fk.side while the fine levels are seeded.  A regrid is bound by the
+// latency of some thirty short launches in a row and its two read-backs, not by their bytes: with
+// the copies and fills merged (adapt_snapshot, clear_lists, counts written by k_compact_skins) and
+// this branch, N0=96 FP32 400 -> 328 us, N0=48 FP16 220 -> 168 us, N0=16 165 -> 141 us.
 // gpurce_regrid (src/tgv3d_amr.cu:722-764)
 static jp_status regrid(jp_solver* s) {
     AmrState* a = s->amr;
     const jp_config& c = s->cfg;
-    ACK(cudaMemsetAsync(a->cnt_dev, 0, sizeof(AdaptCounts), s->stream), "counts");
-    ACK(cudaMemcpyAsync(a->o_ref0, a->ref0, sizeof(int) * a->cnb0, cudaMemcpyDeviceToDevice, s->stream), "snapshot");
-    ACK(cudaMemcpyAsync(a->o_fof0, a->fof0, sizeof(int) * a->cnb0, cudaMemcpyDeviceToDevice, s->stream), "snapshot");
-    ACK(cudaMemcpyAsync(a->o_l1grid, a->l1grid, sizeof(int) * a->NG1, cudaMemcpyDeviceToDevice, s->stream), "snapshot");
-    ACK(cudaMemcpyAsync(a->o_ref1, a->ref1, sizeof(int) * a->cap1, cudaMemcpyDeviceToDevice, s->stream), "snapshot");
-    ACK(cudaMemcpyAsync(a->o_fof1, a->fof1, sizeof(int) * a->cap1, cudaMemcpyDeviceToDevice, s->stream), "snapshot");
+    const cudaStream_t side = a->fk.side;
+    ACK(adapt_snapshot(a->ref0, a->fof0, a->o_ref0, a->o_fof0, a->cnb0, a->l1grid, a->o_l1grid, a->NG1, a->ref1, a->fof1,
+                       a->o_ref1, a->o_fof1, a->cap1, a->cnt_dev, s->stream), "snapshot");
     TRY(mark_l0_by_sensor(s));
     TRY(build_l1(s, true));
+    // the level-1 tables beside the seeding; a failure on the way joins the branch as well
+    ACK(cudaEventRecord(a->fk.fork, s->stream), "fork");
+    ACK(cudaStreamWaitEvent(side, a->fk.fork, 0), "fork");
+    const auto tables1 = [&]() -> jp_status {
+        TRY(clear_lists(s, side));
+        return neighbours1(s, side);
+    };
+    const jp_status st1 = tables1();
+    ACK(cudaEventRecord(a->fk.join, side), "join");
+    JoinOnExit join{s->stream, a->fk.join};
+    TRY(st1);
     if (a->nf1) {
         AmrLaunch L;
         L.nblocks = a->nf1;
@@ -557,6 +596,15 @@ static jp_status regrid(jp_solver* s) {
         a->ndeep = a->cnt_host->ndeep;
         a->hw_nf2 = std::max(a->hw_nf2, (long long)a->nf2);
         if (a->nf2 > a->cap2) TRY(grow_l2(s, a->nf2));  // on failure the solver needs jp_init_tgv
+    }
+    // the skins need the marks of both levels (settled: read_counts waited); the host's counts are set
+    ACK(cudaEventRecord(a->fk.fork2, s->stream), "fork");
+    ACK(cudaStreamWaitEvent(side, a->fk.fork2, 0), "fork");
+    const jp_status st2 = skins(s, side);
+    ACK(cudaEventRecord(a->fk.join2, side), "join");
+    JoinOnExit join2{s->stream, a->fk.join2};
+    TRY(st2);
+    if (a->nf1) {
         ACK(cudaMemsetAsync(a->fof1, 0xFF, sizeof(int) * a->cap1, s->stream), "memset fof1");
         if (a->nref1)
             ACK(adapt_scatter_l2(a->ref1, a->rank, a->nf1, a->cap2, a->fof1, a->rl1, a->l2pl1, a->l2oct, a->cnt_dev,
@@ -581,9 +629,10 @@ static jp_status regrid(jp_solver* s) {
             std::swap(a->f2a, a->f2b);
         }
     }
-    TRY(neighbour_tables(s));
-    TRY(skins(s));
-    return JP_OK;
+    TRY(neighbours2(s, s->stream));
+    TRY(join.now());
+    TRY(join2.now());
+    return skins_readback(s);
 }
 
 cudaError_t AmrFork::create(cudaStream_t like) {
@@ -608,21 +657,6 @@ void AmrFork::destroy() {
     side = nullptr;
     fork = join = fork2 = join2 = nullptr;
 }
-
-// Takes a side branch back into a stream (or a capture) on every return, errors included.
-struct JoinOnExit {
-    cudaStream_t st;
-    cudaEvent_t ev;
-    bool pending = true;
-    jp_status now() {
-        pending = false;
-        ACK(cudaStreamWaitEvent(st, ev, 0), "join");
-        return JP_OK;
-    }
-    ~JoinOnExit() {
-        if (pending) cudaStreamWaitEvent(st, ev, 0);
-    }
-};
 
 // the coarse step and the level-1 ghosts it feeds (prolongation sources of level 0, level-1 fill)
 static jp_status level0_chain(jp_solver* s, cudaStream_t st) {
@@ -1497,8 +1531,11 @@ jp_status amr_load_state(jp_solver* s, std::FILE* f) {
         if (!fread_all(f, raw.data(), pl.second)) return fail(JP_ERR_INVALID, "state file truncated");
         if (pl.second) ACK(cudaMemcpy(pl.first, raw.data(), pl.second, cudaMemcpyHostToDevice), "pool H2D");
     }
-    TRY(fill_lists(s));
-    TRY(skins(s));  // the skin lists again (the same as stored) with the level-1 rest list, counts, prep lists
+    TRY(clear_lists(s, s->stream));
+    TRY(fill_list1(s, s->stream));
+    TRY(fill_list2(s, s->stream));
+    TRY(skins(s, s->stream));  // the skin lists again (the same as stored) with the level-1 rest list, counts, prep lists
+    TRY(skins_readback(s));
     ACK(wait_stream(s), "load");
     skins_landed(a);
     reset_graphs(a);
