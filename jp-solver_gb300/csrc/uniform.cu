@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(TPB, (min_blocks<ST, V, TPB>())) k_stream_coll
 
     const int n = d.n;
     const int nxs = d.nxs;
-    const raw* __restrict__ src = static_cast<const raw*>(d.src);
+    const raw* src = static_cast<const raw*>(d.src);
     raw* __restrict__ dst = static_cast<raw*>(d.dst);
     const int xs = int(seg % nxs);
     const long long r = seg / nxs;
@@ -83,10 +83,10 @@ __global__ void __launch_bounds__(TPB, (min_blocks<ST, V, TPB>())) k_stream_coll
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
         const raw* p = src + q * qs + roff[(1 - cz(q)) * 3 + 1 - cy(q)];  // pull from (y, z) - c_(y,z)
-        L[q] = ld_pack<raw, V>(p + x0);
+        L[q] = ld_step<raw, V>(p + x0);
         E[q] = raw(0);
-        if (cx(q) > 0 && prev_direct) E[q] = ld_one(p + xprev);
-        if (cx(q) < 0 && next_direct) E[q] = ld_one(p + xnext);
+        if (cx(q) > 0 && prev_direct) E[q] = p[xprev];
+        if (cx(q) < 0 && next_direct) E[q] = p[xnext];
     }
     // 2. neighbour values across the vector edge from the adjacent lanes
 #pragma unroll

@@ -15,17 +15,18 @@
 // Every cell goes through LaneBgk and the rounding of FP32 storage exactly as in the single step, in both of
 // the two steps, so the two paths give the same bits.
 //
-// What bounds it (N=256, ncu): 2.56 GB of DRAM traffic per pass (the populations once each way) at 70 % of the
+// What bounds it (N=256, ncu): 2.56 GB of DRAM traffic per pass (the populations once each way) at 73 % of the
 // copy rate; the rest is the alternation of its phases (loads, FP32 pipe, shared memory) at 12 warps per
-// SM, 39 % issue.  Measured per step, single / two in one pass: N=512 2915 / 1889 us (46.0 / 71.0 GLUPS), N=256
-// 364 / 259, N=128 48.0 / 34.6, N=96 17.5 / 16.9, N=32 3.4 / 3.0 (one launch less per two steps).  Shapes
+// SM, 39 % issue.  Measured per step, single / two in one pass: N=512 2915 / 1890 us (46.0 / 71.0 GLUPS), N=256
+// 364 / 261, N=128 48.0 / 34.8, N=96 17.5 / 17.0, N=32 3.4 / 2.9 (one launch less per two steps).  Shapes
 // measured and left: 512 threads (128 registers: spills, and 155 KB of ring leave the loads in flight too
 // little L1) 2315 us at N=512, 320 threads 2080, two CTAs of 256 or 192 threads (more halo) 2447 and 2262; a
 // ring one plane longer, with one barrier per plane, 2333; planes staged by 16-byte cp.async in shared memory
 // 2583; the second step's pulls read twice from the ring instead of held 1930; the two steps on two groups of
-// warps with named barriers 2866 (each plane's chain of load, relax and
-// hand-over is longer than its share of bandwidth).  16-bit storage gains nothing (N=512 FP16 1588 to 1462 us in
-// the same forms, issue-bound, against 1507 for its single step).
+// warps with named barriers 2866 (each plane's chain of load, relax and hand-over is longer than its share of
+// bandwidth).  16-bit storage stays with the single step: its relaxation keeps the per-cell sequence of
+// operations (a regrouped one moves 16-bit results past their rounding), which is issue-bound, and the pass
+// adds instructions (1462 to 1588 us in the forms tried with the regrouped one, against 1507 for that single step).
 #include "kernels.h"
 #include "lattice.cuh"
 #include "uniform_common.cuh"
@@ -88,7 +89,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_stream_collide_pair(const _
         const int row = t / P, col = t - row * P;
         const bool active = row < d.ty + 2;
         const bool inner = row >= 1 && row < d.ty + 1 && col >= 1 && col < P - 1;
-        const float* __restrict__ src = static_cast<const float*>(d.src);
+        const float* src = static_cast<const float*>(d.src);
         float* __restrict__ dst = static_cast<float*>(d.dst);
         const size_t qs = (size_t)n * n * n;
         const unsigned n2 = (unsigned)n * n;
@@ -113,11 +114,11 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_stream_collide_pair(const _
             for (int q = 0; q < Q; ++q) {
                 const float* p = src + q * qs + zo[1 - cz(q)];
                 const unsigned ro = cy(q) > 0 ? rowm : cy(q) < 0 ? rowp : row0;
-                auto one = [&](unsigned x) { return __ldg(reinterpret_cast<const unsigned*>(p + (ro + x))); };
+                auto one = [&](unsigned x) { return ld_step<float, 1>(p + (ro + x)).u32[0]; };
                 if (cx(q) == 0) {
-                    const uint2 v = __ldg(reinterpret_cast<const uint2*>(p + (ro + gx)));
-                    a0[q] = v.x;
-                    a1[q] = v.y;
+                    const Pack<float, 2> v = ld_step<float, 2>(p + (ro + gx));
+                    a0[q] = v.u32[0];
+                    a1[q] = v.u32[1];
                 } else {
                     a0[q] = cx(q) > 0 ? one(xm) : one(gx + 1);
                     a1[q] = cx(q) > 0 ? one(gx) : one(xp);
