@@ -52,7 +52,7 @@ static jp_status batched_step(const std::vector<jp_solver*>& members, cudaStream
                 us[k].src = m->fa;
                 us[k].dst = m->inplace ? m->fa : m->fb;
                 us[k].n = m->n;
-                us[k].set_omega(m->info.omega);
+                us[k].set_omega(m->info.omega, m->bgk);
             }
             if (v[i]->inplace) {
                 ECK(launch_stream_collide_inplace(v[i]->storage, us, (int)cnt, int(v[i]->step_count & 1), v[i]->vec,
@@ -82,7 +82,7 @@ static jp_status batched_pair(const std::vector<jp_solver*>& members, const std:
             us[k].src = m->fa;
             us[k].dst = m->fb;
             us[k].n = m->n;
-            us[k].set_omega(m->info.omega);
+            us[k].set_omega(m->info.omega, m->bgk);
         }
         ECK(launch_stream_collide_pair(us, plans.data() + i, (int)cnt, sms, st),
             "batched two-step pass");

@@ -9,19 +9,31 @@ namespace jp {
 
 // ---- uniform periodic cube, flat SoA layout [q][z][y][x] ----------------------------------------
 
+// Coefficients of the relaxation (LaneBgk, uniform_common.cuh) for one omega: 3 om w and om w of the faces and
+// edges, om w of the rest population, 1/(2 om w) of the faces and edges.
+template <class R>
+struct BgkCoefOf {
+    R om, a1, a2, b0, b1, b2, k1, k2;
+};
+using BgkCoef = BgkCoefOf<float>;
+// Rounded each for itself, the coefficients would gain or lose mass in every step: relaxing a cell changes its
+// mass by (C0 - om) e + (2 K - 1.5 om) j.j / rho with C0 = b0 + 6 b1 + 12 b2 and K = k1 a1^2 + 4 k2 a2^2,
+// which exact ones make zero.  Each is taken within one unit in the last place of its value so that this is smallest
+// (N=64, Re=400, 2000 steps: mass drift 3.2e-7 with the nearest values, 8.1e-9 so, 2.1e-8 by a product chain per
+// population).  The edges' a2 is the nearest, a1 what it leaves of the momentum's 2 a1 + 8 a2 = om (exact).
+BgkCoef bgk_coefficients(float omega);
+
 // One periodic cube of a batched stream-collide launch.
 struct UniSolve {
     const void* src;         // populations at t   (19 * n^3 elements)
     void* dst;               // populations at t+1
     int n;                   // edge
     int nxs;                 // n / V: x segments per row
-    float omega;             // 1/tau (FP32 and shifted storages)
-    float half_inv;          // 1 / (2 omega)
+    BgkCoef bgk;             // of 1/tau (FP32 and shifted storages)
     double omega_d;          // 1/tau (FP64 storage)
     double half_inv_d;       // 1 / (2 omega_d)
-    void set_omega(double w) {
-        omega = float(w);
-        half_inv = 0.5f / omega;
+    void set_omega(double w, const BgkCoef& c) {
+        bgk = c;
         omega_d = w;
         half_inv_d = 0.5 / w;
     }

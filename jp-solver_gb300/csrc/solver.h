@@ -43,6 +43,7 @@ cudaError_t wait_event(cudaEvent_t ev);
 struct jp_solver {
     jp_config cfg{};
     jp_info info{};
+    jp::BgkCoef bgk{};          // uniform: the relaxation's coefficients for info.omega
     int kind = 0;
     int device = 0;
     int storage = 0;

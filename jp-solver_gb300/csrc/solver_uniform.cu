@@ -19,6 +19,35 @@ namespace jp {
         if (e_ != cudaSuccess) return cuda_fail(e_, what);  \
     } while (0)
 
+BgkCoef bgk_coefficients(float omega) {
+    const double om = omega;
+    const float a2 = float(om / 12), a1 = float(0.5 * (om - 8.0 * a2));
+    // the value nearest to x, and its two neighbours
+    const auto near3 = [](double x, float* v) {
+        v[0] = float(x);
+        v[1] = std::nextafter(v[0], 0.f);
+        v[2] = std::nextafter(v[0], 64.f);
+    };
+    float b0[3], b1[3], b2[3], k1[3], k2[3];
+    near3(om / 3, b0);
+    near3(om / 18, b1);
+    near3(om / 36, b2);
+    near3(9 / om, k1);
+    near3(18 / om, k2);
+    BgkCoef best{};
+    double least = -1;
+    for (int i = 0; i < 243; ++i) {
+        const BgkCoef c{omega, a1, a2, b0[i % 3], b1[i / 3 % 3], b2[i / 9 % 3], k1[i / 27 % 3], k2[i / 81]};
+        const double c0 = c.b0 + 6.0 * c.b1 + 12.0 * c.b2, k = c.k1 * (double(a1) * a1) + 4 * c.k2 * (double(a2) * a2);
+        const double off = std::fabs(2 * k - 1.5 * c0) + 0.1 * std::fabs(c0 - om);
+        if (least < 0 || off < least) {
+            least = off;
+            best = c;
+        }
+    }
+    return best;
+}
+
 // nu, tau and the step count exactly as the reference derives them (src/tgv3d_uniform.cu:151-153,
 // src/tgv3d_amr.cu:659-664).
 jp_status common_setup(jp_solver* s) {
@@ -52,6 +81,7 @@ jp_status common_setup(jp_solver* s) {
     in.nu = c.u0 * N / (2.0 * M_PI * c.re);
     in.tau = 3.0 * in.nu + 0.5;
     in.omega = double(float(1.0 / in.tau));
+    s->bgk = bgk_coefficients(float(in.omega));
     if (c.storage == JP_FP64) in.omega = 1.0 / in.tau;
     in.tau1 = 2.0 * in.tau - 0.5;
     in.tau2 = 2.0 * in.tau1 - 0.5;
@@ -222,7 +252,7 @@ jp_status uniform_step(jp_solver* s, int64_t nsteps) {
     UniSolve u;
     std::memset(&u, 0, sizeof u);
     u.n = s->n;
-    u.set_omega(s->info.omega);
+    u.set_omega(s->info.omega, s->bgk);
     if (s->inplace) {
         u.src = u.dst = s->fa;
         for (int64_t i = 0; i < nsteps; ++i) {

@@ -113,8 +113,7 @@ __global__ void __launch_bounds__(TPB, (min_blocks<ST, V, TPB>())) k_stream_coll
         }
 
     // 4. moments, 5. relax and store, one population pair at a time
-    const R om = sizeof(R) == 8 ? R(d.omega_d) : R(d.omega);
-    typename std::conditional<SH, CellBgk16<V>, CellBgk<R, V, SA>>::type c(om, sizeof(R) == 8 ? R(d.half_inv_d) : R(d.half_inv));
+    typename std::conditional<SH, CellBgk16<V>, CellBgk<R, V, SA>>::type c(bgk_of<R>(d));
     c.moments(f);
     if (MAXB == 1 && LATE) step_release();
     const size_t orow = ((size_t)z * n + y) * n + x0;

@@ -84,8 +84,7 @@ __global__ void __launch_bounds__(TPB, (aa_local_min_blocks<ST, V, TPB>())) k_aa
 #pragma unroll
         for (int v = 0; v < V; ++v) f[v][q] = (SA && !SH) ? ST::load(L[q].v[v]) - wgt<R>(q) : ST::load(L[q].v[v]);
 
-    const R om = sizeof(R) == 8 ? R(d.omega_d) : R(d.omega);
-    typename std::conditional<SH, CellBgk16<V>, CellBgk<R, V, SA>>::type c(om, sizeof(R) == 8 ? R(d.half_inv_d) : R(d.half_inv));
+    typename std::conditional<SH, CellBgk16<V>, CellBgk<R, V, SA>>::type c(bgk_of<R>(d));
     c.moments(f);
     {
         R o0[V];
@@ -188,8 +187,7 @@ __global__ void __launch_bounds__(TPB, (aa_stream_min_blocks<ST, V, TPB>())) k_a
             f[v][q] = (SA && !SH) ? ST::load(e) - wgt<R>(q) : ST::load(e);
         }
     // 4. relax in place
-    const R om = sizeof(R) == 8 ? R(d.omega_d) : R(d.omega);
-    typename std::conditional<SH, CellBgk16<V>, CellBgk<R, V, SA>>::type c(om, sizeof(R) == 8 ? R(d.half_inv_d) : R(d.half_inv));
+    typename std::conditional<SH, CellBgk16<V>, CellBgk<R, V, SA>>::type c(bgk_of<R>(d));
     c.moments(f);
 #pragma unroll
     for (int v = 0; v < V; ++v) f[v][0] = c.rest(f, v);

@@ -8,6 +8,7 @@
 #include <type_traits>
 #include <utility>
 
+#include "kernels.h"
 #include "lattice.cuh"
 
 namespace jp {
@@ -111,7 +112,7 @@ constexpr int min_blocks() {
 
 // ---- BGK relaxation of V cells ------------------------------------------------------------------
 // f[v][q] holds the collision inputs of cell v in the collision type R: the shifts g = f - w_q when SA (FP32
-// shifts on load), f itself for FP64.  half_inv = 1 / (2 omega).
+// shifts on load), f itself for FP64.
 //
 // FP32: Blackwell issues two FP32 adds, multiplies or FMAs in one instruction (f32x2; __fadd2_rn,
 // __fmul2_rn, __ffma2_rn, each lane rounded to nearest like its scalar op).  The FP32 steps hold V = 2,
@@ -123,7 +124,7 @@ constexpr int min_blocks() {
 //   S_q = g_q + g_opp, D_q = g_q - g_opp; s = g0 + the S, j = the signed sums of the D, in sum_order
 //   rho = 1 + s (s itself in FP64), inv = 1 / rho (IEEE), e = s - 1.5 inv (jx jx + jy jy + jz jz) (two FMAs)
 //   out0 = (1-om) g0 + om w0 e
-//   a = (3 om w) (c_q . j), t = om w e + (inv / (2 om w)) a a   [= om w rho (4.5 (c.u)^2 - 1.5 u.u) + om w s]
+//   a = (3 om w) (c_q . j), t = om w e + (1/(2 om w) inv) a a   [= om w rho (4.5 (c.u)^2 - 1.5 u.u) + om w s]
 //   u = (1-om)/2 S + t, v = (1-om)/2 D + a; out_q = u + v, out_opp(q) = u - v.
 // Measured against one product chain per population (147 operations; the 16-bit storages keep it, CellBgk16):
 // error against 64 bits of N=64 FP32 after 200 steps 1.4-1.8e-7 -> 1.1-1.5e-7.
@@ -131,6 +132,17 @@ constexpr int min_blocks() {
 __host__ __device__ constexpr int sum_order(int i) {
     constexpr int t[Q / 2] = {1, 3, 7, 9, 5, 11, 13, 15, 17};
     return t[i];
+}
+// the coefficients of a launch's cube: FP32's come with it (bgk_coefficients); FP64's need no such care
+template <class R>
+__device__ __forceinline__ BgkCoefOf<R> bgk_of(const UniSolve& d) {
+    if constexpr (sizeof(R) == 4) {
+        return d.bgk;
+    } else {
+        const double om = d.omega_d, a2 = om * (1.0 / 12.0);
+        return {om, 0.5 * fma(-8.0, a2, om), a2, om * wgt<double>(0), om * wgt<double>(1), om * wgt<double>(7),
+                d.half_inv_d * 18.0, d.half_inv_d * 36.0};
+    }
 }
 // One lane set T (a float, a double, a pair of floats) of the sequence.  SA: the inputs are shifts.
 template <class T, bool SA>
@@ -142,17 +154,9 @@ struct LaneBgk {
     T inv;            // 1 / rho
     T k, b, ax, ay, az;  // of the class at hand (faces, edges)
 
-    // 3 om w of the classes.  A momentum component is relaxed by 2 a1 + 8 a2 in all, which has to be om: the
-    // faces take what the edges' rounding leaves (a common factor off by 3e-8 in every step would be a
-    // systematic gain of momentum).
-    R a1, a2;
+    BgkCoefOf<R> co;
 
-    R kc;  // 1 / (2 om)
-
-    __device__ __forceinline__ LaneBgk(R omega, R half_inv) : om(omega), kc(half_inv) {
-        a2 = omega * (R(1) / R(12));
-        a1 = R(0.5) * fma(R(-8), a2, omega);
-    }
+    __device__ __forceinline__ LaneBgk(const BgkCoefOf<R>& c) : om(c.om), co(c) {}
 
     __device__ __forceinline__ void add_rest(T g0) { s = g0; }
     // the pair (q, q+1), in the order q = sum_order(0), sum_order(1), ...: ga, gb become S, D
@@ -173,14 +177,14 @@ struct LaneBgk {
         s = L::fma(L::mul(L::bc(R(-1.5)), inv), t, s);
     }
     __device__ __forceinline__ T rest(T g0) const {
-        return L::fma(L::bc(R(1) - om), g0, L::mul(L::bc(om * wgt<R>(0)), s));
+        return L::fma(L::bc(R(1) - om), g0, L::mul(L::bc(co.b0), s));
     }
     // relaxed populations q and q+1 = opp(q) (q odd, ascending from 1) from S and D
     __device__ __forceinline__ void pair(int q, T S, T D, T& oa, T& ob) {
         if (q == 1 || q == 7) {
-            const R w = q == 1 ? a1 : a2;
-            b = L::mul(L::bc(om * wgt<R>(q)), s);
-            k = L::mul(L::bc(kc * R(q == 1 ? 18 : 36)), inv);
+            const R w = q == 1 ? co.a1 : co.a2;
+            b = L::mul(L::bc(q == 1 ? co.b1 : co.b2), s);
+            k = L::mul(L::bc(q == 1 ? co.k1 : co.k2), inv);
             ax = L::mul(L::bc(w), jx);
             ay = L::mul(L::bc(w), jy);
             az = L::mul(L::bc(w), jz);
@@ -207,9 +211,9 @@ struct CellBgk {
     T S[NP][Q / 2], D[NP][Q / 2];
 
     template <int... I>
-    __device__ __forceinline__ CellBgk(R omega, R half_inv, std::integer_sequence<int, I...>)
-        : c{((void)I, LaneBgk<T, SA>(omega, half_inv))...} {}
-    __device__ __forceinline__ CellBgk(R omega, R half_inv) : CellBgk(omega, half_inv, std::make_integer_sequence<int, NP>{}) {}
+    __device__ __forceinline__ CellBgk(const BgkCoefOf<R>& co, std::integer_sequence<int, I...>)
+        : c{((void)I, LaneBgk<T, SA>(co))...} {}
+    __device__ __forceinline__ CellBgk(const BgkCoefOf<R>& co) : CellBgk(co, std::make_integer_sequence<int, NP>{}) {}
 
     static __device__ __forceinline__ T get(const R (&f)[V][Q], int p, int q) {
         if constexpr (PAIR) return make_float2(f[2 * p][q], f[2 * p + 1][q]);
@@ -278,7 +282,7 @@ struct CellBgk16 {
     T owr1[NP], owr2[NP], owr3a[NP], owr3b[NP];
     T orest[NP];
 
-    __device__ __forceinline__ explicit CellBgk16(float omega, float) : om(omega), omc(1.f - omega) {}
+    __device__ __forceinline__ explicit CellBgk16(const BgkCoef& co) : om(co.om), omc(1.f - co.om) {}
 
     static __device__ __forceinline__ T get(const float (&f)[V][Q], int p, int q) {
         if constexpr (PAIR) return make_float2(f[2 * p][q], f[2 * p + 1][q]);

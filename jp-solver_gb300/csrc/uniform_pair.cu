@@ -17,8 +17,8 @@
 //
 // What bounds it (N=256, ncu): 2.56 GB of DRAM traffic per pass (the populations once each way) at 73 % of the
 // copy rate; the rest is the alternation of its phases (loads, FP32 pipe, shared memory) at 12 warps per
-// SM, 39 % issue.  Measured per step, single / two in one pass: N=512 2915 / 1890 us (46.0 / 71.0 GLUPS), N=256
-// 364 / 261, N=128 48.0 / 34.8, N=96 17.5 / 17.0, N=32 3.4 / 2.9 (one launch less per two steps).  Shapes
+// SM, 39 % issue.  Measured per step, single / two in one pass: N=512 2915 / 1866 us (46.0 / 71.9 GLUPS), N=256
+// 364 / 254, N=128 48.0 / 34.0, N=96 17.5 / 16.4, N=32 3.4 / 2.9 (one launch less per two steps).  Shapes
 // measured and left: 512 threads (128 registers: spills, and 155 KB of ring leave the loads in flight too
 // little L1) 2315 us at N=512, 320 threads 2080, two CTAs of 256 or 192 threads (more halo) 2447 and 2262; a
 // ring one plane longer, with one barrier per plane, 2333; planes staged by 16-byte cp.async in shared memory
@@ -55,7 +55,7 @@ struct PairSolve {
     void* dst;
     int n, tx, ty, ntx, ntiles, zc;
     int begin;  // first item of the cube in the launch
-    float omega, half_inv;
+    BgkCoef bgk;
 };
 template <int MAXB>
 struct PairBatch {
@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_stream_collide_pair(const _
             char* const wr2 = ring + kRingM;
             if (active) {
                 float2 g[Q];
-                LaneBgk<float2, true> c(d.omega, d.half_inv);
+                LaneBgk<float2, true> c(d.bgk);
                 g[0] = pair_unpack(0, a0[0], a1[0]);
                 c.add_rest(g[0]);
 #pragma unroll
@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_stream_collide_pair(const _
                     if (cx(q) == 0) return pair_unpack(q, w[2 * i], w[2 * i + 1]);
                     return cx(q) > 0 ? pair_unpack(q, w[NT + i - 1], w[i]) : pair_unpack(q, w[NT + i], w[i + 1]);
                 };
-                LaneBgk<float2, true> c(d.omega, d.half_inv);
+                LaneBgk<float2, true> c(d.bgk);
                 float2 g[Q];
                 g[0] = get(0);
                 c.add_rest(g[0]);
@@ -343,8 +343,7 @@ static cudaError_t launch_pair_t(const UniSolve* u, const PairPlan* plans, int c
         s.src = u[i].src;
         s.dst = u[i].dst;
         s.n = u[i].n;
-        s.omega = u[i].omega;
-        s.half_inv = u[i].half_inv;
+        s.bgk = u[i].bgk;
         s.tx = p.tx;
         s.ty = p.ty;
         s.zc = p.zc;
