@@ -44,7 +44,7 @@ constexpr int kMaxBatch = 48;
 template <int MAXB>
 struct UniBatchOf {
     int count;
-    int pad;
+    int release;  // one cube: the CTAs let the successor's in at once (release_early)
     UniSolve s[MAXB];
 };
 using UniBatch = UniBatchOf<kMaxBatch>;

@@ -25,11 +25,8 @@ long long launch_count() { return g_launches.load(std::memory_order_relaxed); }
 
 template <class ST, int V, int TPB, int MAXB>
 __global__ void __launch_bounds__(TPB, (min_blocks<ST, V, TPB>())) k_stream_collide(const __grid_constant__ UniBatchOf<MAXB> b) {
-    // An FP64 CTA keeps its SM's FP64 pipe busy: the successor's CTAs come only when it is done relaxing, or they
-    // would be dealt two to an SM (N=32, 128 CTAs: 28.6 us per step released at once, 11.5 released late)
-    constexpr bool LATE = sizeof(typename ST::real) == 8;
     if (MAXB == 1) {
-        if (!LATE) step_release();
+        if (b.release) step_release();
         step_wait();
     }
     using raw = typename ST::raw;
@@ -115,7 +112,6 @@ __global__ void __launch_bounds__(TPB, (min_blocks<ST, V, TPB>())) k_stream_coll
     // 4. moments, 5. relax and store, one population pair at a time
     typename std::conditional<SH, CellBgk16<V>, CellBgk<R, V, SA>>::type c(bgk_of<R>(d));
     c.moments(f);
-    if (MAXB == 1 && LATE) step_release();
     const size_t orow = ((size_t)z * n + y) * n + x0;
     {
         R o[V];
@@ -159,7 +155,7 @@ template <class ST, int V, int TPB, int MAXB>
 static cudaError_t launch_sc(const UniSolve* solves, int count, cudaStream_t st) {
     UniBatchOf<MAXB> b;
     b.count = count;
-    b.pad = 0;
+    b.release = count == 1 && release_early(ST::shifted, sizeof(typename ST::real) == 8, solves[0].n);
     long long blocks = 0;
     for (int i = 0; i < count; ++i) {
         b.s[i] = solves[i];
@@ -178,7 +174,7 @@ static cudaError_t launch_sc(const UniSolve* solves, int count, cudaStream_t st)
 
 template <class ST, int V>
 static cudaError_t launch_sc_tpb(int tpb, const UniSolve* s, int c, cudaStream_t st) {
-    // one cube in the default mapping: a kernel with one cube's parameters (72 bytes instead of 3.5 KB), launched
+    // one cube in the default mapping: a kernel with one cube's parameters (100 bytes instead of 5 KB), launched
     // as its predecessor drains
     if (c == 1 && tpb == 128) return launch_sc<ST, V, 128, 1>(s, c, st);
     switch (tpb) {

@@ -247,7 +247,7 @@ template <class ST, int V, int TPB>
 static cudaError_t launch_aa(const UniSolve* solves, int count, int parity, cudaStream_t st) {
     UniBatch b;
     b.count = count;
-    b.pad = 0;
+    b.release = 0;
     long long blocks = 0;
     for (int i = 0; i < count; ++i) {
         UniSolve& u = b.s[i];

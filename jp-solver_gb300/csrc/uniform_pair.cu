@@ -59,7 +59,7 @@ struct PairSolve {
 };
 template <int MAXB>
 struct PairBatch {
-    int count, items;
+    int count, items, release;
     PairSolve s[MAXB];
 };
 
@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_stream_collide_pair(const _
     extern __shared__ __align__(16) char ring[];
     const int t = threadIdx.x;
     if (MAXB == 1) {
-        step_release();
+        if (b.release) step_release();
         step_wait();
     }
     for (int it = blockIdx.x; it < b.items; it += gridDim.x) {
@@ -334,6 +334,7 @@ static cudaError_t launch_pair_t(const UniSolve* u, const PairPlan* plans, int c
     PairBatch<MAXB> b;
     b.count = count;
     b.items = 0;
+    b.release = count == 1 && release_early(false, false, u[0].n);
     for (int i = 0; i < count; ++i) {
         PairSolve& s = b.s[i];
         const PairPlan& p = plans[i];
