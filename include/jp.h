@@ -84,7 +84,8 @@ typedef struct jp_config {
 /* jp_config.flags */
 #define JP_FLAG_SKIP_PREP 1      /* AMR profiling: skip prep + ghost fill (breaks physics; --skipprep, src/tgv3d_amr.cu:654) */
 #define JP_FLAG_SKIP_RESTRICT 2  /* AMR profiling: skip restriction (breaks physics; --skiprestr, :655) */
-#define JP_FLAG_GRAPH 4          /* replay the step from captured CUDA graphs (--graph, :656) */
+#define JP_FLAG_GRAPH 4          /* replay the step from captured CUDA graphs (--graph, :656) from the first step on;
+                                    without it an AMR solver does so once a step has been launched four times */
 #define JP_FLAG_DEFER_INIT 8     /* jp_create allocates only: set a sensor override (or populations) and
                                     call jp_init_tgv before the first step, so that even the first
                                     AMR build uses the supplied sensor */
@@ -164,7 +165,9 @@ jp_status jp_diag(jp_solver* s, double out[3]);
 jp_status jp_population_count(const jp_solver* s, int32_t level, int64_t* count);
 
 /* Copy the populations of `level` to a host buffer of `count` values of type `dtype`, in `layout`.
- * Shifted FP16/BF16 storage is returned unshifted (f = w_q + stored). */
+ * Shifted FP16/BF16 storage is returned unshifted (f = w_q + stored).  Another type or order than the
+ * state's is converted on the device, through memory of the solver that holds nothing between steps (an
+ * in-place cube allocates up to 64 MiB for it on first use). */
 jp_status jp_get_populations(jp_solver* s, int32_t level, int32_t layout, int32_t dtype,
                              void* host, int64_t count);
 
@@ -283,10 +286,10 @@ jp_status jp_load_state(jp_solver* s, const char* path);
 
 /* ---- ensembles and serving (extensions; no counterpart in the reference) ------------- */
 
-/* An ensemble steps many solvers of the same device together, on the ensemble's stream, ordered
- * after each member's pending work and before its later work.  Uniform members: one batched
- * stream-collide launch per storage format per lattice step (up to 48 cubes of any sizes per
- * launch).  AMR members: one coarse step (the 1:2:4 subcycle) with one launch per stage over the
+/* An ensemble steps many solvers of the same device together, on the ensemble's streams (uniform and
+ * AMR members beside each other), ordered after each member's pending work and before its later
+ * work.  Uniform members: one batched stream-collide launch per storage format per lattice step, or
+ * per two steps in FP32 (up to 48 cubes of any sizes per launch).  AMR members: one coarse step (the 1:2:4 subcycle) with one launch per stage over the
  * blocks of all members of the same block edge, storage and step threads (up to 48 per launch);
  * jp_ensemble_step(e, k) advances AMR members by k coarse steps.  Regrids and diagnostics stay
  * per solver (jp_regrid, jp_diag) between ensemble steps. */

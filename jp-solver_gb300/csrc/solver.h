@@ -70,6 +70,7 @@ struct jp_solver {
     jp::PairPlan pair_tile{};  // the same in a launch of many cubes
     int sms = 0;               // multiprocessors of the device
     void* io = nullptr;        // population conversion scratch of an in-place cube, allocated on first use
+    size_t io_bytes = 0;
     float* outbuf = nullptr;   // device Q / speed / velocity for output frames, allocated on first use
     // populations staged for the next step (jp_stage_populations): uploaded into `staging` on
     // copy_stream while the solver's stream works, swapped in as fa by the next step

@@ -1116,7 +1116,12 @@ static jp_status graph_step(jp_solver* s, cudaStream_t on = nullptr) {
         if (e != cudaSuccess) return cuda_fail(e, "end capture");
         e = cudaGraphInstantiate(&a->graph[key], g, 0);
         cudaGraphDestroy(g);
-        if (e != cudaSuccess) return cuda_fail(e, "graph instantiate");
+        if (e == cudaSuccess) e = cudaGraphUpload(a->graph[key], s->stream);  // its memory now, not at the first launch
+        if (e != cudaSuccess) {
+            if (a->graph[key]) cudaGraphExecDestroy(a->graph[key]);
+            a->graph[key] = nullptr;
+            return cuda_fail(e, "graph instantiate");
+        }
     }
     ACK(cudaGraphLaunch(a->graph[key], on ? on : s->stream), "graph launch");
     std::swap(a->c0a, a->c0b);  // the fine levels return to their buffers within the step
@@ -1268,16 +1273,25 @@ jp_status amr_init(jp_solver* s) {
 
 // Without JP_FLAG_GRAPH a coarse step is captured once its case (graph_key) has been launched kCaptureAfter times:
 // a run replays (per coarse step, launches / graph: N0=24 71 / 51 us, N0=48 FP16 76 / 59, N0=96 304 / 293; a capture costs
-// 50 to 70 us, paid back by four steps), a handful of steps does not pay for captures.
+// 50 to 70 us, paid back by four steps), a handful of steps does not pay for captures.  Where there is no memory
+// left for a graph the case stays with launches.
 constexpr int kCaptureAfter = 4;
 jp_status amr_step(jp_solver* s, int64_t nsteps) {
     const bool graph = s->cfg.flags & JP_FLAG_GRAPH;
     for (int64_t i = 0; i < nsteps; ++i) {
         AmrState* a = s->amr;
         const int key = graph_key(a);
-        if (graph || a->launched[key] >= kCaptureAfter) {
-            TRY(graph_step(s));
-        } else {
+        bool replay = graph || a->launched[key] >= kCaptureAfter;
+        if (replay) {
+            const jp_status st = graph_step(s);
+            if (st != JP_OK && (graph || a->graph[key])) return st;
+            if (st != JP_OK) {
+                cudaGetLastError();
+                a->launched[key] = INT_MIN / 2;
+                replay = false;
+            }
+        }
+        if (!replay) {
             TRY(base_step(s));
             ++a->launched[key];
         }
@@ -1328,8 +1342,8 @@ jp_status amr_get_output_fields(jp_solver* s, float* q, float* speed, float* vel
     return output_fields_from(s, a->field, false, false, a->N2, q, speed, vel);
 }
 
-// The composite field the diagnostics need, allocated ahead of an amr_diag_async on another stream.
-// the diagnostics' macro buffer, for the blocks the pools hold
+// the diagnostics' macro buffer, for the blocks the pools hold (amr_prepare_diag: ahead of an amr_diag_async on
+// another stream)
 static jp_status ensure_macro(jp_solver* s) {
     AmrState* a = s->amr;
     if (a->macro) return JP_OK;
@@ -1373,7 +1387,7 @@ jp_status amr_diag(jp_solver* s, double out[3]) {
     AmrState* a = s->amr;
     // Where (nearly) every record of the finest grid is a leaf cell the composite field is the shorter way: it
     // needs no lookups (N0=64 refined everywhere 497 us, by leaf blocks 555; N0=96 dynamic, 1 % of the records
-    // leaves, 1087 and 222).
+    // leaves, 1087 and 214).
     if ((double)a->nf2 * a->MB3 > 0.9 * (double)a->N2 * a->N2 * a->N2) {
         TRY(composite(s));
         ACK(launch_diag_field(false, false, a->field, a->N2, s->partials, s->diag_host, s->stream), "diag");

@@ -359,7 +359,7 @@ void uniform_flat_to_raw(const jp_solver* s, const unsigned char* flat, unsigned
 
 // Populations in another type or order than the state's, converted on the device.  The scratch is the next
 // step's target array, whose contents nothing reads between steps; an in-place cube takes an allocation of
-// at most 64 MiB on first use.
+// 64 MiB, or what it can get of that down to 1 MiB, on first use.
 static jp_status uniform_convert(jp_solver* s, int layout, int dtype, void* host, bool to_host_order) {
     PopMap m{};
     m.n = s->n;
@@ -378,9 +378,21 @@ static jp_status uniform_convert(jp_solver* s, int layout, int dtype, void* host
     void* scratch = s->fb;
     size_t bytes = (size_t)Q * s->cells * s->elem;
     if (s->inplace) {
-        bytes = std::min(bytes, (size_t)64 << 20);
-        if (!s->io) JP_CK(dev_alloc(s, &s->io, bytes), "cudaMalloc population scratch");
+        if (!s->io) {
+            s->io_bytes = std::min(bytes, (size_t)64 << 20);
+            cudaError_t e = dev_alloc(s, &s->io, s->io_bytes);
+            while (e == cudaErrorMemoryAllocation && s->io_bytes > ((size_t)1 << 20)) {
+                cudaGetLastError();
+                s->io_bytes /= 2;
+                e = dev_alloc(s, &s->io, s->io_bytes);
+            }
+            if (e != cudaSuccess) {
+                s->io = nullptr;
+                return cuda_fail(e, "cudaMalloc population scratch");
+            }
+        }
         scratch = s->io;
+        bytes = s->io_bytes;
     }
     return convert_populations(s, s->storage, dtype, m, s->fa, scratch, bytes, host, to_host_order);
 }
