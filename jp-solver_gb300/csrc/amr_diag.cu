@@ -168,7 +168,8 @@ __global__ void __launch_bounds__(kLeafThreads) k_leaf_diag(const AmrGrid g, con
             const int s = (face & 1) ? 1 : -1;
             if (unsigned(a + s) < unsigned(MB)) return __ldg(own + c + s * d);
             if ((same >> face) & 1) {
-                const int u = face == 0 ? nb[0] : face == 1 ? nb[1] : face == 2 ? nb[2] : face == 3 ? nb[3] : face == 4 ? nb[4] : nb[5];
+                const int u = face == 0 ? nb[0] : face == 1 ? nb[1] : face == 2 ? nb[2] : face == 3 ? nb[3]
+                            : face == 4 ? nb[4] : nb[5];
                 return __ldg(M + (size_t)u * MB3 + c - s * (MB - 1) * d);
             }
             auto in = [N2](int v) { return v < 0 ? v + N2 : v >= N2 ? v - N2 : v; };

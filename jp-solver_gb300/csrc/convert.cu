@@ -5,7 +5,8 @@
 // type (shifted 16-bit) or order (flat, in-place layouts), these kernels convert between the state and a
 // device scratch that one DMA moves, chunk by chunk.  A warp takes a unit: a row of the flat order, or a
 // block's population; reads and writes are coalesced along x (8 cells at a time in blocks of edge 8).
-// The conversion of N=96 FP16 to blocked FP32 (16.8 M values) takes ~0.03 ms; on one host thread it took 0.2 s.
+// The conversion of N=96 FP16 to blocked FP32 (16.8 M values) takes ~0.03 ms beside its transfer (0.42 ms in
+// all); on one host thread it took 0.2 s.
 // Values are those of the host conversion: f = w_q + stored, stored = round(f - w_q) through float.
 #include "kernels.h"
 #include "lattice.cuh"

@@ -90,7 +90,8 @@ __device__ __forceinline__ void step_release() { asm volatile("griddepcontrol.la
 // room, unevenly, so where the grid is about a wave they double up on some SMs; over several waves they fill the
 // last one's gaps.  us per step, released at once / at the end: FP32 N=8 2.08 / 1.70, N=32 2.92 / 2.87, N=56 4.64 / 4.23,
 // N=64 5.36 / 5.26, N=72 6.62 / 6.68, N=128 34.0 / 34.4, N=192 109.7 / 110.8;
-// FP16 N=24 2.24 / 2.34, N=32 2.95 / 2.36, N=48 3.21 / 3.01, N=56 4.46 / 3.98, N=64 4.31 / 4.50, N=80 6.54 / 6.79; FP64 N=32 28.6 / 11.3 (a CTA keeps its SM's FP64 pipe busy).
+// FP16 N=24 2.24 / 2.34, N=32 2.95 / 2.36, N=48 3.21 / 3.01, N=56 4.46 / 3.98, N=64 4.31 / 4.50, N=80 6.54 / 6.79;
+// FP64 N=32 28.6 / 11.3 (a CTA keeps its SM's FP64 pipe busy).
 [[maybe_unused]] static bool release_early(bool shifted, bool fp64, int n) {
     const long long cells = (long long)n * n * n;
     if (fp64) return false;

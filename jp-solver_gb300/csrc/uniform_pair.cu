@@ -255,7 +255,8 @@ constexpr int kPairAlign = 8;  // x tiles start at 32-byte sectors
 // pairs of cells at even x need an even n; cell indices are 32-bit
 static bool pair_ok(int n, int sms) { return n >= 2 && n % 2 == 0 && n <= 1600 && sms > 0; }
 
-// One cube: every tile width, and the chunks that fill 1 to 16 rounds of CTAs.  The two-step pass is used where the model puts it 5 % ahead.
+// One cube: every tile width, and the chunks that fill 1 to 16 rounds of CTAs.  The two-step pass is used where
+// the model puts it 5 % ahead.
 PairPlan pair_plan(int n, int sms) {
     PairPlan best{};
     if (!pair_ok(n, sms)) return best;
