@@ -554,14 +554,13 @@ static jp_status regrid(jp_solver* s) {
                        a->o_ref1, a->o_fof1, a->cap1, a->cnt_dev, s->stream), "snapshot");
     TRY(mark_l0_by_sensor(s));
     TRY(build_l1(s, true));
+    // the list counts go to zero ahead of the fork: both streams add to them (fill list 1 and the prep lists on
+    // the side, fill list 2 on the solver's own)
+    TRY(clear_lists(s, s->stream));
     // the level-1 tables beside the seeding; a failure on the way joins the branch as well
     ACK(cudaEventRecord(a->fk.fork, s->stream), "fork");
     ACK(cudaStreamWaitEvent(side, a->fk.fork, 0), "fork");
-    const auto tables1 = [&]() -> jp_status {
-        TRY(clear_lists(s, side));
-        return neighbours1(s, side);
-    };
-    const jp_status st1 = tables1();
+    const jp_status st1 = neighbours1(s, side);
     ACK(cudaEventRecord(a->fk.join, side), "join");
     JoinOnExit join{s->stream, a->fk.join};
     TRY(st1);

@@ -1,0 +1,107 @@
+// Checks of the engine's host code on the fake runtime (fake_cudart.h): ./runtime_checks NAME runs one.
+#include "fake_cudart.h"
+
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+
+#include "amr_kernels.h"
+#include "jp.h"
+
+using jp::amr::AdaptCounts;
+
+static int failures = 0;
+#define CHECK(x)                                                            \
+    do {                                                                    \
+        if (!(x)) {                                                         \
+            std::printf("%s:%d: %s (%s)\n", __FILE__, __LINE__, #x, jp_last_error()); \
+            ++failures;                                                     \
+        }                                                                   \
+    } while (0)
+
+static bool is(const fake::Op& o, const char* kernel) {
+    return o.kind == fake::Op::KERNEL && o.name.find(kernel) != std::string::npos;
+}
+template <class T>
+static T arg(const fake::Op& o, int i) {
+    return *static_cast<T*>(o.args[i]);
+}
+
+// ---- an AMR solver of 64 coarse blocks whose adaptation kernels "find" the grid in `grid` ----
+static AdaptCounts grid;
+static jp_solver* amr(double max_gb, int flags = 0) {
+    jp_config c;
+    jp_config_default(&c, JP_AMR);
+    c.n = 32;
+    c.l1_mode = c.l2_mode = JP_REFINE_SENSOR;
+    c.frac1 = 0.25;
+    c.develop_steps = 1;
+    c.max_gb = max_gb;
+    c.flags = flags;
+    jp_solver* s = nullptr;
+    CHECK(jp_create(&c, &s) == JP_OK);
+    return s;
+}
+static void set_grid(int nref0, int nref1) {
+    grid = AdaptCounts{};
+    grid.nref0 = nref0;
+    grid.nf1 = 8 * nref0;
+    grid.nref1 = nref1;
+    grid.nf2 = 8 * nref1;
+    grid.n_skin0 = nref0;
+    grid.n_skin1 = nref1;
+}
+static void supply_grid() {
+    fake::on_d2h = [](void* dst, size_t bytes) {
+        if (bytes == sizeof(AdaptCounts)) std::memcpy(dst, &grid, bytes);
+    };
+}
+
+// Every list of the coarse step grows from a count that a fill has set to zero: on every route through an
+// adaptation the fill is ordered after the last use of the count and before the kernel that adds to it.
+static void regrid_orders_list_counts() {
+    struct Use {
+        size_t op;
+        const char* count;
+    };
+    std::vector<Use> uses;
+    fake::on_kernel = [&](fake::Op& o) {
+        const int i = is(o, "k_fill_list") ? 2 : is(o, "k_prep_list") ? 7 : is(o, "k_prep_cells") ? 4 : -1;
+        if (i >= 0) uses.push_back({fake::ops.size() - 1, arg<const char*>(o, i)});
+    };
+    supply_grid();
+    set_grid(16, 10);
+    jp_solver* s = amr(64.0);
+    for (int k = 0; k < 3; ++k) {
+        CHECK(jp_step(s, 2) == JP_OK);
+        set_grid(15 + k, 12 - k);
+        CHECK(jp_regrid(s) == JP_OK);
+    }
+    CHECK(uses.size() == 4 * 6);  // one initial build, three regrids
+    std::map<const char*, size_t> last;
+    for (const Use& u : uses) {
+        long long fill = -1;
+        for (size_t i = 0; i < u.op; ++i) {
+            const fake::Op& o = fake::ops[i];
+            if (o.kind == fake::Op::MEMSET && u.count >= o.dst && u.count < o.dst + o.bytes) fill = (long long)i;
+        }
+        CHECK(fill >= 0);
+        if (fill < 0) continue;
+        CHECK(fake::before(fake::ops[fill], fake::ops[u.op]));
+        if (last.count(u.count)) CHECK(fake::before(fake::ops[last[u.count]], fake::ops[fill]));
+        last[u.count] = u.op;
+    }
+    jp_destroy(s);
+}
+
+int main(int argc, char** argv) {
+    const std::map<std::string, void (*)()> checks = {
+        {"regrid_orders_list_counts", regrid_orders_list_counts},
+    };
+    const auto it = argc == 2 ? checks.find(argv[1]) : checks.end();
+    if (it == checks.end()) return 2;
+    it->second();
+    for (const std::string& f : fake::faults) std::printf("%s\n", f.c_str());
+    std::printf("%d failed checks, %zu faults\n", failures, fake::faults.size());
+    return failures || !fake::faults.empty() ? 1 : 0;
+}
