@@ -581,6 +581,7 @@ void amr_task(jp_server* sv, Job* j) {
     } else {
         auto t = clk::now();
         st = jp_regrid(j->s);
+        if (st == JP_OK) st = amr_prepare_diag(j->s);  // a pool that grew took the diagnostics' buffer with it
         sv->add(&jp_server_stats::regrid_s, seconds_since(t), &jp_server_stats::regrids);
     }
     if (st == JP_OK && j->dg) {  // into slot 2 of the solver's pinned read-back area (slots 0, 1: tick)

@@ -55,6 +55,7 @@ struct AmrState {
     bool skins_pending = false;  // n_skin0/1 arrive with the read-back skins() queued (skins_landed)
     float* field = nullptr;   // composite field of the output frames, allocated on first use
     float* macro = nullptr;   // leaf blocks' macroscopic values of the diagnostics (launch_amr_diag)
+    size_t macro_blocks = 0;  // blocks macro holds (ensure_macro)
     std::vector<void*> owned;
     // Block counts the step kernels read on the device ({nf1, nf2, n_skin0, n_skin1, nref0, nref1}):
     // the step launches grids sized for the pool capacities, so one captured step serves every grid
@@ -284,11 +285,11 @@ static void update_bytes(jp_solver* s) {
                                      ((size_t)a->cap1 + a->cap2) * Q * a->SH) * a->elem);
 }
 
-// the diagnostics' macro buffer, if there is one, for new pool capacities
-static jp_status regrow_macro(jp_solver* s) {
-    AmrState* a = s->amr;
-    if (!a->macro) return JP_OK;
-    return regrow(s, a->macro, 4 * ((size_t)a->cnb0 + a->cap1 + a->cap2) * a->MB3, 0);
+// The diagnostics' macro buffer goes with the pools it was sized by; the next diagnostic allocates it again, so
+// a pool's growth does not depend on memory for it.
+static void drop_macro(AmrState* a) {
+    dfree(a, a->macro);
+    a->macro_blocks = 0;
 }
 
 // Reallocate the arrays sized by the level-1 capacity; keep: the payload the migration reads and
@@ -317,7 +318,8 @@ static jp_status set_cap1(jp_solver* s, int cap, bool keep) {
     ACK(cudaMemsetAsync(a->ref1, 0, sizeof(int) * cap, s->stream), "memset");
     a->cap1 = cap;
     update_bytes(s);
-    return regrow_macro(s);
+    drop_macro(a);
+    return JP_OK;
 }
 
 static jp_status set_cap2(jp_solver* s, int cap, bool keep) {
@@ -333,7 +335,8 @@ static jp_status set_cap2(jp_solver* s, int cap, bool keep) {
     reset_graphs(a);
     a->cap2 = cap;
     update_bytes(s);
-    return regrow_macro(s);
+    drop_macro(a);
+    return JP_OK;
 }
 
 // Pools grow on overflow instead of being written past their end (the reference sizes them with
@@ -484,7 +487,7 @@ static jp_status initial_build(jp_solver* s) {
         a->cap2 = 8;
     }
     if (a->nf2 > a->cap2) return fail(JP_ERR_CAPACITY, "level-2 pool overflow: %d > %d", a->nf2, a->cap2);
-    dfree(a, a->macro);  // sized by the level-2 capacity: allocated again by the next diagnostic
+    drop_macro(a);
     dfree(a, a->f2a);
     dfree(a, a->f2b);
     dfree(a, a->gh2);
@@ -1341,12 +1344,21 @@ jp_status amr_get_output_fields(jp_solver* s, float* q, float* speed, float* vel
     return output_fields_from(s, a->field, false, false, a->N2, q, speed, vel);
 }
 
-// the diagnostics' macro buffer, for the blocks the pools hold (amr_prepare_diag: ahead of an amr_diag_async on
-// another stream)
+// The diagnostics' macro buffer (amr_prepare_diag: ahead of an amr_diag_async on another stream), for the grid at
+// hand: sized by the blocks the pools hold, so that regrids within them keep it, or where there is no memory for
+// that by the grid's own.
+static size_t grid_blocks(const AmrState* a) { return (size_t)a->cnb0 + a->nf1 + a->nf2; }
 static jp_status ensure_macro(jp_solver* s) {
     AmrState* a = s->amr;
-    if (a->macro) return JP_OK;
-    return dalloc(a, &a->macro, 4 * ((size_t)a->cnb0 + a->cap1 + a->cap2) * a->MB3, "cudaMalloc leaf macro values");
+    if (a->macro && a->macro_blocks >= grid_blocks(a)) return JP_OK;
+    drop_macro(a);
+    jp_status st = JP_OK;
+    for (const size_t blocks : {(size_t)a->cnb0 + a->cap1 + a->cap2, grid_blocks(a)}) {
+        st = dalloc(a, &a->macro, 4 * blocks * a->MB3, "cudaMalloc leaf macro values");
+        if (st == JP_OK) a->macro_blocks = blocks;
+        if (st != JP_ERR_NOMEM) return st;
+    }
+    return st;
 }
 
 // out[3]: device or pinned host memory
@@ -1371,6 +1383,7 @@ static jp_status launch_diag(jp_solver* s, cudaStream_t st, double* out) {
 }
 
 jp_status amr_prepare_diag(jp_solver* s) {
+    if (s->amr->macro && s->amr->macro_blocks >= grid_blocks(s->amr)) return JP_OK;
     TRY(ensure_macro(s));
     ACK(wait_stream(s), "leaf macro values");
     return JP_OK;
@@ -1378,7 +1391,8 @@ jp_status amr_prepare_diag(jp_solver* s) {
 
 // the diagnostics of the current state on another stream, into pinned host_out[3]; buffers prepared before
 jp_status amr_diag_async(jp_solver* s, cudaStream_t st, double* host_out) {
-    if (!s->amr->macro) return fail(JP_ERR_STATE, "amr_diag_async: buffers not prepared");
+    if (!s->amr->macro || s->amr->macro_blocks < grid_blocks(s->amr))
+        return fail(JP_ERR_STATE, "amr_diag_async: buffers not prepared");
     return launch_diag(s, st, host_out);
 }
 

@@ -51,10 +51,20 @@ static void set_grid(int nref0, int nref1) {
     grid.n_skin0 = nref0;
     grid.n_skin1 = nref1;
 }
+static jp_solver* watched = nullptr;  // its level-1 capacity decides whether the grid overflows
 static void supply_grid() {
     fake::on_d2h = [](void* dst, size_t bytes) {
-        if (bytes == sizeof(AdaptCounts)) std::memcpy(dst, &grid, bytes);
+        if (bytes != sizeof(AdaptCounts)) return;
+        jp_amr_counts c;
+        const bool over = watched && jp_amr_get_counts(watched, &c) == JP_OK && grid.nf1 > c.cap1;
+        grid.err = over ? jp::amr::ADAPT_ERR_CAP1 : 0;
+        std::memcpy(dst, &grid, bytes);
     };
+}
+// k_leaf_macro writes the values of every unit of its grid
+static void check_leaf_macro(fake::Op& o) {
+    if (is(o, "k_leaf_macro") && fake::room(arg<const void*>(o, 4)) < (size_t)o.grid.x * 512 * 16)
+        fake::fault("k_leaf_macro past its buffer");
 }
 
 // Every list of the coarse step grows from a count that a fill has set to zero: on every route through an
@@ -94,9 +104,63 @@ static void regrid_orders_list_counts() {
     jp_destroy(s);
 }
 
+// Whichever allocation of a pool's growth fails, a later diagnostic writes within its buffer: also once
+// there is memory again and a grid is built that the grown capacities hold.
+static void growth_out_of_memory_then_diag() {
+    supply_grid();
+    fake::on_kernel = check_leaf_macro;
+    double d[3];
+    for (const bool level1 : {false, true}) {
+        for (int k = 0; k < 80; ++k) {
+            set_grid(16, 10);
+            jp_solver* s = watched = amr(64.0);
+            CHECK(jp_diag(s, d) == JP_OK);
+            if (level1) set_grid(40, 10);   // 320 blocks, 184 held
+            else set_grid(16, 40);          // 320 blocks, 200 held
+            fake::fail_from = fake::fail_to = fake::allocations + k;
+            const jp_status grown = jp_regrid(s);
+            const bool reached = fake::allocations > fake::fail_from;
+            fake::fail_to = -1;
+            CHECK(grown == (reached ? JP_ERR_NOMEM : JP_OK));
+            if (level1) set_grid(45, 20);
+            else set_grid(22, 48);
+            jp_status st = jp_regrid(s);
+            if (st == JP_ERR_STATE) st = jp_init_tgv(s);
+            CHECK(st == JP_OK);
+            CHECK(jp_diag(s, d) == JP_OK);
+            jp_destroy(s);
+            watched = nullptr;
+            if (!reached) break;
+        }
+    }
+}
+
+// Out of memory for a buffer of the pools' size, a diagnostic takes one of the grid's own.
+static void diag_buffer_of_the_grid() {
+    supply_grid();
+    fake::on_kernel = check_leaf_macro;
+    double d[3];
+    set_grid(16, 10);
+    jp_solver* s = amr(64.0);
+    fake::fail_from = fake::fail_to = fake::allocations;
+    CHECK(jp_diag(s, d) == JP_OK);
+    fake::fail_to = -1;
+    set_grid(22, 20);
+    CHECK(jp_regrid(s) == JP_OK);
+    CHECK(jp_diag(s, d) == JP_OK);
+    const long long held = fake::allocations;
+    set_grid(16, 24);
+    CHECK(jp_regrid(s) == JP_OK);
+    CHECK(jp_diag(s, d) == JP_OK);
+    CHECK(fake::allocations == held);  // a regrid within the pools keeps the buffer
+    jp_destroy(s);
+}
+
 int main(int argc, char** argv) {
     const std::map<std::string, void (*)()> checks = {
         {"regrid_orders_list_counts", regrid_orders_list_counts},
+        {"growth_out_of_memory_then_diag", growth_out_of_memory_then_diag},
+        {"diag_buffer_of_the_grid", diag_buffer_of_the_grid},
     };
     const auto it = argc == 2 ? checks.find(argv[1]) : checks.end();
     if (it == checks.end()) return 2;

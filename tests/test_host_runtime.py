@@ -32,7 +32,8 @@ def checks(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("name", ["regrid_orders_list_counts"])
+@pytest.mark.parametrize("name", ["regrid_orders_list_counts", "growth_out_of_memory_then_diag",
+                                  "diag_buffer_of_the_grid"])
 def test_host_code(checks, name):
     r = subprocess.run([checks, name], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout + r.stderr

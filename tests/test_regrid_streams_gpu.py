@@ -66,3 +66,22 @@ def test_regrids_beside_busy_streams_bit_exact(storage):
             assert a == b
         else:
             np.testing.assert_array_equal(a, b)
+
+
+def test_diagnostics_after_a_pool_grew(tmp_path):
+    # the buffer of the first diagnostic belongs to the smaller pools; a solver that loads the state, which has
+    # not taken a diagnostic before, gives the same numbers
+    n = 32
+    kw = dict(n=n, re=800.0, l1_mode="sensor", l2_mode="sensor", frac1=0.1, frac2=0.1, develop_steps=2, max_gb=16.0)
+    with J.Solver("amr", **kw) as s, J.Solver("amr", **kw) as t:
+        s.diag()
+        cap = s.counts()
+        s.set_sensor_override(np.ones(cap["cnb0"], dtype=np.float32), np.ones((2 * n // 8) ** 3, dtype=np.float32))
+        s.regrid()                                           # every block ties at the threshold
+        grown = s.counts()
+        assert grown["cap1"] > cap["cap1"] and grown["cap2"] > cap["cap2"]
+        s.step(1)
+        p = str(tmp_path / "grown.jps")
+        s.save_state(p)
+        t.load_state(p)
+        assert s.diag() == t.diag()
