@@ -254,7 +254,10 @@ typedef struct jp_amr_counts {
 
 /* Rebuild the refinement from the current state: sensor, exact threshold, marks, tables, migration of
  * the fine payloads, skin lists (gpurce_regrid, src/tgv3d_amr.cu:722-764).  Synchronous; only block
- * counts cross to the host.  JP_ERR_CAPACITY if a pool would overflow. */
+ * counts cross to the host.  JP_ERR_CAPACITY if a pool would overflow and max_gb allows no growth: on level 1
+ * the previous grid stays and the solve goes on.  On level 2 the next grid is half built by then: after
+ * that, as after any other failure half-way (JP_ERR_NOMEM), the solver holds the coarse level alone, and jp_step,
+ * jp_diag, jp_regrid and ensemble steps return JP_ERR_STATE until jp_init_tgv or jp_load_state. */
 jp_status jp_regrid(jp_solver* s);
 
 /* Block counts, capacities and high-water marks of an AMR solver. */

@@ -152,10 +152,15 @@ jp_status jp_init_tgv(jp_solver* s) {
     return s->kind == JP_UNIFORM ? uniform_init(s) : amr_init(s);
 }
 
+static jp_status not_ready() {
+    return fail(JP_ERR_STATE, "no state to work on (created with JP_FLAG_DEFER_INIT, or an adaptation failed half-way): "
+                "call jp_init_tgv first");
+}
+
 jp_status jp_step(jp_solver* s, int64_t nsteps) {
     if (!s) return fail(JP_ERR_INVALID, "null solver");
     if (nsteps < 0) return fail(JP_ERR_INVALID, "negative step count");
-    if (!s->initialized) return fail(JP_ERR_STATE, "solver created with JP_FLAG_DEFER_INIT: call jp_init_tgv first");
+    if (!s->initialized) return not_ready();
     cudaSetDevice(s->device);
     return s->kind == JP_UNIFORM ? uniform_step(s, nsteps) : amr_step(s, nsteps);
 }
@@ -169,7 +174,7 @@ jp_status jp_sync(jp_solver* s) {
 
 jp_status jp_diag(jp_solver* s, double out[3]) {
     if (!s || !out) return fail(JP_ERR_INVALID, "jp_diag: null argument");
-    if (!s->initialized) return fail(JP_ERR_STATE, "solver created with JP_FLAG_DEFER_INIT: call jp_init_tgv first");
+    if (!s->initialized) return not_ready();
     cudaSetDevice(s->device);
     return s->kind == JP_UNIFORM ? uniform_diag(s, out) : amr_diag(s, out);
 }
@@ -241,7 +246,7 @@ static jp_status need_amr(const jp_solver* s) {
 jp_status jp_regrid(jp_solver* s) {
     jp_status st = need_amr(s);
     if (st != JP_OK) return st;
-    if (!s->initialized) return fail(JP_ERR_STATE, "solver created with JP_FLAG_DEFER_INIT: call jp_init_tgv first");
+    if (!s->initialized) return not_ready();
     cudaSetDevice(s->device);
     return amr_regrid(s);
 }

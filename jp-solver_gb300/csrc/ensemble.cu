@@ -259,6 +259,10 @@ jp_status jp_ensemble_step(jp_ensemble* e, int64_t nsteps) {
     if (!e) return fail(JP_ERR_INVALID, "null ensemble");
     if (nsteps < 0) return fail(JP_ERR_INVALID, "negative step count");
     ECK(cudaSetDevice(e->device), "cudaSetDevice");
+    for (jp_solver* m : e->members)
+        if (m->kind == JP_AMR && !m->initialized)
+            return fail(JP_ERR_STATE, "an AMR member has no grid (JP_FLAG_DEFER_INIT, or an adaptation failed half-way): "
+                        "call jp_init_tgv first");
     for (jp_solver* m : e->members) {  // after each member's pending work
         if (m->kind == JP_UNIFORM && nsteps > 0) {  // populations staged for the next step
             const jp_status taken = uniform_take_staged(m);

@@ -362,7 +362,7 @@ static jp_status grow_l2(jp_solver* s, int needed) {
 }
 
 // exclusive scan of the marks and the level-1 tables; on overflow of the level-1 pool nothing is
-// written, the pool grows and the tables are built again.  If the pool cannot grow the error stands
+// written, the pool grows and the tables are built again.  If the budget allows no growth the error stands
 // and, in a regrid (restore_marks), the previous marks come back: the old grid stays valid.
 static jp_status build_l1(jp_solver* s, bool restore_marks) {
     AmrState* a = s->amr;
@@ -371,13 +371,14 @@ static jp_status build_l1(jp_solver* s, bool restore_marks) {
     TRY(read_counts(s));
     if (a->cnt_host->err & ADAPT_ERR_CAP1) {
         jp_status g = grow_l1(s, a->cnt_host->nf1);
+        if (g != JP_ERR_CAPACITY) s->initialized = false;  // the old grid's tables went with the arrays
         if (g == JP_OK) {
             a->cnt_host->err = 0;
             ACK(cudaMemsetAsync(&a->cnt_dev->err, 0, sizeof(int), s->stream), "counts");
             ACK(adapt_build_l1(a->ref0, a->cnb0, a->cgx, a->l1gx, a->cap1, a->rank, a->fof0, a->rl0, a->pcb, a->oct,
                                a->l1grid, a->f1pos, a->cnt_dev, s->stream), "build L1");
             TRY(read_counts(s));
-        } else if (restore_marks) {
+        } else if (restore_marks && g == JP_ERR_CAPACITY) {
             ACK(cudaMemcpyAsync(a->ref0, a->o_ref0, sizeof(int) * a->cnb0, cudaMemcpyDeviceToDevice, s->stream), "restore");
             ACK(wait_stream(s), "restore");
             return g;
@@ -557,6 +558,7 @@ static jp_status regrid(jp_solver* s) {
                        a->o_ref1, a->o_fof1, a->cap1, a->cnt_dev, s->stream), "snapshot");
     TRY(mark_l0_by_sensor(s));
     TRY(build_l1(s, true));
+    s->initialized = false;  // between two grids until amr_regrid has seen the end of this
     // the list counts go to zero ahead of the fork: both streams add to them (fill list 1 and the prep lists on
     // the side, fill list 2 on the solver's own)
     TRY(clear_lists(s, s->stream));
@@ -597,7 +599,7 @@ static jp_status regrid(jp_solver* s) {
         a->nf2 = a->cnt_host->nf2;
         a->ndeep = a->cnt_host->ndeep;
         a->hw_nf2 = std::max(a->hw_nf2, (long long)a->nf2);
-        if (a->nf2 > a->cap2) TRY(grow_l2(s, a->nf2));  // on failure the solver needs jp_init_tgv
+        if (a->nf2 > a->cap2) TRY(grow_l2(s, a->nf2));
     }
     // the skins need the marks of both levels (settled: read_counts waited); the host's counts are set
     ACK(cudaEventRecord(a->fk.fork2, s->stream), "fork");
@@ -1251,8 +1253,28 @@ void amr_destroy(jp_solver* s) {
     s->amr = nullptr;
 }
 
+// An adaptation that failed half-way leaves tables of two grids, or block counts that the pools do not hold.  The
+// solver goes back to what JP_FLAG_DEFER_INIT creates: the coarse level alone, no fine blocks, not
+// initialised (capi.cu refuses steps, diagnostics and regrids), so that whatever else is called reads and
+// writes within its arrays.
+static void drop_grid(jp_solver* s) {
+    AmrState* a = s->amr;
+    reset_graphs(a);
+    a->nref0 = a->nf1 = a->nref1 = a->nf2 = a->n_skin0 = a->n_skin1 = a->ndeep = 0;
+    a->skins_pending = false;
+    if (!a->l2oct) a->cap2 = 0;  // the last of the level-2 arrays that initial_build allocates
+    cudaMemsetAsync(a->l1grid, 0xFF, sizeof(int) * a->NG1, s->stream);
+    cudaMemsetAsync(a->ref0, 0, sizeof(int) * a->cnb0, s->stream);
+    cudaMemsetAsync(a->fof0, 0xFF, sizeof(int) * a->cnb0, s->stream);
+    cudaMemsetAsync(a->ref1, 0, sizeof(int) * a->cap1, s->stream);
+    cudaMemsetAsync(a->fof1, 0xFF, sizeof(int) * a->cap1, s->stream);
+    cudaMemsetAsync(a->step_cnt, 0, sizeof(int) * SC_ALL, s->stream);
+    wait_stream(s);  // the call that failed has its status; a failure here is the next call's
+    update_bytes(s);
+}
+
 // TGV state on the coarse grid and the initial build (with the sensor override, if one is set)
-jp_status amr_init(jp_solver* s) {
+static jp_status init_grid(jp_solver* s) {
     AmrState* a = s->amr;
     reset_graphs(a);
     AmrLaunch L;
@@ -1268,9 +1290,15 @@ jp_status amr_init(jp_solver* s) {
     skins_landed(a);
     reset_graphs(a);  // the level-2 pool was allocated anew
     s->step_count = 0;
-    s->initialized = true;
     update_bytes(s);
     return JP_OK;
+}
+jp_status amr_init(jp_solver* s) {
+    s->initialized = false;
+    const jp_status st = init_grid(s);
+    if (st == JP_OK) s->initialized = true;
+    else drop_grid(s);
+    return st;
 }
 
 // Without JP_FLAG_GRAPH a coarse step is captured once its case (graph_key) has been launched kCaptureAfter times:
@@ -1314,10 +1342,18 @@ jp_status amr_set_step_map(jp_solver* s, int vec, int tpb) {
 }
 
 jp_status amr_regrid(jp_solver* s) {
-    TRY(regrid(s));  // the captured steps stay valid unless a pool grew (grow_l1/grow_l2 drop them)
-    ACK(wait_stream(s), "regrid");
-    skins_landed(s->amr);
-    return JP_OK;
+    jp_status st = regrid(s);  // the captured steps stay valid unless a pool grew (grow_l1/grow_l2 drop them)
+    if (st == JP_OK) {
+        const cudaError_t e = wait_stream(s);
+        if (e != cudaSuccess) st = cuda_fail(e, "regrid");
+    }
+    if (st == JP_OK) {
+        skins_landed(s->amr);
+        s->initialized = true;
+    } else if (!s->initialized) {
+        drop_grid(s);
+    }
+    return st;
 }
 
 static jp_status composite(jp_solver* s) {

@@ -156,11 +156,68 @@ static void diag_buffer_of_the_grid() {
     jp_destroy(s);
 }
 
+// A regrid whose level-2 blocks neither fit nor may grow leaves no count that the pools do not hold: the calls that
+// need a grid refuse, every other stays within its arrays, and a new initial state or a state file brings the
+// solver back.
+static void refused_level2_growth_leaves_no_grid() {
+    supply_grid();
+    fake::on_kernel = check_leaf_macro;
+    double d[3];
+    set_grid(16, 10);
+    const std::string path = "refused.jps";
+    jp_solver* s = watched = amr(0.075);  // 384 blocks of 184,589 bytes, not 584
+    CHECK(jp_diag(s, d) == JP_OK);
+    CHECK(jp_save_state(s, path.c_str()) == JP_OK);
+    jp_ensemble* e = nullptr;
+    CHECK(jp_ensemble_create(0, &e) == JP_OK && jp_ensemble_add(e, s) == JP_OK);
+    for (int k = 0; k < 2; ++k) {
+        set_grid(20, 40);  // 320 blocks, 200 held
+        CHECK(jp_regrid(s) == JP_ERR_CAPACITY);
+        CHECK(jp_diag(s, d) == JP_ERR_STATE);
+        CHECK(jp_step(s, 1) == JP_ERR_STATE);
+        CHECK(jp_regrid(s) == JP_ERR_STATE);
+        CHECK(jp_ensemble_step(e, 1) == JP_ERR_STATE);
+        jp_amr_counts c;
+        CHECK(jp_amr_get_counts(s, &c) == JP_OK && c.nf1 <= c.cap1 && c.nf2 <= c.cap2);
+        std::vector<int> table(4096);
+        for (int t = JP_TABLE_REF0; t <= JP_TABLE_DEEP; ++t) {
+            int64_t n = 0;
+            CHECK(jp_get_table(s, t, table.data(), (int64_t)table.size(), &n) == JP_OK);
+        }
+        for (int level = 0; level < 3; ++level) {
+            int64_t n = 0;
+            CHECK(jp_population_count(s, level, &n) == JP_OK);
+            std::vector<double> p(n + 1);
+            CHECK(jp_get_populations(s, level, JP_LAYOUT_BLOCKED, JP_F32, p.data(), n) == JP_OK);
+            CHECK(jp_get_populations(s, level, JP_LAYOUT_BLOCKED, JP_F64, p.data(), n) == JP_OK);
+        }
+        CHECK(jp_save_state(s, "dropped.jps") == JP_OK);
+        set_grid(16, 10);
+        CHECK((k == 0 ? jp_init_tgv(s) : jp_load_state(s, path.c_str())) == JP_OK);
+        CHECK(jp_step(s, 1) == JP_OK && jp_diag(s, d) == JP_OK && jp_ensemble_step(e, 1) == JP_OK);
+        CHECK(jp_amr_get_counts(s, &c) == JP_OK && c.nf2 == 80);
+    }
+    set_grid(30, 10);  // level 1 refused: the grid at hand stays
+    CHECK(jp_regrid(s) == JP_ERR_CAPACITY);
+    jp_amr_counts c;
+    CHECK(jp_amr_get_counts(s, &c) == JP_OK && c.nf1 == 128 && c.nf2 == 80);
+    CHECK(jp_step(s, 1) == JP_OK && jp_diag(s, d) == JP_OK);
+    set_grid(16, 40);  // an initial build that does not fit
+    CHECK(jp_init_tgv(s) == JP_ERR_CAPACITY);
+    CHECK(jp_diag(s, d) == JP_ERR_STATE);
+    CHECK(jp_amr_get_counts(s, &c) == JP_OK && c.nf2 <= c.cap2);
+    set_grid(16, 10);
+    CHECK(jp_init_tgv(s) == JP_OK && jp_diag(s, d) == JP_OK);
+    jp_ensemble_destroy(e);
+    jp_destroy(s);
+}
+
 int main(int argc, char** argv) {
     const std::map<std::string, void (*)()> checks = {
         {"regrid_orders_list_counts", regrid_orders_list_counts},
         {"growth_out_of_memory_then_diag", growth_out_of_memory_then_diag},
         {"diag_buffer_of_the_grid", diag_buffer_of_the_grid},
+        {"refused_level2_growth_leaves_no_grid", refused_level2_growth_leaves_no_grid},
     };
     const auto it = argc == 2 ? checks.find(argv[1]) : checks.end();
     if (it == checks.end()) return 2;

@@ -1,4 +1,4 @@
-"""Regrids of an AMR solve beside other work on the device, on a GB300.
+"""Regrids of an AMR solve, on a GB300: beside other work on the device, with pools that grow, and refused.
 
 A regrid builds its tables and lists on two streams; what it leaves must not depend on how these are scheduled.
 The same run of steps and regrids, alone and while an ensemble of other solves keeps the device busy from
@@ -85,3 +85,43 @@ def test_diagnostics_after_a_pool_grew(tmp_path):
         s.save_state(p)
         t.load_state(p)
         assert s.diag() == t.diag()
+
+
+def test_refused_level2_growth_needs_a_new_state(tmp_path):
+    # ties on level 1 ask for more level-2 blocks than the budget holds: the regrid reports it, the calls that need
+    # a grid refuse, and a state file or a new initial state brings the solve back to the same bits
+    n, cnb0, ng1 = 32, 64, 512
+    rng = np.random.default_rng(3)
+    sen0 = (2.0 * (np.arange(cnb0) < cnb0 // 2) + 0.5 * rng.random(cnb0)).astype(np.float32)
+    with J.Solver("amr", n=n, re=800.0, l1_mode="sensor", l2_mode="sensor", frac1=0.5, frac2=0.1, develop_steps=2,
+                  max_gb=0.11, flags=J.FLAG_DEFER_INIT) as s:
+        distinct = rng.random(ng1).astype(np.float32)
+
+        def start():
+            s.set_sensor_override(sen0, distinct)
+            s.init_tgv()
+            s.step(2)
+            return s.diag()
+
+        first = start()
+        assert 0 < s.counts()["nf2"] <= s.counts()["cap2"] < 1024
+        p = str(tmp_path / "ok.jps")
+        s.save_state(p)
+        for back in ("load", "init"):
+            s.set_sensor_override(sen0, np.ones(ng1, dtype=np.float32))
+            with pytest.raises(J.JPError) as x:
+                s.regrid()
+            assert x.value.status == 3                           # JP_ERR_CAPACITY
+            for call in (s.diag, s.regrid, lambda: s.step(1)):
+                with pytest.raises(J.JPError) as x:
+                    call()
+                assert x.value.status == 5                       # JP_ERR_STATE
+            c = s.counts()
+            assert c["nf1"] == c["nf2"] == 0
+            assert [s.population_count(lv) for lv in range(3)] == [19 * n ** 3, 0, 0]
+            assert s.output_fields()[0].size == (4 * n) ** 3     # of the coarse level
+            if back == "load":
+                s.load_state(p)
+                assert s.diag() == first
+            else:
+                assert start() == first
