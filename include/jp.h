@@ -74,7 +74,10 @@ typedef struct jp_config {
     double max_gb;           /* HBM ceiling for the fine pools in GiB; 0 = 75% of free memory */
     int32_t device;          /* CUDA device ordinal */
     int32_t threads_per_block; /* 0 = default; uniform: 64..512; AMR steps: 64 (MB=4), 128/256/512 */
-    int32_t vec;             /* cells per thread along x in the uniform step; 0 = tuned default */
+    int32_t vec;             /* cells per thread along x in the uniform step; 0 = tuned default.  A uniform
+                                solver with vec or threads_per_block set takes every step alone in that
+                                mapping; with both 0, FP32 steps go two in one pass where that is faster
+                                (the same bits) */
     int32_t flags;           /* JP_FLAG_* */
     int32_t buffer;          /* AMR sensor modes: dilate the refinement marks by this many block layers
                                 (--buffer; parsed but unused by the reference, src/tgv3d_amr.cu:648) */
@@ -383,7 +386,8 @@ jp_status jp_server_get_stats(const jp_server* sv, jp_server_stats* out);
 /* ---- autotuning (extension; no counterpart in the reference) ------------------------- */
 
 /* Time `steps` steps of each candidate and write the fastest into *cfg: for a uniform solver the
- * thread mapping (cells per thread `vec` x `threads_per_block`), for an AMR solver the block edge
+ * thread mapping (cells per thread `vec` x `threads_per_block`; both 0 where the default mapping with
+ * two-step passes is faster than any mapping of single steps), for an AMR solver the block edge
  * `mb` in {4, 8, 16} dividing n and the threads per CTA of its level steps (`threads_per_block`
  * 64 at MB=4, else 128, 256 or 512; the reference fixes MB at compile time and MB=16 cannot run
  * there, its kernels would need 4096 threads per block).  *best receives the winner's lattice

@@ -27,7 +27,8 @@ extern "C" jp_status jp_autotune(jp_config* cfg, int32_t steps, double* best) {
         const int tpbs[4] = {64, 128, 256, 512};
         int bv = s->vec, bt = s->tpb;
         const double cells = double(s->cells);
-        // the mapping belongs to the single step; two-step passes, where they are used, do not follow it
+        // the mapping belongs to the single step; where two-step passes in the default mapping are faster than
+        // any, the answer is that (vec and threads_per_block 0)
         const bool two = s->pair.use;
         s->pair.use = false;
         for (int v : vecs) {
@@ -62,7 +63,11 @@ extern "C" jp_status jp_autotune(jp_config* cfg, int32_t steps, double* best) {
                 jp_destroy(s);
                 return st;
             }
-            *best = std::max(*best, cells * steps / (double(ms) * 1e-3));
+            const double rate = cells * steps / (double(ms) * 1e-3);
+            if (rate > *best) {
+                *best = rate;
+                bv = bt = 0;
+            }
         }
         jp_destroy(s);
         cfg->vec = bv;

@@ -136,7 +136,8 @@ jp_status uniform_create(jp_solver* s) {
     }
     JP_CK(cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, s->device), "cudaDeviceGetAttribute");
     s->solo_vec = pick_solo_vec(s);
-    if (!s->inplace && s->storage == JP_FP32) {
+    // a mapping that the caller chose is that of every step; two-step passes have one of their own
+    if (!s->inplace && s->storage == JP_FP32 && !c.vec && !c.threads_per_block) {
         s->pair = pair_plan(s->n, s->sms);
         s->pair_tile = pair_tile_plan(s->n, s->sms);
     }

@@ -42,7 +42,8 @@ int main(int argc, char** argv) {
     if (argd(argc, argv, "--autotune", 0.0) > 0.5) {
         double best = 0.0;
         ck(jp_autotune(&cfg, 10, &best), "autotune");
-        std::printf("[autotune] vec=%d threads/block=%d  %.1f MLUPS\n", cfg.vec, cfg.threads_per_block, best / 1e6);
+        if (cfg.vec) std::printf("[autotune] vec=%d threads/block=%d  %.1f MLUPS\n", cfg.vec, cfg.threads_per_block, best / 1e6);
+        else std::printf("[autotune] default mapping, two steps per pass  %.1f MLUPS\n", best / 1e6);
     }
     jp_solver* s = nullptr;
     ck(jp_create(&cfg, &s), "create");

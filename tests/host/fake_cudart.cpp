@@ -12,6 +12,7 @@ std::vector<std::string> faults;
 std::function<void(Op&)> on_kernel;
 std::function<void(void*, size_t)> on_d2h;
 std::function<cudaError_t(const std::string&)> launch_error;
+std::function<float()> elapsed;
 long long allocations = 0, fail_from = 1, fail_to = 0;
 size_t free_bytes = (size_t)64 << 30;
 
@@ -309,7 +310,7 @@ cudaError_t cudaEventSynchronize(cudaEvent_t e) {
 }
 cudaError_t cudaEventQuery(cudaEvent_t e) { return cudaEventSynchronize(e); }
 cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) {
-    *ms = 1.f;
+    *ms = elapsed ? elapsed() : 1.f;
     return cudaSuccess;
 }
 

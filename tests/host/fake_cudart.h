@@ -38,6 +38,7 @@ extern std::function<void(Op&)> on_kernel;                           // sees eve
 extern std::function<void(void* dst, size_t bytes)> on_d2h;          // after a device-to-host copy
 extern long long allocations;                                        // device allocations so far
 extern long long fail_from, fail_to;                                 // those with these indices fail
+extern std::function<float()> elapsed;                               // milliseconds between two events
 extern size_t free_bytes;                                            // what cudaMemGetInfo reports
 extern std::function<cudaError_t(const std::string& kernel)> launch_error;  // result of a launch
 // the allocation that holds p: bytes from p to its end (0: none)

@@ -212,12 +212,72 @@ static void refused_level2_growth_leaves_no_grid() {
     jp_destroy(s);
 }
 
+static int count(const char* kernel, size_t from) {
+    int n = 0;
+    for (size_t i = from; i < fake::ops.size(); ++i) n += is(fake::ops[i], kernel);
+    return n;
+}
+static jp_solver* cube(int n, int vec, int tpb) {
+    jp_config c;
+    jp_config_default(&c, JP_UNIFORM);
+    c.n = n;
+    c.vec = vec;
+    c.threads_per_block = tpb;
+    jp_solver* s = nullptr;
+    CHECK(jp_create(&c, &s) == JP_OK);
+    return s;
+}
+
+// A thread mapping that the caller chose is that of every step, alone and in an ensemble; with none, FP32 cubes of
+// these sizes step two at a time.  The autotuner answers with the mapping whose rate it reports.
+static void chosen_mapping_takes_every_step() {
+    const int maps[4][2] = {{0, 0}, {4, 0}, {0, 256}, {2, 128}};
+    for (const auto& m : maps) {
+        const bool chosen = m[0] || m[1];
+        jp_solver* s = cube(32, m[0], m[1]);
+        size_t from = fake::ops.size();
+        CHECK(jp_step(s, 5) == JP_OK);
+        CHECK(count("k_stream_collide_pair", from) == (chosen ? 0 : 2));
+        CHECK(count("k_stream_collide", from) == (chosen ? 5 : 3));
+        jp_destroy(s);
+        jp_ensemble* e = nullptr;
+        CHECK(jp_ensemble_create(0, &e) == JP_OK);
+        std::vector<jp_solver*> v;
+        for (int n : {32, 48, 64, 96, 128, 32, 48, 64, 96, 128}) {
+            v.push_back(cube(n, m[0], m[1]));
+            CHECK(jp_ensemble_add(e, v.back()) == JP_OK);
+        }
+        from = fake::ops.size();
+        CHECK(jp_ensemble_step(e, 5) == JP_OK);
+        CHECK(count("k_stream_collide_pair", from) == (chosen ? 0 : 2));
+        CHECK(count("k_stream_collide", from) == (chosen ? 5 : 3));
+        jp_ensemble_destroy(e);
+        for (jp_solver* x : v) jp_destroy(x);
+    }
+    for (const bool two_faster : {true, false}) {
+        // a single step takes 1 ms, a two-step pass 1.5 or 2.5
+        size_t from = fake::ops.size();
+        fake::elapsed = [&] {  // of four steps
+            return !is(fake::ops.back(), "k_stream_collide_pair") ? 4.f : two_faster ? 3.f : 5.f;
+        };
+        jp_config c;
+        jp_config_default(&c, JP_UNIFORM);
+        c.n = 32;
+        double best = 0;
+        CHECK(jp_autotune(&c, 4, &best) == JP_OK);
+        CHECK(count("k_stream_collide_pair", from) > 0);
+        CHECK((c.vec == 0) == two_faster && (c.threads_per_block == 0) == two_faster);
+        CHECK(best == 32.0 * 32 * 32 * 4 / ((two_faster ? 3.0 : 4.0) * 1e-3));
+    }
+}
+
 int main(int argc, char** argv) {
     const std::map<std::string, void (*)()> checks = {
         {"regrid_orders_list_counts", regrid_orders_list_counts},
         {"growth_out_of_memory_then_diag", growth_out_of_memory_then_diag},
         {"diag_buffer_of_the_grid", diag_buffer_of_the_grid},
         {"refused_level2_growth_leaves_no_grid", refused_level2_growth_leaves_no_grid},
+        {"chosen_mapping_takes_every_step", chosen_mapping_takes_every_step},
     };
     const auto it = argc == 2 ? checks.find(argv[1]) : checks.end();
     if (it == checks.end()) return 2;
