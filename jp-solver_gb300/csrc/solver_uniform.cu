@@ -26,7 +26,7 @@ BgkCoef bgk_coefficients(float omega) {
     const auto near3 = [](double x, float* v) {
         v[0] = float(x);
         v[1] = std::nextafter(v[0], 0.f);
-        v[2] = std::nextafter(v[0], 64.f);
+        v[2] = std::nextafter(v[0], INFINITY);
     };
     float b0[3], b1[3], b2[3], k1[3], k2[3];
     near3(om / 3, b0);

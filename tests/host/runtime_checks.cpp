@@ -5,8 +5,12 @@
 #include <cstdlib>
 #include <cstring>
 
+#include <algorithm>
+#include <cmath>
+
 #include "amr_kernels.h"
 #include "jp.h"
+#include "kernels.h"
 
 using jp::amr::AdaptCounts;
 
@@ -271,6 +275,31 @@ static void chosen_mapping_takes_every_step() {
     }
 }
 
+// The relaxation's coefficients are the combination of each value's nearest float and its two neighbours that
+// keeps mass best, at every viscosity (1 / (omega w) is above 64 for omega below 0.28).
+static void coefficients_search_both_neighbours() {
+    for (float omega : {1.99f, 1.6f, 1.0f, 0.5f, 0.29f, 0.27f, 0.2f, 0.1357f, 0.08f, 0.031f, 0.0021f, 3.3e-5f}) {
+        const jp::BgkCoef c = jp::bgk_coefficients(omega);
+        const double om = omega;
+        const auto off = [&](double b0, double b1, double b2, double k1, double k2) {
+            const double c0 = b0 + 6 * b1 + 12 * b2;
+            const double k = k1 * (double(c.a1) * c.a1) + 4 * k2 * (double(c.a2) * c.a2);
+            return std::fabs(2 * k - 1.5 * c0) + 0.1 * std::fabs(c0 - om);
+        };
+        std::vector<float> v[5];
+        const double exact[5] = {om / 3, om / 18, om / 36, 9 / om, 18 / om};
+        for (int i = 0; i < 5; ++i)
+            for (float to : {-INFINITY, float(exact[i]), INFINITY}) v[i].push_back(std::nextafter(float(exact[i]), to));
+        double least = INFINITY;
+        for (float b0 : v[0])
+            for (float b1 : v[1])
+                for (float b2 : v[2])
+                    for (float k1 : v[3])
+                        for (float k2 : v[4]) least = std::min(least, off(b0, b1, b2, k1, k2));
+        CHECK(off(c.b0, c.b1, c.b2, c.k1, c.k2) == least);
+    }
+}
+
 int main(int argc, char** argv) {
     const std::map<std::string, void (*)()> checks = {
         {"regrid_orders_list_counts", regrid_orders_list_counts},
@@ -278,6 +307,7 @@ int main(int argc, char** argv) {
         {"diag_buffer_of_the_grid", diag_buffer_of_the_grid},
         {"refused_level2_growth_leaves_no_grid", refused_level2_growth_leaves_no_grid},
         {"chosen_mapping_takes_every_step", chosen_mapping_takes_every_step},
+        {"coefficients_search_both_neighbours", coefficients_search_both_neighbours},
     };
     const auto it = argc == 2 ? checks.find(argv[1]) : checks.end();
     if (it == checks.end()) return 2;

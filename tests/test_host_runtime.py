@@ -32,8 +32,14 @@ def checks(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("name", ["regrid_orders_list_counts", "growth_out_of_memory_then_diag",
-                                  "diag_buffer_of_the_grid", "refused_level2_growth_leaves_no_grid", "chosen_mapping_takes_every_step"])
+@pytest.mark.parametrize("name", [
+    "regrid_orders_list_counts",
+    "growth_out_of_memory_then_diag",
+    "diag_buffer_of_the_grid",
+    "refused_level2_growth_leaves_no_grid",
+    "chosen_mapping_takes_every_step",
+    "coefficients_search_both_neighbours",
+])
 def test_host_code(checks, name, tmp_path):
     r = subprocess.run([checks, name], capture_output=True, text=True, timeout=120, cwd=tmp_path)
     assert r.returncode == 0, r.stdout + r.stderr
