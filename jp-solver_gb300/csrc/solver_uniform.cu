@@ -391,7 +391,6 @@ static jp_status uniform_convert(jp_solver* s, int layout, int dtype, void* host
                 s->io = nullptr;
                 return cuda_fail(e, "cudaMalloc population scratch");
             }
-            s->info.bytes_state += (int64_t)s->io_bytes;
         }
         scratch = s->io;
         bytes = s->io_bytes;

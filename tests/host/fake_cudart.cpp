@@ -13,7 +13,6 @@ std::function<void(Op&)> on_kernel;
 std::function<void(void*, size_t)> on_d2h;
 std::function<cudaError_t(const std::string&)> launch_error;
 std::function<float()> elapsed;
-std::function<void(size_t)> on_alloc;
 long long allocations = 0, fail_from = 1, fail_to = 0;
 size_t free_bytes = (size_t)64 << 30;
 
@@ -76,7 +75,6 @@ cudaError_t alloc(void** p, size_t n) {
     *p = nullptr;
     const long long k = allocations++;
     if (k >= fail_from && k <= fail_to) return cudaErrorMemoryAllocation;
-    if (on_alloc) on_alloc(n);
     *p = std::calloc(1, n);
     device[(const char*)*p] = n;
     return *p ? cudaSuccess : cudaErrorMemoryAllocation;

@@ -36,7 +36,6 @@ extern std::vector<Op> ops;
 extern std::vector<std::string> faults;                              // accesses outside an allocation
 extern std::function<void(Op&)> on_kernel;                           // sees every launch, with its arguments
 extern std::function<void(void* dst, size_t bytes)> on_d2h;          // after a device-to-host copy
-extern std::function<void(size_t bytes)> on_alloc;                   // every device allocation that succeeds
 extern long long allocations;                                        // device allocations so far
 extern long long fail_from, fail_to;                                 // those with these indices fail
 extern std::function<float()> elapsed;                               // milliseconds between two events
