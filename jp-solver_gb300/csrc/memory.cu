@@ -30,6 +30,18 @@ void dev_free(jp_solver* s, void* p) {
     }
 }
 
+cudaError_t scratch_alloc(jp_solver* s, void** p, size_t bytes) {
+    *p = nullptr;
+    if (s->pool) return cudaMallocFromPoolAsync(p, bytes, s->pool, s->stream);
+    return cudaMallocAsync(p, bytes, s->stream);
+}
+
+void scratch_free(jp_solver* s, void* p) {
+    if (!p) return;
+    cudaFreeAsync(p, s->stream);
+    if (!s->pool) cudaStreamSynchronize(s->stream);  // the pool trims itself when a stream is waited for
+}
+
 cudaError_t wait_stream(jp_solver* s) {
     if (!s->pool) return cudaStreamSynchronize(s->stream);
     if (!s->ev_wait) {

@@ -24,6 +24,10 @@ size_t storage_bytes(int storage);
 // run by a server: no device-wide synchronisation when they come and go), else cudaMalloc/cudaFree.
 cudaError_t dev_alloc(jp_solver* s, void** p, size_t bytes);
 void dev_free(jp_solver* s, void* p);
+// Device memory for the length of a call, on the solver's stream: its pool's, else the device's default pool, which
+// gives it back at the free.  Neither call waits for the device.
+cudaError_t scratch_alloc(jp_solver* s, void** p, size_t bytes);
+void scratch_free(jp_solver* s, void* p);
 // Small pinned host buffers (<= 256 bytes: diagnostic and count read-backs) from process-wide slabs
 // that are never returned to the driver, so creating and destroying solvers never calls
 // cudaFreeHost (which synchronises the device).
@@ -69,8 +73,6 @@ struct jp_solver {
     jp::PairPlan pair{};       // two steps in one pass, where pair.use (uniform_pair.cu)
     jp::PairPlan pair_tile{};  // the same in a launch of many cubes
     int sms = 0;               // multiprocessors of the device
-    void* io = nullptr;        // population conversion scratch of an in-place cube, allocated on first use
-    size_t io_bytes = 0;
     float* outbuf = nullptr;   // device Q / speed / velocity for output frames, allocated on first use
     // populations staged for the next step (jp_stage_populations): uploaded into `staging` on
     // copy_stream while the solver's stream works, swapped in as fa by the next step

@@ -169,8 +169,6 @@ void uniform_free(jp_solver* s) {
     dev_free(s, s->partials);
     pinned_slot_free(s->diag_host);
     dev_free(s, s->outbuf);
-    dev_free(s, s->io);
-    s->io = nullptr;
     s->outbuf = nullptr;
     s->fa = s->fb = s->field = nullptr;
     s->partials = s->diag_host = nullptr;
@@ -360,7 +358,7 @@ void uniform_flat_to_raw(const jp_solver* s, const unsigned char* flat, unsigned
 
 // Populations in another type or order than the state's, converted on the device.  The scratch is the next
 // step's target array, whose contents nothing reads between steps; an in-place cube takes an allocation of
-// 64 MiB, or what it can get of that down to 1 MiB, on first use.
+// 64 MiB, or what it can get of that down to 1 MiB, for the length of the call.
 static jp_status uniform_convert(jp_solver* s, int layout, int dtype, void* host, bool to_host_order) {
     PopMap m{};
     m.n = s->n;
@@ -379,23 +377,18 @@ static jp_status uniform_convert(jp_solver* s, int layout, int dtype, void* host
     void* scratch = s->fb;
     size_t bytes = (size_t)Q * s->cells * s->elem;
     if (s->inplace) {
-        if (!s->io) {
-            s->io_bytes = std::min(bytes, (size_t)64 << 20);
-            cudaError_t e = dev_alloc(s, &s->io, s->io_bytes);
-            while (e == cudaErrorMemoryAllocation && s->io_bytes > ((size_t)1 << 20)) {
-                cudaGetLastError();
-                s->io_bytes /= 2;
-                e = dev_alloc(s, &s->io, s->io_bytes);
-            }
-            if (e != cudaSuccess) {
-                s->io = nullptr;
-                return cuda_fail(e, "cudaMalloc population scratch");
-            }
+        bytes = std::min(bytes, (size_t)64 << 20);
+        cudaError_t e = scratch_alloc(s, &scratch, bytes);
+        while (e == cudaErrorMemoryAllocation && bytes > ((size_t)1 << 20)) {
+            cudaGetLastError();
+            bytes /= 2;
+            e = scratch_alloc(s, &scratch, bytes);
         }
-        scratch = s->io;
-        bytes = s->io_bytes;
+        if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc population scratch");
     }
-    return convert_populations(s, s->storage, dtype, m, s->fa, scratch, bytes, host, to_host_order);
+    const jp_status st = convert_populations(s, s->storage, dtype, m, s->fa, scratch, bytes, host, to_host_order);
+    if (s->inplace) scratch_free(s, scratch);
+    return st;
 }
 
 jp_status uniform_get_populations(jp_solver* s, int level, int layout, int dtype, void* host, int64_t count) {

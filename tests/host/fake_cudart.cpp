@@ -116,6 +116,11 @@ bool before(const Op& a, const Op& b) {
     const auto it = b.clock.find(&of(a.stream));
     return it != b.clock.end() && it->second >= a.at && &a != &b;
 }
+size_t allocated() {
+    size_t n = 0;
+    for (const auto& d : device) n += d.second;
+    return n;
+}
 size_t room(const void* p) {
     auto it = device.upper_bound((const char*)p);
     if (it == device.begin()) return 0;
@@ -222,6 +227,7 @@ cudaError_t cudaFree(void* p) {
     return cudaSuccess;
 }
 cudaError_t cudaMallocFromPoolAsync(void** p, size_t n, cudaMemPool_t, cudaStream_t) { return keep(alloc(p, n)); }
+cudaError_t cudaMallocAsync(void** p, size_t n, cudaStream_t) { return keep(alloc(p, n)); }
 cudaError_t cudaFreeAsync(void* p, cudaStream_t) {
     release(p);
     return cudaSuccess;

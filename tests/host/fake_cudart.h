@@ -41,6 +41,7 @@ extern long long fail_from, fail_to;                                 // those wi
 extern std::function<float()> elapsed;                               // milliseconds between two events
 extern size_t free_bytes;                                            // what cudaMemGetInfo reports
 extern std::function<cudaError_t(const std::string& kernel)> launch_error;  // result of a launch
+size_t allocated();  // device bytes allocated now
 // the allocation that holds p: bytes from p to its end (0: none)
 size_t room(const void* p);
 void fault(const std::string& what);

@@ -221,12 +221,13 @@ static int count(const char* kernel, size_t from) {
     for (size_t i = from; i < fake::ops.size(); ++i) n += is(fake::ops[i], kernel);
     return n;
 }
-static jp_solver* cube(int n, int vec, int tpb) {
+static jp_solver* cube(int n, int vec, int tpb, int flags = 0) {
     jp_config c;
     jp_config_default(&c, JP_UNIFORM);
     c.n = n;
     c.vec = vec;
     c.threads_per_block = tpb;
+    c.flags = flags;
     jp_solver* s = nullptr;
     CHECK(jp_create(&c, &s) == JP_OK);
     return s;
@@ -300,6 +301,26 @@ static void coefficients_search_both_neighbours() {
     }
 }
 
+// An in-place cube holds one population array: the memory that a conversion takes goes back with it.
+static void in_place_conversions_keep_no_memory() {
+    for (const int n : {8, 32, 64}) {
+        jp_solver* s = cube(n, 0, 0, JP_FLAG_INPLACE);
+        const int64_t count = 19LL * n * n * n;
+        std::vector<double> p(count);
+        jp_info before, after;
+        CHECK(jp_get_info(s, &before) == JP_OK);
+        const size_t held = fake::allocated();
+        for (int k = 0; k < 2; ++k) {
+            CHECK(jp_get_populations(s, 0, JP_LAYOUT_FLAT, JP_F64, p.data(), count) == JP_OK);
+            CHECK(fake::allocated() == held);
+            CHECK(jp_set_populations(s, 0, JP_LAYOUT_BLOCKED, JP_F32, p.data(), count) == JP_OK);
+            CHECK(fake::allocated() == held);
+        }
+        CHECK(jp_get_info(s, &after) == JP_OK && after.bytes_state == before.bytes_state);
+        jp_destroy(s);
+    }
+}
+
 int main(int argc, char** argv) {
     const std::map<std::string, void (*)()> checks = {
         {"regrid_orders_list_counts", regrid_orders_list_counts},
@@ -308,6 +329,7 @@ int main(int argc, char** argv) {
         {"refused_level2_growth_leaves_no_grid", refused_level2_growth_leaves_no_grid},
         {"chosen_mapping_takes_every_step", chosen_mapping_takes_every_step},
         {"coefficients_search_both_neighbours", coefficients_search_both_neighbours},
+        {"in_place_conversions_keep_no_memory", in_place_conversions_keep_no_memory},
     };
     const auto it = argc == 2 ? checks.find(argv[1]) : checks.end();
     if (it == checks.end()) return 2;
