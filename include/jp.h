@@ -170,7 +170,8 @@ jp_status jp_population_count(const jp_solver* s, int32_t level, int64_t* count)
 /* Copy the populations of `level` to a host buffer of `count` values of type `dtype`, in `layout`.
  * Shifted FP16/BF16 storage is returned unshifted (f = w_q + stored).  Another type or order than the
  * state's is converted on the device, through memory of the solver that holds nothing between steps (an
- * in-place cube allocates up to 64 MiB for the length of the call). */
+ * in-place cube allocates up to 64 MiB for the length of the call; where there is no memory for that it
+ * converts 32 KiB at a time). */
 jp_status jp_get_populations(jp_solver* s, int32_t level, int32_t layout, int32_t dtype,
                              void* host, int64_t count);
 

@@ -73,6 +73,7 @@ struct jp_solver {
     jp::PairPlan pair{};       // two steps in one pass, where pair.use (uniform_pair.cu)
     jp::PairPlan pair_tile{};  // the same in a launch of many cubes
     int sms = 0;               // multiprocessors of the device
+    void* io = nullptr;        // in-place cubes: population conversion scratch for when there is no memory left
     float* outbuf = nullptr;   // device Q / speed / velocity for output frames, allocated on first use
     // populations staged for the next step (jp_stage_populations): uploaded into `staging` on
     // copy_stream while the solver's stream works, swapped in as fa by the next step

@@ -112,6 +112,10 @@ static int pick_solo_vec(const jp_solver* s) {
     return ctas < (s->storage == JP_FP32 ? 4 : 2) * s->sms ? 2 : 4;
 }
 
+// Conversion scratch that an in-place cube is created with: one unit of any order and type (a block of edge 16, or
+// a row of up to 4096 cells, of doubles).
+constexpr size_t kIoBytes = 16 * 16 * 16 * 8;
+
 jp_status uniform_create(jp_solver* s) {
     jp_status st = common_setup(s);
     if (st != JP_OK) return st;
@@ -145,6 +149,7 @@ jp_status uniform_create(jp_solver* s) {
     s->info.bytes_state = (int64_t)((s->inplace ? 1 : 2) * bytes);
     JP_CK(dev_alloc(s, &s->fa, bytes), "cudaMalloc populations");
     if (!s->inplace) JP_CK(dev_alloc(s, &s->fb, bytes), "cudaMalloc populations");
+    if (s->inplace) JP_CK(dev_alloc(s, &s->io, kIoBytes), "cudaMalloc population scratch");
     JP_CK(dev_alloc(s, (void**)&s->partials, sizeof(double) * kDiagPartials), "cudaMalloc partials");
     JP_CK(cudaMemsetAsync(diag_err_word(s->partials), 0, 2 * sizeof(int), s->stream), "clear diag error word");
     s->diag_host = (double*)pinned_slot_alloc();
@@ -169,6 +174,8 @@ void uniform_free(jp_solver* s) {
     dev_free(s, s->partials);
     pinned_slot_free(s->diag_host);
     dev_free(s, s->outbuf);
+    dev_free(s, s->io);
+    s->io = nullptr;
     s->outbuf = nullptr;
     s->fa = s->fb = s->field = nullptr;
     s->partials = s->diag_host = nullptr;
@@ -358,7 +365,8 @@ void uniform_flat_to_raw(const jp_solver* s, const unsigned char* flat, unsigned
 
 // Populations in another type or order than the state's, converted on the device.  The scratch is the next
 // step's target array, whose contents nothing reads between steps; an in-place cube takes an allocation of
-// 64 MiB, or what it can get of that down to 1 MiB, for the length of the call.
+// 64 MiB, or what it can get of that down to 1 MiB, for the length of the call, and where there is no memory for
+// that the few KiB it was created with.
 static jp_status uniform_convert(jp_solver* s, int layout, int dtype, void* host, bool to_host_order) {
     PopMap m{};
     m.n = s->n;
@@ -374,20 +382,26 @@ static jp_status uniform_convert(jp_solver* s, int layout, int dtype, void* host
         m.len = m.mb * m.mb * m.mb;
         m.units = Q * g * g * g;
     }
-    void* scratch = s->fb;
+    void *scratch = s->fb, *taken = nullptr;
     size_t bytes = (size_t)Q * s->cells * s->elem;
     if (s->inplace) {
         bytes = std::min(bytes, (size_t)64 << 20);
-        cudaError_t e = scratch_alloc(s, &scratch, bytes);
+        cudaError_t e = scratch_alloc(s, &taken, bytes);
         while (e == cudaErrorMemoryAllocation && bytes > ((size_t)1 << 20)) {
             cudaGetLastError();
             bytes /= 2;
-            e = scratch_alloc(s, &scratch, bytes);
+            e = scratch_alloc(s, &taken, bytes);
         }
-        if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc population scratch");
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            bytes = kIoBytes;
+        } else if (e != cudaSuccess) {
+            return cuda_fail(e, "cudaMalloc population scratch");
+        }
+        scratch = taken ? taken : s->io;
     }
     const jp_status st = convert_populations(s, s->storage, dtype, m, s->fa, scratch, bytes, host, to_host_order);
-    if (s->inplace) scratch_free(s, scratch);
+    scratch_free(s, taken);
     return st;
 }
 

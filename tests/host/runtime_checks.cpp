@@ -216,7 +216,7 @@ static void refused_level2_growth_leaves_no_grid() {
     jp_destroy(s);
 }
 
-static int count(const char* kernel, size_t from) {
+static int count_of(const char* kernel, size_t from) {
     int n = 0;
     for (size_t i = from; i < fake::ops.size(); ++i) n += is(fake::ops[i], kernel);
     return n;
@@ -242,8 +242,8 @@ static void chosen_mapping_takes_every_step() {
         jp_solver* s = cube(32, m[0], m[1]);
         size_t from = fake::ops.size();
         CHECK(jp_step(s, 5) == JP_OK);
-        CHECK(count("k_stream_collide_pair", from) == (chosen ? 0 : 2));
-        CHECK(count("k_stream_collide", from) == (chosen ? 5 : 3));
+        CHECK(count_of("k_stream_collide_pair", from) == (chosen ? 0 : 2));
+        CHECK(count_of("k_stream_collide", from) == (chosen ? 5 : 3));
         jp_destroy(s);
         jp_ensemble* e = nullptr;
         CHECK(jp_ensemble_create(0, &e) == JP_OK);
@@ -254,8 +254,8 @@ static void chosen_mapping_takes_every_step() {
         }
         from = fake::ops.size();
         CHECK(jp_ensemble_step(e, 5) == JP_OK);
-        CHECK(count("k_stream_collide_pair", from) == (chosen ? 0 : 2));
-        CHECK(count("k_stream_collide", from) == (chosen ? 5 : 3));
+        CHECK(count_of("k_stream_collide_pair", from) == (chosen ? 0 : 2));
+        CHECK(count_of("k_stream_collide", from) == (chosen ? 5 : 3));
         jp_ensemble_destroy(e);
         for (jp_solver* x : v) jp_destroy(x);
     }
@@ -270,7 +270,7 @@ static void chosen_mapping_takes_every_step() {
         c.n = 32;
         double best = 0;
         CHECK(jp_autotune(&c, 4, &best) == JP_OK);
-        CHECK(count("k_stream_collide_pair", from) > 0);
+        CHECK(count_of("k_stream_collide_pair", from) > 0);
         CHECK((c.vec == 0) == two_faster && (c.threads_per_block == 0) == two_faster);
         CHECK(best == 32.0 * 32 * 32 * 4 / ((two_faster ? 3.0 : 4.0) * 1e-3));
     }
@@ -321,6 +321,28 @@ static void in_place_conversions_keep_no_memory() {
     }
 }
 
+// With no device memory left, populations still convert: through the other array, or in place through the scratch
+// that the cube was created with.
+static void conversions_without_memory() {
+    for (const int flags : {0, (int)JP_FLAG_INPLACE}) {
+        jp_solver* s = cube(32, 0, 0, flags);
+        const int64_t count = 19LL * 32 * 32 * 32;
+        std::vector<double> p(count);
+        fake::fail_from = fake::allocations;
+        fake::fail_to = 1LL << 60;
+        for (const int layout : {(int)JP_LAYOUT_FLAT, (int)JP_LAYOUT_BLOCKED})
+            for (const int dtype : {(int)JP_F32, (int)JP_F64}) {
+                CHECK(jp_get_populations(s, 0, layout, dtype, p.data(), count) == JP_OK);
+                CHECK(jp_set_populations(s, 0, layout, dtype, p.data(), count) == JP_OK);
+            }
+        fake::fail_to = -1;
+        const size_t from = fake::ops.size();
+        CHECK(jp_get_populations(s, 0, JP_LAYOUT_FLAT, JP_F64, p.data(), count) == JP_OK);
+        CHECK(count_of("k_convert", from) == 2);
+        jp_destroy(s);
+    }
+}
+
 int main(int argc, char** argv) {
     const std::map<std::string, void (*)()> checks = {
         {"regrid_orders_list_counts", regrid_orders_list_counts},
@@ -330,6 +352,7 @@ int main(int argc, char** argv) {
         {"chosen_mapping_takes_every_step", chosen_mapping_takes_every_step},
         {"coefficients_search_both_neighbours", coefficients_search_both_neighbours},
         {"in_place_conversions_keep_no_memory", in_place_conversions_keep_no_memory},
+        {"conversions_without_memory", conversions_without_memory},
     };
     const auto it = argc == 2 ? checks.find(argv[1]) : checks.end();
     if (it == checks.end()) return 2;

@@ -40,6 +40,7 @@ def checks(tmp_path_factory):
     "chosen_mapping_takes_every_step",
     "coefficients_search_both_neighbours",
     "in_place_conversions_keep_no_memory",
+    "conversions_without_memory",
 ])
 def test_host_code(checks, name, tmp_path):
     r = subprocess.run([checks, name], capture_output=True, text=True, timeout=120, cwd=tmp_path)
