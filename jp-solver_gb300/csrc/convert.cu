@@ -113,10 +113,10 @@ jp_status convert_populations(jp_solver* s, int storage, int dtype, const PopMap
     const size_t unit = (size_t)m.len * (dtype == JP_F64 ? 8 : 4);
     const long long chunk = (long long)(scratch_bytes / unit);
     if (chunk < 1) return fail(JP_ERR_NOMEM, "population scratch of %zu bytes", scratch_bytes);
-    for (long long u = 0; u < m.units; u += chunk) {
+    cudaError_t e = cudaSuccess;
+    for (long long u = 0; u < m.units && e == cudaSuccess; u += chunk) {
         const long long k = std::min(chunk, m.units - u);
         char* const h = static_cast<char*>(host) + (size_t)u * unit;
-        cudaError_t e = cudaSuccess;
         if (to_host_order) {
             e = launch(storage, dtype, m, state, scratch, u, k, true, s->stream);
             if (e == cudaSuccess) e = cudaMemcpyAsync(h, scratch, (size_t)k * unit, cudaMemcpyDeviceToHost, s->stream);
@@ -124,9 +124,9 @@ jp_status convert_populations(jp_solver* s, int storage, int dtype, const PopMap
             e = cudaMemcpyAsync(scratch, h, (size_t)k * unit, cudaMemcpyHostToDevice, s->stream);
             if (e == cudaSuccess) e = launch(storage, dtype, m, state, scratch, u, k, false, s->stream);
         }
-        if (e != cudaSuccess) return cuda_fail(e, "population conversion");
     }
-    const cudaError_t e = cudaStreamSynchronize(s->stream);
+    const cudaError_t w = cudaStreamSynchronize(s->stream);  // also after a failure: the copies use the caller's memory
+    if (e == cudaSuccess) e = w;
     if (e != cudaSuccess) return cuda_fail(e, "population conversion");
     return JP_OK;
 }

@@ -343,6 +343,30 @@ static void conversions_without_memory() {
     }
 }
 
+// A conversion that fails half-way returns with none of its copies still reading or writing the caller's memory.
+static void failed_conversion_waits_for_its_copies() {
+    for (const int chunk : {1, 2, 3}) {
+        jp_solver* s = cube(32, 0, 0, JP_FLAG_INPLACE);
+        const int64_t count = 19LL * 32 * 32 * 32;
+        std::vector<double> p(count);
+        int launches = 0;
+        fake::fail_from = fake::allocations;  // many chunks
+        fake::fail_to = 1LL << 60;
+        fake::launch_error = [&](const std::string& k) {
+            if (k.find("k_convert") == std::string::npos || ++launches < chunk) return cudaSuccess;
+            return cudaErrorLaunchOutOfResources;
+        };
+        CHECK(jp_get_populations(s, 0, JP_LAYOUT_FLAT, JP_F64, p.data(), count) == JP_ERR_CUDA);
+        CHECK(fake::copies_in_flight() == 0);
+        launches = 0;
+        CHECK(jp_set_populations(s, 0, JP_LAYOUT_FLAT, JP_F64, p.data(), count) == JP_ERR_CUDA);
+        CHECK(fake::copies_in_flight() == 0);
+        fake::launch_error = nullptr;
+        fake::fail_to = -1;
+        jp_destroy(s);
+    }
+}
+
 int main(int argc, char** argv) {
     const std::map<std::string, void (*)()> checks = {
         {"regrid_orders_list_counts", regrid_orders_list_counts},
@@ -353,6 +377,7 @@ int main(int argc, char** argv) {
         {"coefficients_search_both_neighbours", coefficients_search_both_neighbours},
         {"in_place_conversions_keep_no_memory", in_place_conversions_keep_no_memory},
         {"conversions_without_memory", conversions_without_memory},
+        {"failed_conversion_waits_for_its_copies", failed_conversion_waits_for_its_copies},
     };
     const auto it = argc == 2 ? checks.find(argv[1]) : checks.end();
     if (it == checks.end()) return 2;
