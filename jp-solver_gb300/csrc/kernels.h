@@ -131,5 +131,6 @@ cudaError_t launch_qspeed(bool field_is_double, bool float_diff, const void* fie
 // Count of kernel launches issued by this library (for the bench's launch accounting).
 void note_launch(int k = 1);
 long long launch_count();
+long long thread_launch_count();  // of the calling thread
 
 }  // namespace jp

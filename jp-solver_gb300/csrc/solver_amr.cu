@@ -68,6 +68,7 @@ struct AmrState {
     // move (pool growth, new initial build) or the launch shape changes.
     cudaGraphExec_t graph[16] = {};
     int launched[16] = {};       // coarse steps taken by direct launches, per graph key
+    int kernels[16] = {};        // kernels of a captured step
     float *c0_home = nullptr, *f1_home = nullptr, *f2_home = nullptr;
     AmrFork fk;  // a coarse step's level-0 chain runs on fk.side, beside the first level-2 pair (base_step)
 };
@@ -1103,7 +1104,9 @@ static jp_status graph_step(jp_solver* s, cudaStream_t on = nullptr) {
     if (!a->graph[key]) {
         float *c0a = a->c0a, *c0b = a->c0b, *f1a = a->f1a, *f1b = a->f1b, *f2a = a->f2a, *f2b = a->f2b;
         ACK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal), "begin capture");
+        const long long counted = thread_launch_count();
         jp_status st = base_step(s);
+        a->kernels[key] = int(thread_launch_count() - counted);
         cudaGraph_t g = nullptr;
         cudaError_t e = cudaStreamEndCapture(s->stream, &g);
         // the capture only recorded the step; the replay below performs it
@@ -1313,7 +1316,9 @@ jp_status amr_step(jp_solver* s, int64_t nsteps) {
         const int key = graph_key(a);
         bool replay = graph || a->launched[key] >= kCaptureAfter;
         if (replay) {
+            const bool captured = a->graph[key] != nullptr;  // before: the capture counts the first replay's kernels
             const jp_status st = graph_step(s);
+            if (st == JP_OK && captured && !graph) note_launch(a->kernels[key]);
             if (st != JP_OK && (graph || a->graph[key])) return st;
             if (st != JP_OK) {
                 cudaGetLastError();

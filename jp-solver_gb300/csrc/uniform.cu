@@ -20,7 +20,12 @@
 namespace jp {
 
 static std::atomic<long long> g_launches{0};
-void note_launch(int k) { g_launches.fetch_add(k, std::memory_order_relaxed); }
+static thread_local long long t_launches = 0;
+void note_launch(int k) {
+    g_launches.fetch_add(k, std::memory_order_relaxed);
+    t_launches += k;
+}
+long long thread_launch_count() { return t_launches; }
 long long launch_count() { return g_launches.load(std::memory_order_relaxed); }
 
 template <class ST, int V, int TPB, int MAXB>

@@ -367,6 +367,27 @@ static void failed_conversion_waits_for_its_copies() {
     }
 }
 
+// Coarse steps without JP_FLAG_GRAPH count their kernels alike, launched directly or replayed.
+static void replayed_steps_count_their_kernels() {
+    supply_grid();
+    for (const int nref1 : {10, 0}) {
+        set_grid(16, nref1);
+        jp_solver* s = amr(64.0);
+        int64_t each = 0;
+        for (int k = 0; k < 16; ++k) {
+            const int64_t c0 = jp_launch_count();
+            CHECK(jp_step(s, 1) == JP_OK);
+            const int64_t n = jp_launch_count() - c0;
+            if (k == 0) each = n;
+            CHECK(n == each && n > 0);
+        }
+        size_t replays = 0;
+        for (const fake::Op& o : fake::ops) replays += o.kind == fake::Op::GRAPH_LAUNCH;
+        CHECK(replays > 0);
+        jp_destroy(s);
+    }
+}
+
 int main(int argc, char** argv) {
     const std::map<std::string, void (*)()> checks = {
         {"regrid_orders_list_counts", regrid_orders_list_counts},
@@ -378,6 +399,7 @@ int main(int argc, char** argv) {
         {"in_place_conversions_keep_no_memory", in_place_conversions_keep_no_memory},
         {"conversions_without_memory", conversions_without_memory},
         {"failed_conversion_waits_for_its_copies", failed_conversion_waits_for_its_copies},
+        {"replayed_steps_count_their_kernels", replayed_steps_count_their_kernels},
     };
     const auto it = argc == 2 ? checks.find(argv[1]) : checks.end();
     if (it == checks.end()) return 2;
