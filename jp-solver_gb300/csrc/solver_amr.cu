@@ -1123,7 +1123,8 @@ static jp_status graph_step(jp_solver* s, cudaStream_t on = nullptr) {
         if (e != cudaSuccess) return cuda_fail(e, "end capture");
         e = cudaGraphInstantiate(&a->graph[key], g, 0);
         cudaGraphDestroy(g);
-        if (e == cudaSuccess) e = cudaGraphUpload(a->graph[key], s->stream);  // its memory now, not at the first launch
+        // its memory now, not at the first launch; on the stream that replays it, behind which alone that launch is ordered
+        if (e == cudaSuccess) e = cudaGraphUpload(a->graph[key], on ? on : s->stream);
         if (e != cudaSuccess) {
             if (a->graph[key]) cudaGraphExecDestroy(a->graph[key]);
             a->graph[key] = nullptr;

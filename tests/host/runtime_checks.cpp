@@ -11,6 +11,7 @@
 #include "amr_kernels.h"
 #include "jp.h"
 #include "kernels.h"
+#include "solver.h"
 
 using jp::amr::AdaptCounts;
 
@@ -388,6 +389,28 @@ static void replayed_steps_count_their_kernels() {
     }
 }
 
+// A captured step replayed on another stream than the solver's: its upload is ordered before it.
+static void upload_precedes_replay_on_its_stream() {
+    supply_grid();
+    set_grid(16, 10);
+    jp_solver* s = amr(64.0, JP_FLAG_GRAPH);
+    cudaStream_t lane;
+    CHECK(cudaStreamCreateWithFlags(&lane, cudaStreamNonBlocking) == cudaSuccess);
+    const size_t from = fake::ops.size();
+    for (int k = 0; k < 4; ++k) CHECK(jp::amr_graph_step_on(s, lane) == JP_OK);
+    const fake::Op* upload = nullptr;
+    int replays = 0;
+    for (size_t i = from; i < fake::ops.size(); ++i) {
+        const fake::Op& o = fake::ops[i];
+        if (o.kind == fake::Op::GRAPH_UPLOAD) upload = &o;
+        if (o.kind != fake::Op::GRAPH_LAUNCH) continue;
+        ++replays;
+        CHECK(o.stream == lane && upload && fake::before(*upload, o));
+    }
+    CHECK(replays == 4);
+    jp_destroy(s);
+}
+
 int main(int argc, char** argv) {
     const std::map<std::string, void (*)()> checks = {
         {"regrid_orders_list_counts", regrid_orders_list_counts},
@@ -400,6 +423,7 @@ int main(int argc, char** argv) {
         {"conversions_without_memory", conversions_without_memory},
         {"failed_conversion_waits_for_its_copies", failed_conversion_waits_for_its_copies},
         {"replayed_steps_count_their_kernels", replayed_steps_count_their_kernels},
+        {"upload_precedes_replay_on_its_stream", upload_precedes_replay_on_its_stream},
     };
     const auto it = argc == 2 ? checks.find(argv[1]) : checks.end();
     if (it == checks.end()) return 2;
