@@ -146,6 +146,7 @@ template <> struct Lanes<float> {
     using real = float;
     static __device__ __forceinline__ float bc(float s) { return s; }
     static __device__ __forceinline__ float add(float a, float b) { return __fadd_rn(a, b); }
+    static __device__ __forceinline__ float neg(float a) { return -a; }
     static __device__ __forceinline__ float sub(float a, float b) { return __fadd_rn(a, -b); }
     static __device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
     static __device__ __forceinline__ float fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
@@ -155,6 +156,7 @@ template <> struct Lanes<double> {
     using real = double;
     static __device__ __forceinline__ double bc(double s) { return s; }
     static __device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, b); }
+    static __device__ __forceinline__ double neg(double a) { return -a; }
     static __device__ __forceinline__ double sub(double a, double b) { return __dadd_rn(a, -b); }
     static __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
     static __device__ __forceinline__ double fma(double a, double b, double c) { return __fma_rn(a, b, c); }
@@ -164,7 +166,7 @@ template <> struct Lanes<float2> {
     using real = float;
     static __device__ __forceinline__ float2 bc(float s) { return make_float2(s, s); }
     static __device__ __forceinline__ float2 add(float2 a, float2 b) { return __fadd2_rn(a, b); }
-    // a - b as a + (-b): an add is never merged with the product before it (an FMA by -1 can be)
+    static __device__ __forceinline__ float2 neg(float2 a) { return make_float2(-a.x, -a.y); }
     static __device__ __forceinline__ float2 sub(float2 a, float2 b) { return __fadd2_rn(a, make_float2(-b.x, -b.y)); }
     static __device__ __forceinline__ float2 mul(float2 a, float2 b) { return __fmul2_rn(a, b); }
     static __device__ __forceinline__ float2 fma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }

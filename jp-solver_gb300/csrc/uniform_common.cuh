@@ -130,9 +130,11 @@ constexpr int min_blocks() {
 // __fmul2_rn, __ffma2_rn, each lane rounded to nearest like its scalar op).  The FP32 steps hold V = 2,
 // 4 or 8 cells per thread, so the relaxation runs on pairs of cells and issues half the FP32
 // instructions; an odd V runs the same sequence on single floats.  FP64 runs it on single doubles.  Every
-// operation is spelled out (no contraction left to the compiler), so a cell's result does not depend on
-// V, and the pull, two-step and in-place steps, which share this code, produce the same bits.  The
-// sequence per cell, 117 operations and a reciprocal (the FP64 step is bound by its FP64 rate):
+// operation is spelled out, so a cell's result does not depend on V, and the pull, two-step and in-place steps, which
+// share this code, produce the same bits.  (The packed intrinsics keep each rounding, but the compiler may
+// still merge a packed product into the sum that alone uses it; where it does, LaneBgk::pair says FMA.)  The
+// sequence per cell, 117 operations and a reciprocal (the FP64 step is bound by its FP64 rate; FP32 merges one
+// product):
 //   S_q = g_q + g_opp, D_q = g_q - g_opp; s = g0 + the S, j = the signed sums of the D, in sum_order
 //   rho = 1 + s (s itself in FP64), inv = 1 / rho (IEEE), e = s - 1.5 inv (jx jx + jy jy + jz jz) (two FMAs)
 //   out0 = (1-om) g0 + om w0 e
@@ -201,10 +203,16 @@ struct LaneBgk {
             ay = L::mul(L::bc(w), jy);
             az = L::mul(L::bc(w), jz);
         }
-        // om times the antisymmetric part: 3 om w c.j (c's first non-zero component is positive for odd q)
+        // om times the antisymmetric part: 3 om w c.j (c's first non-zero component is positive for odd q).  FP32: the
+        // product by jx and the sum in one FMA for the edges along x, which the compiler makes of a packed
+        // product and sum that have no other use for the product; written out, single floats take it too.
         T a = cx(q) != 0 ? ax : (cy(q) != 0 ? ay : az);
-        if (cx(q) != 0 && cy(q) != 0) a = cy(q) > 0 ? L::add(a, ay) : L::sub(a, ay);
-        if ((cx(q) != 0 || cy(q) != 0) && cz(q) != 0) a = cz(q) > 0 ? L::add(a, az) : L::sub(a, az);
+        if ((cx(q) != 0) + (cy(q) != 0) + (cz(q) != 0) == 2) {
+            const bool plus = cz(q) != 0 ? cz(q) > 0 : cy(q) > 0;
+            const T other = cz(q) != 0 ? az : ay;
+            if (sizeof(R) == 4 && cx(q) != 0) a = L::fma(L::bc(co.a2), jx, plus ? other : L::neg(other));
+            else a = plus ? L::add(a, other) : L::sub(a, other);
+        }
         const T t = L::fma(L::mul(k, a), a, b);  // om times the symmetric part
         const T h = L::bc(R(0.5) * (R(1) - om));
         const T u = L::fma(h, S, t), v = L::fma(h, D, a);
