@@ -87,7 +87,7 @@ typedef struct jp_config {
 /* jp_config.flags */
 #define JP_FLAG_SKIP_PREP 1      /* AMR profiling: skip prep + ghost fill (breaks physics; --skipprep, src/tgv3d_amr.cu:654) */
 #define JP_FLAG_SKIP_RESTRICT 2  /* AMR profiling: skip restriction (breaks physics; --skiprestr, :655) */
-#define JP_FLAG_GRAPH 4          /* replay the step from captured CUDA graphs (--graph, :656) from the first step on;
+#define JP_FLAG_GRAPH 4          /* replay the step from recorded CUDA graphs (--graph, :656) from the first step on;
                                     without it an AMR solver does so once a step has been launched four times */
 #define JP_FLAG_DEFER_INIT 8     /* jp_create allocates only: set a sensor override (or populations) and
                                     call jp_init_tgv before the first step, so that even the first

@@ -2,6 +2,8 @@
 // shape rules of the AMR kernels.  The kernels themselves are in amr_kernels.cuh.
 #include "amr_kernels.cuh"
 
+#include <algorithm>
+
 namespace jp {
 namespace amr {
 
@@ -31,6 +33,25 @@ cudaError_t amr_batch_launch(int storage, int mb, int op, int tpb, bool fuse, co
         case 2: return amr_batch_launch_st<StBF16>(mb, op, tpb, fuse, B, st);
     }
     return cudaErrorInvalidValue;
+}
+
+void StepGraph::kernel(const void* f, dim3 grid, dim3 cta, size_t smem, void** args, cudaStream_t st) {
+    if (err != cudaSuccess) return;
+    cudaKernelNodeParams p = {};
+    p.func = const_cast<void*>(f);
+    p.gridDim = grid;
+    p.blockDim = cta;
+    p.sharedMemBytes = (unsigned)smem;
+    p.kernelParams = args;
+    std::vector<cudaGraphNode_t>& after = tail[st];
+    cudaGraphNode_t node = nullptr;
+    err = cudaGraphAddKernelNode(&node, graph, after.data(), after.size(), &p);
+    after.assign(1, node);
+}
+void StepGraph::wait(cudaStream_t st, cudaEvent_t e) {
+    std::vector<cudaGraphNode_t>& after = tail[st];
+    for (cudaGraphNode_t n : mark[e])
+        if (std::find(after.begin(), after.end(), n) == after.end()) after.push_back(n);
 }
 
 int shell_cells(int mb) { return 6 * mb * mb + 12 * mb; }

@@ -9,6 +9,8 @@
 // a d_* device function that takes the block index, shared by the single-solve kernel (k_*) and the
 // batched kernels over many solves (kb_*).
 #pragma once
+#include <tuple>
+
 #include "amr_common.cuh"
 #include "amr_kernels.h"
 #include "kernels.h"
@@ -889,24 +891,38 @@ __global__ void __launch_bounds__(256) k_composite(const typename ST::raw* __res
 #define POOL(p) reinterpret_cast<typename ST::raw*>(p)
 #define CPOOL(p) reinterpret_cast<const typename ST::raw*>(p)
 
+// a kernel of the coarse step: launched, or added to the graph that records the step
+template <class... P, class... A>
+static void run(const AmrLaunch& L, void (*kern)(P...), dim3 grid, dim3 cta, size_t smem, A... a) {
+    if (!L.rec) {
+        kern<<<grid, cta, smem, L.st>>>(static_cast<P>(a)...);
+        return;
+    }
+    std::tuple<P...> p(static_cast<P>(a)...);
+    std::apply([&](auto&... v) {
+        void* args[] = {const_cast<void*>(static_cast<const void*>(&v))...};
+        L.rec->kernel(reinterpret_cast<const void*>(kern), grid, cta, smem, args, L.st);
+    }, p);
+}
+
 // the steps with TPB threads per CTA (the block's MB^3 cells split evenly)
 template <int MB, class ST, int TPB>
 static void launch_steps(const AmrLaunch& L, int op) {
     using G = Geo<MB>;
     if (op == OP_STEP_L0) {
-        k_step_l0<MB, ST, TPB><<<L.nblocks, TPB, 0, L.st>>>(CPOOL(L.in), POOL(L.out), L.cgx, L.omega);
+        run(L, k_step_l0<MB, ST, TPB>, L.nblocks, TPB, 0, CPOOL(L.in), POOL(L.out), L.cgx, L.omega);
         return;
     }
     const int* parent = L.t0;  // pcb (level 1) or l2pl1 (level 2)
     if constexpr (MB <= 8) {
         if (L.out2) {
-            k_step_fine<MB, ST, TPB, true><<<L.nblocks, TPB, sizeof(float) * Q * G::MB3, L.st>>>(
+            run(L, k_step_fine<MB, ST, TPB, true>, L.nblocks, TPB, sizeof(float) * Q * G::MB3,
                 CPOOL(L.in), POOL(L.out), CPOOL(L.aux), L.nbt, parent, L.t1, L.omega, POOL(L.out2), L.scale, L.nlim);
             return;
         }
     }
-    k_step_fine<MB, ST, TPB, false><<<L.nblocks, TPB, 0, L.st>>>(CPOOL(L.in), POOL(L.out), CPOOL(L.aux), L.nbt,
-                                                                 parent, L.t1, L.omega, nullptr, 0.f, L.nlim);
+    run(L, k_step_fine<MB, ST, TPB, false>, L.nblocks, TPB, 0, CPOOL(L.in), POOL(L.out), CPOOL(L.aux), L.nbt, parent,
+        L.t1, L.omega, nullptr, 0.f, L.nlim);
 }
 
 // the fine steps on rows of four cells (MB = 8, 16)
@@ -921,16 +937,16 @@ static void launch_rows(const AmrLaunch& L) {
     if (L.out2) {
         const int cap = rows_grid_cap<MB, ST, true>();
         if (sizeof(typename ST::raw) == 4 && L.nblocks > 16 * cap)
-            k_step_fine_rows<MB, ST, true, false><<<L.nblocks, T, sm, L.st>>>(
+            run(L, k_step_fine_rows<MB, ST, true, false>, L.nblocks, T, sm,
                 CPOOL(L.in), POOL(L.out), CPOOL(L.aux), L.nbt, L.t0, L.t1, L.omega, POOL(L.out2), L.scale, L.nlim);
         else
-            k_step_fine_rows<MB, ST, true, true><<<std::min(L.nblocks, cap), T, sm, L.st>>>(
+            run(L, k_step_fine_rows<MB, ST, true, true>, std::min(L.nblocks, cap), T, sm,
                 CPOOL(L.in), POOL(L.out), CPOOL(L.aux), L.nbt, L.t0, L.t1, L.omega, POOL(L.out2), L.scale, L.nlim);
     } else if (L.list) {  // the listed blocks only (L.nblocks: the list's capacity)
-        k_step_fine_rows_listed<MB, ST><<<std::min(L.nblocks, rows_listed_grid_cap<MB, ST>()), T, 0, L.st>>>(
+        run(L, k_step_fine_rows_listed<MB, ST>, std::min(L.nblocks, rows_listed_grid_cap<MB, ST>()), T, 0,
             CPOOL(L.in), POOL(L.out), CPOOL(L.aux), L.nbt, L.omega, L.nlim, L.list);
     } else {
-        k_step_fine_rows<MB, ST, false, true><<<std::min(L.nblocks, rows_grid_cap<MB, ST, false>()), T, 0, L.st>>>(
+        run(L, k_step_fine_rows<MB, ST, false, true>, std::min(L.nblocks, rows_grid_cap<MB, ST, false>()), T, 0,
             CPOOL(L.in), POOL(L.out), CPOOL(L.aux), L.nbt, L.t0, L.t1, L.omega, nullptr, 0.f, L.nlim);
     }
 }
@@ -976,19 +992,19 @@ static cudaError_t dispatch(const AmrLaunch& L, int op) {
                 L.iout, L.t0, L.t1, L.t2, L.t3, L.t4, L.t5, L.l1gx, L.nblocks);
             break;
         case OP_PREP:
-            k_prep<MB, ST><<<std::max(1, std::min((L.nblocks + 255) / 256, prep_grid_cap<MB, ST>())), 256, 0, L.st>>>(
+            run(L, k_prep<MB, ST>, std::max(1, std::min((L.nblocks + 255) / 256, prep_grid_cap<MB, ST>())), 256, 0,
                 CPOOL(L.in), POOL(L.out), L.list, L.scale, L.nlim, L.t0);
             break;
         case OP_FILL_L1:
-            k_fill_l1<MB, ST><<<std::max(1, std::min((L.nblocks + 255) / 256, fill_grid_cap<MB, ST, 1>())), 256, 0,
-                                L.st>>>(CPOOL(L.in), POOL(L.out), L.t0, L.t1, L.cgx, L.n, L.list, L.nlim);
+            run(L, k_fill_l1<MB, ST>, std::max(1, std::min((L.nblocks + 255) / 256, fill_grid_cap<MB, ST, 1>())), 256, 0,
+                CPOOL(L.in), POOL(L.out), L.t0, L.t1, L.cgx, L.n, L.list, L.nlim);
             break;
         case OP_FILL_L2:
-            k_fill_l2<MB, ST><<<std::max(1, std::min((L.nblocks + 255) / 256, fill_grid_cap<MB, ST, 2>())), 256, 0,
-                                L.st>>>(CPOOL(L.in), POOL(L.out), L.t0, L.t1, L.t2, L.t3, L.l1gx, L.n1, L.list, L.nlim);
+            run(L, k_fill_l2<MB, ST>, std::max(1, std::min((L.nblocks + 255) / 256, fill_grid_cap<MB, ST, 2>())), 256, 0,
+                CPOOL(L.in), POOL(L.out), L.t0, L.t1, L.t2, L.t3, L.l1gx, L.n1, L.list, L.nlim);
             break;
         case OP_RESTRICT:
-            k_restrict<MB, ST><<<L.nblocks, cta, 0, L.st>>>(POOL(L.out), CPOOL(L.in), L.list, L.t0, L.scale, L.nlim);
+            run(L, k_restrict<MB, ST>, L.nblocks, cta, 0, POOL(L.out), CPOOL(L.in), L.list, L.t0, L.scale, L.nlim);
             break;
         case OP_SEED_L1:
             k_seed_l1<MB, ST><<<L.nblocks, cta, 0, L.st>>>(CPOOL(L.in), POOL(L.out), CPOOL(L.aux), L.t0, L.t1, L.t2,
@@ -1009,7 +1025,7 @@ static cudaError_t dispatch(const AmrLaunch& L, int op) {
                 reinterpret_cast<float*>(L.out));
             break;
         }
-        case OP_WARM:  // launch shapes of the rows steps, preps and fills, found before any graph capture
+        case OP_WARM:  // launch shapes of the rows steps, preps and fills, found before a step is recorded
             prep_grid_cap<MB, ST>();
             fill_grid_cap<MB, ST, 1>();
             fill_grid_cap<MB, ST, 2>();
@@ -1023,7 +1039,7 @@ static cudaError_t dispatch(const AmrLaunch& L, int op) {
             return cudaErrorInvalidValue;
     }
     note_launch();
-    return cudaGetLastError();
+    return L.rec ? L.rec->err : cudaGetLastError();
 }
 
 // ---- batched launches: one grid over the blocks of many solves ------------------------------------

@@ -2,6 +2,9 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <map>
+#include <vector>
+
 namespace jp {
 namespace amr {
 
@@ -28,13 +31,27 @@ enum AmrOp {
     OP_NBTAB_L1,       // iout = level-1 neighbour table (nblocks = nf1); t0 pcb, t1 oct, t2 ref0, t3 fof0
     OP_NBTAB_L2,       // iout = level-2 neighbour table (nblocks = nf2); t0 l2pl1, t1 l2oct, t2 f1pos,
                        // t3 l1grid, t4 ref1, t5 fof1
-    OP_WARM            // no launch: find the resident grid of the row steps (before any graph capture)
+    OP_WARM            // no launch: find the resident grid of the row steps (before a step is recorded)
+};
+
+// A coarse step recorded as a graph: its kernels as nodes, ordered as the streams and events of base_step order the
+// launches.  Built by hand, not by capturing streams: while any stream is captured, a call of any other thread
+// that waits for the device (cudaDeviceSynchronize) fails, and breaks the capture.
+struct StepGraph {
+    cudaGraph_t graph = nullptr;
+    cudaError_t err = cudaSuccess;  // of the first node that failed
+    std::map<cudaStream_t, std::vector<cudaGraphNode_t>> tail;  // what the stream's next kernel follows
+    std::map<cudaEvent_t, std::vector<cudaGraphNode_t>> mark;   // the same at an event's record
+    void kernel(const void* f, dim3 grid, dim3 cta, size_t smem, void** args, cudaStream_t st);
+    void record(cudaEvent_t e, cudaStream_t st) { mark[e] = tail[st]; }
+    void wait(cudaStream_t st, cudaEvent_t e);
 };
 
 // Population arrays (pools, prolongation sources, ghost shells) are in the solver's storage format
 // (FP32, or shifted FP16/BF16); sensor values and the composite field are float.
 struct AmrLaunch {
     cudaStream_t st = nullptr;
+    StepGraph* rec = nullptr;  // the step kernels (OP_STEP_L0 to OP_RESTRICT): a node of this graph instead of a launch
     int nblocks = 0;
     const void* in = nullptr;
     void* out = nullptr;
@@ -49,7 +66,7 @@ struct AmrLaunch {
     int vec = 0;               // fine steps: 4 = rows of four cells per thread, 1 = a cell per thread
                                // (0: default_step_vec)
     // device count of the blocks to process (prep, fill, fine step, restrict): the grid is sized
-    // for the capacity and CTAs past *nlim return, so a captured step stays valid after a regrid
+    // for the capacity and CTAs past *nlim return, so a recorded step stays valid after a regrid
     const int* nlim = nullptr;
     int cgx = 0, n = 0, l1gx = 0, n1 = 0, n2 = 0;
     float omega = 0.f, scale = 0.f;

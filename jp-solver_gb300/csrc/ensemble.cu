@@ -728,7 +728,7 @@ bool lane_round(jp_server* sv, jp_server::Lane& L) {
                 std::vector<jp_solver*> ms;
                 for (size_t i = 0; i < g.size(); ++i)
                     if (ks[i] > t) ms.push_back(g[i]->s);
-                // a group of one with graph replay replays its captured step instead (one launch)
+                // a group of one with graph replay replays its recorded step instead (one launch)
                 const bool alone = ms.size() == 1 && (ms[0]->cfg.flags & JP_FLAG_GRAPH);
                 st = alone ? amr_graph_step_on(ms[0], L.stream) : amr_batch_step(ms, L.stream, &L.fk);
                 moved += (long long)ms.size();

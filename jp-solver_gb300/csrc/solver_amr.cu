@@ -58,17 +58,18 @@ struct AmrState {
     size_t macro_blocks = 0;  // blocks macro holds (ensure_macro)
     std::vector<void*> owned;
     // Block counts the step kernels read on the device ({nf1, nf2, n_skin0, n_skin1, nref0, nref1}):
-    // the step launches grids sized for the pool capacities, so one captured step serves every grid
+    // the step launches grids sized for the pool capacities, so one recorded step serves every grid
     // a regrid builds within them.
     int* step_cnt = nullptr;
     int* step_cnt_host = nullptr;  // pinned staging of the upload
-    // captured base_step graphs, one per combination of the ping-pong parities of the three levels
+    // recorded base_step graphs, one per combination of the ping-pong parities of the three levels
     // (a coarse step swaps level 0 once and the fine levels an even number of times; a regrid's
     // seeding swaps a fine level once) and of whether there is a level 2.  Dropped only when buffers
     // move (pool growth, new initial build) or the launch shape changes.
     cudaGraphExec_t graph[16] = {};
     int launched[16] = {};       // coarse steps taken by direct launches, per graph key
-    int kernels[16] = {};        // kernels of a captured step
+    int kernels[16] = {};        // kernels of a recorded step
+    StepGraph* rec = nullptr;    // while base_step records: its launches and events go to this graph
     float *c0_home = nullptr, *f1_home = nullptr, *f2_home = nullptr;
     AmrFork fk;  // a coarse step's level-0 chain runs on fk.side, beside the first level-2 pair (base_step)
 };
@@ -79,7 +80,7 @@ enum { SC_NF1 = 0, SC_NF2, SC_SKIN0, SC_SKIN1, SC_NREF0, SC_NREF1, SC_COUNT, SC_
 // CTAs per member of a batched prep or fill (its threads walk the member's cell list)
 constexpr int kBatchPrepCtas = 64;
 
-// drop the captured steps and take the current buffers as the parity reference
+// drop the recorded steps and take the current buffers as the parity reference
 static void reset_graphs(AmrState* a) {
     for (auto& g : a->graph)
         if (g) {
@@ -128,6 +129,7 @@ static size_t pf(const AmrState* a, size_t n) { return (n * a->elem + 3) / 4; }
 
 static jp_status launch(jp_solver* s, int op, AmrLaunch L, cudaStream_t st = nullptr) {
     L.st = st ? st : s->stream;
+    L.rec = s->amr->rec;
     cudaError_t e = amr_launch(s->amr->storage, s->amr->MB, op, L);
     if (e != cudaSuccess) return cuda_fail(e, "AMR kernel launch");
     return JP_OK;
@@ -530,18 +532,31 @@ static jp_status initial_build(jp_solver* s) {
     return skins_readback(s);
 }
 
-// Takes a side branch back into a stream (or a capture) on every return, errors included.
+// events between the streams of a step, or of the graph that records it
+static cudaError_t record_event(StepGraph* rec, cudaEvent_t ev, cudaStream_t st) {
+    if (!rec) return cudaEventRecord(ev, st);
+    rec->record(ev, st);
+    return cudaSuccess;
+}
+static cudaError_t wait_for_event(StepGraph* rec, cudaStream_t st, cudaEvent_t ev) {
+    if (!rec) return cudaStreamWaitEvent(st, ev, 0);
+    rec->wait(st, ev);
+    return cudaSuccess;
+}
+
+// Takes a side branch back into a stream (or a graph) on every return, errors included.
 struct JoinOnExit {
     cudaStream_t st;
     cudaEvent_t ev;
     bool pending = true;
+    StepGraph* rec = nullptr;
     jp_status now() {
         pending = false;
-        ACK(cudaStreamWaitEvent(st, ev, 0), "join");
+        ACK(wait_for_event(rec, st, ev), "join");
         return JP_OK;
     }
     ~JoinOnExit() {
-        if (pending) cudaStreamWaitEvent(st, ev, 0);
+        if (pending) wait_for_event(rec, st, ev);
     }
 };
 
@@ -699,7 +714,7 @@ static jp_status level0_chain(jp_solver* s, cudaStream_t st) {
 // level-2 pair (level-1 sources, level-2 fill, two level-2 substeps restricting into level 1) share
 // no array: 2:1 balance keeps level 2 away from level 0, so level-2 ghosts come from level 1 alone.
 // They meet at the first level-1 substep, which reads the level-1 ghosts and the restricted level 1.
-// The level-0 chain therefore runs on a side stream (a branch of the captured graph), and the short
+// The level-0 chain therefore runs on a side stream (a branch of the recorded graph), and the short
 // latency-bound fills and preps of one chain overlap the bandwidth-bound steps of the other.  Every
 // kernel sees the same inputs as in one stream: results are unchanged.
 static jp_status base_step(jp_solver* s) {
@@ -713,19 +728,19 @@ static jp_status base_step(jp_solver* s) {
     // graph 26.7 / 23.5 us, N0=48 FP16 direct launches 81.7 / 66 us.
     const bool l2 = a->nf2 > 0;
     if (l2) {
-        ACK(cudaEventRecord(a->fk.fork, s->stream), "fork");
-        ACK(cudaStreamWaitEvent(a->fk.side, a->fk.fork, 0), "fork");
+        ACK(record_event(a->rec, a->fk.fork, s->stream), "fork");
+        ACK(wait_for_event(a->rec, a->fk.side, a->fk.fork), "fork");
     }
     const jp_status st0 = level0_chain(s, l2 ? a->fk.side : s->stream);
-    if (l2) ACK(cudaEventRecord(a->fk.join, a->fk.side), "join");
-    JoinOnExit join{s->stream, a->fk.join, l2};
+    if (l2) ACK(record_event(a->rec, a->fk.join, a->fk.side), "join");
+    JoinOnExit join{s->stream, a->fk.join, l2, a->rec};
     TRY(st0);
     // The first level-1 substep in two parts: its skin blocks (the only ones the next level-2 pair
     // reads, through the prep cells, and the only ones that pair restricts into), then the others on
     // the side branch, beside the whole second level-2 pair; they join before the last level-1
     // substep.  Each block is stepped as in one launch (rows mapping).
     const bool split = l2 && a->MB >= 8 && (a->vec ? a->vec : default_step_vec(a->MB)) == 4;
-    JoinOnExit join2{s->stream, a->fk.join2, false};
+    JoinOnExit join2{s->stream, a->fk.join2, false, a->rec};
     for (int s1 = 0; s1 < 2; ++s1) {
         if (l2 && !skip_prep) {
             AmrLaunch L;
@@ -805,13 +820,13 @@ static jp_status base_step(jp_solver* s) {
             K.list = a->skin1;
             K.nlim = cnt + SC_SKIN1;
             TRY(launch(s, OP_STEP_L1, K));
-            ACK(cudaEventRecord(a->fk.fork2, s->stream), "fork");
-            ACK(cudaStreamWaitEvent(a->fk.side, a->fk.fork2, 0), "fork");
+            ACK(record_event(a->rec, a->fk.fork2, s->stream), "fork");
+            ACK(wait_for_event(a->rec, a->fk.side, a->fk.fork2), "fork");
             AmrLaunch R = S;  // the others, on the side branch
             R.list = a->rest1;
             R.nlim = cnt + SC_REST1;
             const jp_status sr = launch(s, OP_STEP_L1, R, a->fk.side);
-            ACK(cudaEventRecord(a->fk.join2, a->fk.side), "join");
+            ACK(record_event(a->rec, a->fk.join2, a->fk.side), "join");
             join2.pending = true;
             TRY(sr);
         } else {
@@ -1093,7 +1108,7 @@ bool amr_batch_compatible(const jp_solver* a, const jp_solver* b) {
            a->amr->vec == b->amr->vec && (a->cfg.flags & skip) == (b->cfg.flags & skip);
 }
 
-// base_step replayed from a captured graph (captured on first use for each parity combination)
+// base_step replayed from a graph (recorded on first use for each parity combination)
 static int graph_key(const AmrState* a) {
     return (a->c0a == a->c0_home ? 0 : 1) | (a->f1a == a->f1_home ? 0 : 2) | (a->f2a == a->f2_home ? 0 : 4) |
            (a->nf2 > 0 ? 0 : 8);
@@ -1103,26 +1118,24 @@ static jp_status graph_step(jp_solver* s, cudaStream_t on = nullptr) {
     const int key = graph_key(a);
     if (!a->graph[key]) {
         float *c0a = a->c0a, *c0b = a->c0b, *f1a = a->f1a, *f1b = a->f1b, *f2a = a->f2a, *f2b = a->f2b;
-        ACK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal), "begin capture");
+        StepGraph rec;
+        ACK(cudaGraphCreate(&rec.graph, 0), "graph create");
         const long long counted = thread_launch_count();
+        a->rec = &rec;
         jp_status st = base_step(s);
+        a->rec = nullptr;
         a->kernels[key] = int(thread_launch_count() - counted);
-        cudaGraph_t g = nullptr;
-        cudaError_t e = cudaStreamEndCapture(s->stream, &g);
-        // the capture only recorded the step; the replay below performs it
+        // the step was only recorded; the replay below performs it
         a->c0a = c0a;
         a->c0b = c0b;
         a->f1a = f1a;
         a->f1b = f1b;
         a->f2a = f2a;
         a->f2b = f2b;
-        if (st != JP_OK) {
-            if (g) cudaGraphDestroy(g);
-            return st;
-        }
-        if (e != cudaSuccess) return cuda_fail(e, "end capture");
-        e = cudaGraphInstantiate(&a->graph[key], g, 0);
-        cudaGraphDestroy(g);
+        cudaError_t e = cudaSuccess;
+        if (st == JP_OK) e = cudaGraphInstantiate(&a->graph[key], rec.graph, 0);
+        cudaGraphDestroy(rec.graph);
+        if (st != JP_OK) return st;
         // its memory now, not at the first launch; on the stream that replays it, behind which alone that launch is ordered
         if (e == cudaSuccess) e = cudaGraphUpload(a->graph[key], on ? on : s->stream);
         if (e != cudaSuccess) {
@@ -1136,8 +1149,8 @@ static jp_status graph_step(jp_solver* s, cudaStream_t on = nullptr) {
     return JP_OK;
 }
 
-// One coarse step replayed from the solver's captured graph on another stream `st` (ordered there
-// like a batched step; the capture itself runs on the solver's idle stream).
+// One coarse step replayed from the solver's recorded graph on another stream `st` (ordered there
+// like a batched step).
 jp_status amr_graph_step_on(jp_solver* s, cudaStream_t st) {
     TRY(graph_step(s, st));
     ++s->step_count;
@@ -1305,21 +1318,21 @@ jp_status amr_init(jp_solver* s) {
     return st;
 }
 
-// Without JP_FLAG_GRAPH a coarse step is captured once its case (graph_key) has been launched kCaptureAfter times:
-// a run replays (per coarse step, launches / graph: N0=24 71 / 51 us, N0=48 FP16 76 / 59, N0=96 304 / 293; a capture costs
-// 50 to 70 us, paid back by four steps), a handful of steps does not pay for captures.  Where there is no memory
+// Without JP_FLAG_GRAPH a coarse step is recorded once its case (graph_key) has been launched kRecordAfter times:
+// a run replays (per coarse step, launches / graph: N0=24 71 / 51 us, N0=48 FP16 76 / 59, N0=96 304 / 293; a recording costs
+// 50 to 70 us, paid back by four steps), a handful of steps does not pay for recordings.  Where there is no memory
 // left for a graph the case stays with launches.
-constexpr int kCaptureAfter = 4;
+constexpr int kRecordAfter = 4;
 jp_status amr_step(jp_solver* s, int64_t nsteps) {
     const bool graph = s->cfg.flags & JP_FLAG_GRAPH;
     for (int64_t i = 0; i < nsteps; ++i) {
         AmrState* a = s->amr;
         const int key = graph_key(a);
-        bool replay = graph || a->launched[key] >= kCaptureAfter;
+        bool replay = graph || a->launched[key] >= kRecordAfter;
         if (replay) {
-            const bool captured = a->graph[key] != nullptr;  // before: the capture counts the first replay's kernels
+            const bool recorded = a->graph[key] != nullptr;  // before: the recording counts the first replay's kernels
             const jp_status st = graph_step(s);
-            if (st == JP_OK && captured && !graph) note_launch(a->kernels[key]);
+            if (st == JP_OK && recorded && !graph) note_launch(a->kernels[key]);
             if (st != JP_OK && (graph || a->graph[key])) return st;
             if (st != JP_OK) {
                 cudaGetLastError();
@@ -1348,7 +1361,7 @@ jp_status amr_set_step_map(jp_solver* s, int vec, int tpb) {
 }
 
 jp_status amr_regrid(jp_solver* s) {
-    jp_status st = regrid(s);  // the captured steps stay valid unless a pool grew (grow_l1/grow_l2 drop them)
+    jp_status st = regrid(s);  // the recorded steps stay valid unless a pool grew (grow_l1/grow_l2 drop them)
     if (st == JP_OK) {
         const cudaError_t e = wait_stream(s);
         if (e != cudaSuccess) st = cuda_fail(e, "regrid");

@@ -13,6 +13,7 @@ std::function<void(Op&)> on_kernel;
 std::function<void(void*, size_t)> on_d2h;
 std::function<cudaError_t(const std::string&)> launch_error;
 std::function<float()> elapsed;
+std::vector<std::vector<Node>> graphs;
 long long allocations = 0, fail_from = 1, fail_to = 0;
 size_t free_bytes = (size_t)64 << 30;
 
@@ -322,6 +323,7 @@ cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) {
 
 // ---- graphs ----
 cudaError_t cudaStreamBeginCapture(cudaStream_t s, cudaStreamCaptureMode) {
+    record(Op::CAPTURE, s);
     of(s).capturing = true;
     return cudaSuccess;
 }
@@ -334,8 +336,29 @@ cudaError_t cudaGraphInstantiate(cudaGraphExec_t* x, cudaGraph_t, unsigned long 
     *x = (cudaGraphExec_t)std::malloc(1);
     return cudaSuccess;
 }
+// a graph is its index in graphs, plus one; a node its index in its graph, plus one
+cudaError_t cudaGraphCreate(cudaGraph_t* g, unsigned) {
+    graphs.emplace_back();
+    *g = (cudaGraph_t)graphs.size();
+    return cudaSuccess;
+}
+cudaError_t cudaGraphAddKernelNode(cudaGraphNode_t* node, cudaGraph_t g, const cudaGraphNode_t* deps, size_t n,
+                                   const cudaKernelNodeParams* p) {
+    std::vector<Node>& nodes = graphs[(size_t)g - 1];
+    Node k{kernels[p->func], {}};
+    std::set<size_t> after;
+    for (size_t i = 0; i < n; ++i) {
+        const size_t d = (size_t)deps[i] - 1;
+        after.insert(d);
+        after.insert(nodes[d].after.begin(), nodes[d].after.end());
+    }
+    k.after.assign(after.begin(), after.end());
+    nodes.push_back(k);
+    *node = (cudaGraphNode_t)nodes.size();
+    return cudaSuccess;
+}
 cudaError_t cudaGraphDestroy(cudaGraph_t g) {
-    std::free(g);
+    if ((size_t)g > graphs.size()) std::free(g);
     return cudaSuccess;
 }
 cudaError_t cudaGraphExecDestroy(cudaGraphExec_t x) {

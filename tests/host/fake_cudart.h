@@ -19,7 +19,7 @@ namespace fake {
 using Clock = std::map<const void*, unsigned>;  // by stream; the host under nullptr
 
 struct Op {
-    enum Kind { KERNEL, MEMSET, COPY, GRAPH_LAUNCH, GRAPH_UPLOAD } kind;
+    enum Kind { KERNEL, MEMSET, COPY, GRAPH_LAUNCH, GRAPH_UPLOAD, CAPTURE } kind;
     std::string name;      // kernel: its (mangled) name
     cudaStream_t stream;
     Clock clock;
@@ -31,6 +31,11 @@ struct Op {
     size_t bytes;
 };
 bool before(const Op& a, const Op& b);  // a is ordered before b
+struct Node {              // a kernel node of a graph built by hand
+    std::string name;
+    std::vector<size_t> after;  // indices of the nodes it depends on, directly or not
+};
+extern std::vector<std::vector<Node>> graphs;  // every graph created
 
 extern std::vector<Op> ops;
 extern std::vector<std::string> faults;                              // accesses outside an allocation

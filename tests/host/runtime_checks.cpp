@@ -411,6 +411,35 @@ static void upload_precedes_replay_on_its_stream() {
     jp_destroy(s);
 }
 
+// Steps become graphs without a stream capture, which would make other threads' calls that wait for the device
+// fail meanwhile, and a graph's kernels are ordered exactly as the launches of the step are.
+static void graphs_order_kernels_as_streams_do() {
+    supply_grid();
+    for (const int flags : {0, (int)JP_FLAG_GRAPH, (int)JP_FLAG_SKIP_PREP, (int)JP_FLAG_SKIP_RESTRICT})
+        for (const int nref1 : {10, 0}) {
+            set_grid(16, nref1);
+            jp_solver* s = amr(64.0, flags & JP_FLAG_GRAPH ? 0 : flags);  // one step by launches
+            size_t from = fake::ops.size();
+            CHECK(jp_step(s, 1) == JP_OK);
+            const std::vector<fake::Op> direct(fake::ops.begin() + (long)from, fake::ops.end());
+            jp_solver* g = flags & JP_FLAG_GRAPH ? amr(64.0, flags) : s;
+            from = fake::ops.size();
+            CHECK(jp_step(g, 8) == JP_OK);
+            for (size_t i = from; i < fake::ops.size(); ++i) CHECK(fake::ops[i].kind != fake::Op::CAPTURE);
+            CHECK(!fake::graphs.empty());
+            if (fake::graphs.empty()) return;
+            const std::vector<fake::Node>& nodes = fake::graphs.back();
+            CHECK(nodes.size() == direct.size());
+            // the same kernels in the order of issue
+            for (size_t i = 0; i < nodes.size() && i < direct.size(); ++i) CHECK(nodes[i].name == direct[i].name);
+            for (size_t i = 0; i < nodes.size() && i < direct.size(); ++i)
+                for (size_t j = 0; j < i; ++j)
+                    CHECK(std::count(nodes[i].after.begin(), nodes[i].after.end(), j) == (fake::before(direct[j], direct[i]) ? 1 : 0));
+            if (g != s) jp_destroy(g);
+            jp_destroy(s);
+        }
+}
+
 int main(int argc, char** argv) {
     const std::map<std::string, void (*)()> checks = {
         {"regrid_orders_list_counts", regrid_orders_list_counts},
@@ -424,6 +453,7 @@ int main(int argc, char** argv) {
         {"failed_conversion_waits_for_its_copies", failed_conversion_waits_for_its_copies},
         {"replayed_steps_count_their_kernels", replayed_steps_count_their_kernels},
         {"upload_precedes_replay_on_its_stream", upload_precedes_replay_on_its_stream},
+        {"graphs_order_kernels_as_streams_do", graphs_order_kernels_as_streams_do},
     };
     const auto it = argc == 2 ? checks.find(argv[1]) : checks.end();
     if (it == checks.end()) return 2;
