@@ -296,8 +296,9 @@ jp_status jp_load_state(jp_solver* s, const char* path);
 /* An ensemble steps many solvers of the same device together, on the ensemble's streams (uniform and
  * AMR members beside each other), ordered after each member's pending work and before its later
  * work.  Uniform members: one batched stream-collide launch per storage format per lattice step, or
- * per two steps in FP32 (up to 48 cubes of any sizes per launch).  AMR members: one coarse step (the 1:2:4 subcycle) with one launch per stage over the
- * blocks of all members of the same block edge, storage and step threads (up to 48 per launch);
+ * per two steps in FP32 (up to 48 cubes of any sizes per launch).  AMR members: one coarse step (the
+ * 1:2:4 subcycle) with one launch per stage over the blocks of all members of the same block edge,
+ * storage and step threads (up to 48 per launch);
  * jp_ensemble_step(e, k) advances AMR members by k coarse steps.  Regrids and diagnostics stay
  * per solver (jp_regrid, jp_diag) between ensemble steps. */
 typedef struct jp_ensemble jp_ensemble;

@@ -92,6 +92,9 @@ __device__ __forceinline__ void step_release() { asm volatile("griddepcontrol.la
 // N=64 5.36 / 5.26, N=72 6.62 / 6.68, N=128 34.0 / 34.4, N=192 109.7 / 110.8;
 // FP16 N=24 2.24 / 2.34, N=32 2.95 / 2.36, N=48 3.21 / 3.01, N=56 4.46 / 3.98, N=64 4.31 / 4.50, N=80 6.54 / 6.79;
 // FP64 N=32 28.6 / 11.3 (a CTA keeps its SM's FP64 pipe busy).
+// The two-step pass (N=8, 32, 128 and 192 above) goes by the same rule, for its figures alone: its CTAs fill an SM's
+// registers each and its grid has at most one per SM, so a successor's CTA takes an SM that has none or whose
+// CTA has ended; that is worth 1 % either way.
 [[maybe_unused]] static bool release_early(bool shifted, bool fp64, int n) {
     const long long cells = (long long)n * n * n;
     if (fp64) return false;

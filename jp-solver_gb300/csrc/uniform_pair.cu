@@ -6,7 +6,7 @@
 // on the tile and a one-cell halo around it (a thread per pair of x-adjacent cells, the populations
 // pulled from global memory), keeps the relaxed populations in a ring of planes in shared memory, and
 // takes the second step of the plane before, whose pulls come out of the ring.  HBM moves 152 B per two
-// updates plus the chunks' two halo planes; the tile's halo (29 % of the first step's cells at 64 x 9) is
+// updates plus the chunks' two halo planes; the tile's halo (23 % of the first step's cells at 64 x 9) is
 // recomputed and its loads hit L2, where the neighbouring tiles' CTAs have just read the same rows.  A
 // population takes a plane's slot in the ring only while a second step still needs it: c_z = +1 for
 // three planes, 0 for two, -1 for one; the populations with c_x = c_y = 0 never leave their thread.
