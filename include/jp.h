@@ -287,7 +287,8 @@ jp_status jp_set_sensor_override(jp_solver* s, const float* sen0, const float* s
  * counts, capacities, block tables and the populations of the blocks in use.  jp_load_state into a
  * solver created with the same kind, n, mb, storage, Re, u0 and refinement modes (t*, diagnostic
  * and regrid cadence may differ) continues bit for bit where the saved solve was, including later
- * regrids.  JP_ERR_INVALID for a file of another configuration, ABI or a truncated file. */
+ * regrids.  JP_ERR_INVALID for a file of another configuration, ABI or a truncated file.  A load that fails
+ * past the file's headers leaves an AMR solver without a grid, as jp_regrid does half-way. */
 jp_status jp_save_state(jp_solver* s, const char* path);
 jp_status jp_load_state(jp_solver* s, const char* path);
 

@@ -3,8 +3,8 @@
 // The reference (src/tgv3d_amr.cu:514-549) writes the state as a field on the finest grid, (4 N0)^3 records,
 // and reduces that field with its six neighbours.  A coarse cell is 64 equal records there and a level-1 cell 8,
 // so most of those cells have no gradient of their own: in the dynamic case (N0=96; 520 coarse and 172 level-1
-// blocks refined) 3.4 M leaf cells stand for 56.6 M records.  Here the leaf cells' macroscopic values are computed once per cell (k_leaf_macro), and the
-// reduction walks the leaf blocks and adds a cell's sub-cells in closed form:
+// blocks refined) 3.4 M leaf cells stand for 56.6 M records.  Here the leaf cells' macroscopic values are computed
+// once per cell (k_leaf_macro), and the reduction walks the leaf blocks and adds a cell's sub-cells in closed form:
 //   a cell of edge f = 4, 2, 1 records has along each axis the half differences lo = (v - v_minus) / 2 in its
 //   first layer of records, hi = (v_plus - v) / 2 in its last and zero between (f = 1: (v_plus - v_minus) / 2), so
 //   sum over its f^3 records of (A - B)^2, A along one axis and B along another, is

@@ -300,6 +300,7 @@ static void drop_macro(AmrState* a) {
 static jp_status set_cap1(jp_solver* s, int cap, bool keep) {
     AmrState* a = s->amr;
     const size_t blk = (size_t)Q * a->MB3, old = keep ? std::min(a->cap1, cap) : 0;
+    a->cap1 = std::min(a->cap1, cap);  // what every array holds, also when one below cannot be had
     TRY(regrow(s, a->f1a, pf(a, cap * blk), pf(a, old * blk)));  // payload the migration reads
     TRY(regrow(s, a->f1b, pf(a, cap * blk), 0));
     TRY(regrow(s, a->gh1, pf(a, (size_t)cap * Q * a->SH), 0));
@@ -328,6 +329,7 @@ static jp_status set_cap1(jp_solver* s, int cap, bool keep) {
 static jp_status set_cap2(jp_solver* s, int cap, bool keep) {
     AmrState* a = s->amr;
     const size_t blk = (size_t)Q * a->MB3, old = keep ? std::min(a->cap2, cap) : 0;
+    a->cap2 = std::min(a->cap2, cap);
     TRY(regrow(s, a->f2a, pf(a, cap * blk), pf(a, old * blk)));  // payload the migration reads
     TRY(regrow(s, a->f2b, pf(a, cap * blk), 0));
     TRY(regrow(s, a->gh2, pf(a, (size_t)cap * Q * a->SH), 0));
@@ -1578,13 +1580,14 @@ jp_status amr_save_state(jp_solver* s, std::FILE* f) {
     return JP_OK;
 }
 
-jp_status amr_load_state(jp_solver* s, std::FILE* f) {
+static jp_status load_grid(jp_solver* s, std::FILE* f, bool* touched) {
     AmrState* a = s->amr;
     int64_t h[16];
     if (!fread_all(f, h, sizeof h)) return fail(JP_ERR_INVALID, "state file truncated");
     if (h[0] < 8 || h[1] < 8 || h[5] < 0 || h[5] > h[0] || h[7] < 0 || h[7] > h[1] || h[8] > a->cnb0 || h[9] > h[0])
         return fail(JP_ERR_INVALID, "state file: inconsistent block counts");
     ACK(wait_stream(s), "load");
+    *touched = true;
     if (h[0] != a->cap1) TRY(set_cap1(s, (int)h[0], false));
     if (h[1] != a->cap2) TRY(set_cap2(s, (int)h[1], false));
     a->cap_nref0 = (int)h[2];
@@ -1623,6 +1626,15 @@ jp_status amr_load_state(jp_solver* s, std::FILE* f) {
     reset_graphs(a);
     update_bytes(s);
     return JP_OK;
+}
+jp_status amr_load_state(jp_solver* s, std::FILE* f) {
+    bool touched = false;
+    const jp_status st = load_grid(s, f, &touched);
+    if (st != JP_OK && touched) {  // tables of two grids, arrays that have moved under the recorded steps
+        s->initialized = false;
+        drop_grid(s);
+    }
+    return st;
 }
 
 jp_status amr_get_counts(jp_solver* s, jp_amr_counts* o) {

@@ -440,6 +440,76 @@ static void graphs_order_kernels_as_streams_do() {
         }
 }
 
+// A state file that ends early, or memory that does, half-way through a load leaves no mixture of two grids (and no
+// recorded steps of arrays that have moved): the solver has no grid until a load or a new initial state succeeds.
+static void failed_load_leaves_no_grid() {
+    supply_grid();
+    fake::on_kernel = check_leaf_macro;
+    double d[3];
+    set_grid(20, 18);
+    jp_solver* big = amr(64.0);
+    set_grid(16, 10);
+    CHECK(jp_save_state(big, "big.jps") == JP_OK);
+    jp_destroy(big);
+    std::FILE* f = std::fopen("big.jps", "rb");
+    std::vector<char> bytes(64 << 20);
+    bytes.resize(std::fread(bytes.data(), 1, bytes.size(), f));
+    std::fclose(f);
+    jp_solver* s = amr(64.0);
+    const auto refused = [&](jp_status want) {
+        CHECK(jp_load_state(s, "cut.jps") == want);
+        CHECK(jp_step(s, 1) == JP_ERR_STATE && jp_diag(s, d) == JP_ERR_STATE);
+        set_grid(16, 10);
+        CHECK(jp_init_tgv(s) == JP_OK && jp_step(s, 12) == JP_OK && jp_diag(s, d) == JP_OK);
+    };
+    const auto cut = [&](size_t n) {
+        std::FILE* out = std::fopen("cut.jps", "wb");
+        std::fwrite(bytes.data(), 1, n, out);
+        std::fclose(out);
+    };
+    CHECK(jp_step(s, 12) == JP_OK);  // recorded
+    cut(100);
+    CHECK(jp_load_state(s, "cut.jps") == JP_ERR_INVALID);  // within the headers: nothing touched
+    CHECK(jp_step(s, 1) == JP_OK);
+    for (const size_t n : {(size_t)300, (size_t)5000, bytes.size() / 2, bytes.size() - 4}) {
+        cut(n);
+        refused(JP_ERR_INVALID);
+    }
+    cut(bytes.size());
+    for (int k = 0; k < 7; ++k) {  // the level-2 pool's arrays
+        fake::fail_from = fake::fail_to = fake::allocations + k;
+        refused(JP_ERR_NOMEM);
+    }
+    fake::fail_to = -1;
+    CHECK(jp_load_state(s, "cut.jps") == JP_OK && jp_step(s, 12) == JP_OK && jp_diag(s, d) == JP_OK);
+    jp_destroy(s);
+    // into pools larger than the file's, whose arrays shrink one by one
+    for (int k = 0; k < 60; ++k) {
+        set_grid(16, 10);
+        s = watched = amr(64.0);
+        set_grid(40, 40);
+        CHECK(jp_regrid(s) == JP_OK);
+        fake::fail_from = fake::fail_to = fake::allocations + k;
+        const jp_status st = jp_load_state(s, "big.jps");
+        fake::fail_to = -1;
+        set_grid(40, 40);
+        CHECK(st == JP_ERR_NOMEM ? jp_init_tgv(s) == JP_OK : st == JP_OK);
+        jp_amr_counts c;
+        CHECK(jp_step(s, 2) == JP_OK && jp_diag(s, d) == JP_OK && jp_amr_get_counts(s, &c) == JP_OK);
+        std::vector<float> p(19 * 512 * 2000);
+        for (int level = 0; level < 3; ++level) {
+            int64_t n = 0;
+            CHECK(jp_population_count(s, level, &n) == JP_OK);
+            CHECK(jp_get_populations(s, level, JP_LAYOUT_BLOCKED, JP_F32, p.data(), n) == JP_OK);
+        }
+        CHECK(c.nf1 <= c.cap1 && c.nf2 <= c.cap2);
+        watched = nullptr;
+        jp_destroy(s);
+        if (st == JP_OK) break;
+        CHECK(k < 59);
+    }
+}
+
 int main(int argc, char** argv) {
     const std::map<std::string, void (*)()> checks = {
         {"regrid_orders_list_counts", regrid_orders_list_counts},
@@ -454,6 +524,7 @@ int main(int argc, char** argv) {
         {"replayed_steps_count_their_kernels", replayed_steps_count_their_kernels},
         {"upload_precedes_replay_on_its_stream", upload_precedes_replay_on_its_stream},
         {"graphs_order_kernels_as_streams_do", graphs_order_kernels_as_streams_do},
+        {"failed_load_leaves_no_grid", failed_load_leaves_no_grid},
     };
     const auto it = argc == 2 ? checks.find(argv[1]) : checks.end();
     if (it == checks.end()) return 2;

@@ -45,6 +45,7 @@ def checks(tmp_path_factory):
     "replayed_steps_count_their_kernels",
     "upload_precedes_replay_on_its_stream",
     "graphs_order_kernels_as_streams_do",
+    "failed_load_leaves_no_grid",
 ])
 def test_host_code(checks, name, tmp_path):
     r = subprocess.run([checks, name], capture_output=True, text=True, timeout=120, cwd=tmp_path)
